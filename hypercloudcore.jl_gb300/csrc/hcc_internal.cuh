@@ -304,6 +304,7 @@ template <typename T> struct StageArgs {
     const int8_t *nbmin;              // EPD2: neighbourhood minimum of the orders
     T *grad;                          // [i * Br * M]
     const T *U;                       // stage state Y_s
+    T *lam;                           // CFL step: per particle the axis speeds (Euler), lam_stride(D) apart
     double *wflux64;                  // FP64 Euler WENO: per particle F_d(U)_m and lambda_d of the stage state
     T *K;                             // K_E[s]
     int full;                         // 1: every particle; 0: the members of a tile worklist
