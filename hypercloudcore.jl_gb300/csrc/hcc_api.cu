@@ -209,7 +209,7 @@ struct hcc_ctx {
     double *inv_r64 = nullptr, *inv_d64 = nullptr, *dw64 = nullptr, *dw1_64 = nullptr;
     uint8_t *ok_r = nullptr, *ok_d = nullptr, *ok_1 = nullptr;
     float *dist32 = nullptr, *w32 = nullptr, *dw32 = nullptr, *dw1_32 = nullptr, *inv_r32 = nullptr, *gw32 = nullptr;
-    int32_t *status = nullptr, *status2 = nullptr, *root = nullptr;
+    int32_t *status = nullptr, *root = nullptr;
     int32_t *blist = nullptr, *bsrc = nullptr; int64_t nbnd = 0;
     // state (element type double or float)
     void *rhos = nullptr, *cand = nullptr, *grad = nullptr;
@@ -256,7 +256,7 @@ struct hcc_ctx {
         for (int q = 0; q < HCC_MAX_STAGES; ++q) { dfree(Xs[q]); dfree(KXs[q]); }
     }
     bool u2_plateau_on() const { return cfg.mood_criterion == HCC_MOOD_U2 && cfg.u2_plateau > 0.0; }
-    unsigned long long *d_counters = nullptr;   // [0..1] drop counters, [2] dt bits, [3..4] search stats
+    unsigned long long *d_counters = nullptr;   // [0..1] drop counters, [2] dt bits, [3..5] search stats
     unsigned long long *h_counters = nullptr;   // pinned mirror
     double *d_mass = nullptr;
     bool have_cloud = false, have_nb = false, have_geom = false, have_state = false;
@@ -348,7 +348,7 @@ struct hcc_ctx {
         dfree(pos); dfree(bnd); dfree(tags); dfree(vol); dfree(bin_of); dfree(cellp); dfree(cnt);
         dfree(pos32); dfree(pmax32); dfree(wops); dfree(wcnt); dfree(wchol); dfree(wok); dfree(wflux64);
         dfree(ok_r); dfree(ok_d); dfree(ok_1); dfree(inv_r64); dfree(inv_d64); dfree(inv_r32);
-        dfree(status); dfree(status2); dfree(root); dfree(blist); dfree(bsrc);
+        dfree(status); dfree(root); dfree(blist); dfree(bsrc);
         for (void **p : {&rhos, &cand, &grad, &xfer}) { if (*p) cudaFree(*p); *p = nullptr; }
         for (int s = 0; s < HCC_MAX_STAGES; ++s)
             for (void **p : {&Y[s], &KE[s], &KI[s]}) { if (*p) cudaFree(*p); *p = nullptr; }
@@ -1271,7 +1271,6 @@ hcc_status hcc_upload_cloud(hcc_ctx *c, int64_t n, const double *pos, const uint
     HCC_TRY(c->alloc(c->inv_d64, size_t(np) * c->Bd * c->Bd, "inv_d"));
     if (c->f32) HCC_TRY(c->alloc(c->inv_r32, size_t(np) * c->Br * c->Br, "inv_r32"));
     HCC_TRY(c->alloc(c->status, np, "status"));
-    HCC_TRY(c->alloc(c->status2, np, "status2"));
     HCC_TRY(c->alloc(c->root, np, "root"));
     const size_t sb = size_t(np) * M * c->esz();
     HCC_TRY(c->valloc(c->rhos, sb, "rhos"));
@@ -1306,6 +1305,15 @@ hcc_status hcc_upload_cloud(hcc_ctx *c, int64_t n, const double *pos, const uint
     HCC_TRY(c->cuda(cudaMemcpyAsync(c->bnd, is_boundary, n, cudaMemcpyHostToDevice, c->stream), "upload is_boundary"));
     HCC_TRY(c->cuda(cudaMemcpyAsync(c->tags, tags, n * sizeof(int32_t), cudaMemcpyHostToDevice, c->stream), "upload tags"));
     HCC_TRY(c->cuda(cudaMemcpyAsync(c->vol, v.data(), n * sizeof(double), cudaMemcpyHostToDevice, c->stream), "upload volumes"));
+    std::vector<int32_t> bl;
+    for (int64_t i = 0; i < n; ++i)
+        if (is_boundary[i]) bl.push_back(int32_t(i));
+    c->nbnd = int64_t(bl.size());
+    HCC_TRY(c->alloc(c->blist, bl.size(), "boundary list"));
+    HCC_TRY(c->alloc(c->bsrc, bl.size(), "boundary sources"));
+    if (!bl.empty())
+        HCC_TRY(c->cuda(cudaMemcpyAsync(c->blist, bl.data(), bl.size() * sizeof(int32_t), cudaMemcpyHostToDevice,
+                                        c->stream), "boundary list"));
     HCC_TRY(c->sync("upload cloud"));
     c->have_cloud = true;
     return HCC_OK;
@@ -1318,7 +1326,7 @@ hcc_status hcc_build_neighbours(hcc_ctx *c) {
     const hcc_config &f = c->cfg;
     const int D = c->D;
     hcc_status st;
-    // GlobalBins (NeighborLogic.jl:22-40) and the 3^D window of every bin (_fill_bin_neighbors!, :43-76), on the host
+    // GlobalBins (NeighborLogic.jl:22-40); the 3^D windows of the bins come with the cell list (k_bin_windows)
     c->nbins = 1;
     for (int d = 0; d < 3; ++d) { c->dims[d] = 1; c->csize[d] = 1.0; }
     for (int d = 0; d < D; ++d) {
@@ -1330,42 +1338,11 @@ hcc_status hcc_build_neighbours(hcc_ctx *c) {
     }
     if (c->nbins > (int64_t(1) << 30)) return c->fail(HCC_ERR_CAPACITY, "too many cell-list bins");
     c->noff = D == 1 ? 3 : (D == 2 ? 9 : 27);
-    std::vector<int64_t> binnb(size_t(c->nbins) * c->noff);
-    for (int64_t b = 0; b < c->nbins; ++b) {
-        int cart[3] = {0, 0, 0};
-        int64_t r = b;
-        for (int d = 0; d < D; ++d) { cart[d] = int(r % c->dims[d]); r /= c->dims[d]; }
-        int64_t raw[27];
-        for (int w = 0; w < c->noff; ++w) {
-            int q = w;
-            bool valid = true;
-            int64_t lin = 0, stride = 1;
-            for (int d = 0; d < D; ++d) {
-                int off = q % 3 - 1;
-                q /= 3;
-                int nc = cart[d] + off;
-                if (nc < 0 || nc >= c->dims[d]) {
-                    if (f.periodic[d]) nc = ((nc % c->dims[d]) + c->dims[d]) % c->dims[d];
-                    else { valid = false; nc = 0; }
-                }
-                lin += nc * stride;
-                stride *= c->dims[d];
-            }
-            raw[w] = valid ? lin : c->nbins;
-        }
-        for (int w = 0; w < c->noff; ++w) {
-            bool rep = false;
-            for (int k = 0; k < w; ++k) rep = rep || raw[k] == raw[w];
-            binnb[size_t(b) * c->noff + w] = rep ? c->nbins : raw[w];
-        }
-    }
     c->free_bins();
-    HCC_TRY(c->alloc(c->binnb, binnb.size(), "bin windows"));
+    HCC_TRY(c->alloc(c->binnb, size_t(c->nbins) * c->noff, "bin windows"));
     HCC_TRY(c->alloc(c->cell_count, c->nbins + 1, "cell counts"));
     HCC_TRY(c->alloc(c->cell_cursor, c->nbins + 1, "cell cursor"));
     HCC_TRY(c->alloc(c->cell_start, c->nbins + 2, "cell start"));
-    HCC_TRY(c->cuda(cudaMemcpyAsync(c->binnb, binnb.data(), binnb.size() * sizeof(int64_t), cudaMemcpyHostToDevice,
-                                    c->stream), "upload bin windows"));
     SearchArgs a{};
     a.n = c->n; a.npad = c->npad; a.D = D; a.pos = c->pos;
     const double R = f.radius;
@@ -1382,6 +1359,7 @@ hcc_status hcc_build_neighbours(hcc_ctx *c) {
     a.nbins = c->nbins; a.noff = c->noff; a.binnb = c->binnb;
     a.bin_of = c->bin_of; a.cell_count = c->cell_count; a.cell_start = c->cell_start; a.cell_cursor = c->cell_cursor;
     a.cellp = c->cellp; a.cnt = c->cnt;
+    a.bnd = c->bnd;
     a.R_sq = R * R;
     a.alpha = f.weight_alpha;
     a.invR2 = 1.0 / (R * R);
@@ -1395,11 +1373,12 @@ hcc_status hcc_build_neighbours(hcc_ctx *c) {
     }
     if ((st = search_bins(a, c->stream, c->err)) != HCC_OK) return st;
     if ((st = search_count(a, c->stream, c->d_counters + 3, c->err)) != HCC_OK) return st;
-    HCC_TRY(c->cuda(cudaMemcpyAsync(c->h_counters + 3, c->d_counters + 3, 2 * sizeof(unsigned long long),
+    HCC_TRY(c->cuda(cudaMemcpyAsync(c->h_counters + 3, c->d_counters + 3, 3 * sizeof(unsigned long long),
                                     cudaMemcpyDeviceToHost, c->stream), "search stats"));
     HCC_TRY(c->sync("neighbour count"));
     const int64_t kmax = int64_t(c->h_counters[3]);
     c->total_nb = int64_t(c->h_counters[4]);
+    c->min_nb_interior = c->n_interior > 0 ? int32_t(c->h_counters[5]) : 0;
     if (f.slot_capacity > 0 && kmax > f.slot_capacity)
         return c->fail(HCC_ERR_CAPACITY, "max neighbours above the reserved slot capacity");
     c->free_slots();
@@ -1411,14 +1390,7 @@ hcc_status hcc_build_neighbours(hcc_ctx *c) {
     a.nidx = c->nidx; a.w = c->w64; a.dist = c->dist64; a.kmax = c->kmax;
     if ((st = search_write(a, c->stream, c->err)) != HCC_OK) return st;
     HCC_TRY(c->sync("neighbour write"));
-    c->launches_total += 7;
-    {
-        std::vector<int32_t> cnt(c->n);
-        HCC_TRY(c->cuda(cudaMemcpy(cnt.data(), c->cnt, c->n * 4, cudaMemcpyDeviceToHost), "counts"));
-        int32_t mn = INT32_MAX;
-        for (int64_t i = 0; i < c->n; ++i) if (!c->h_bnd[i]) mn = std::min(mn, cnt[i]);
-        c->min_nb_interior = mn == INT32_MAX ? 0 : mn;
-    }
+    c->launches_total += 8;
     c->have_nb = true;
     c->have_geom = false;
     return HCC_OK;
@@ -1651,7 +1623,6 @@ hcc_status hcc_prepare_geometry(hcc_ctx *c) {
     const size_t slots = size_t(std::max(c->kmax, 1)) * c->npad;
     HCC_TRY(c->alloc(c->dw64, slots * D, "divergence weights"));
     if (c->need_dw1) HCC_TRY(c->alloc(c->dw1_64, slots * D, "degree-1 weights"));
-    cudaMemsetAsync(c->dw64, 0, slots * D * sizeof(double), c->stream);
     MlsArgs m{};
     m.n = c->n; m.npad = c->npad; m.D = D; m.rdeg = c->rdeg; m.Br = c->Br; m.ddeg = c->ddeg; m.Bd = c->Bd;
     m.max_order = c->max_order; m.DO = c->DO; m.need_dw1 = c->need_dw1;
@@ -1672,23 +1643,24 @@ hcc_status hcc_prepare_geometry(hcc_ctx *c) {
     }
     if (c->moment()) {
         HCC_TRY(c->alloc(c->mw64, slots * D, "moment weights"));
-        cudaMemsetAsync(c->mw64, 0, slots * D * sizeof(double), c->stream);
         m.mw = c->mw64;
         m.aligned = c->cfg.flux == HCC_FLUX_ALIGNED;
     }
-    if ((st = mls_prepare(m, c->stream, c->err)) != HCC_OK) return st;
+    m.linear = !c->no_recon() && c->rdeg == 1;     // order <= 2: both fits are linear
     if (c->f32) {
         HCC_TRY(c->alloc(c->dist32, slots * D, "distances f32"));
         HCC_TRY(c->alloc(c->w32, slots, "weights f32"));
         HCC_TRY(c->alloc(c->dw32, slots * D, "divergence weights f32"));
-        launch_cast_f64_to_f32(c->dist64, c->dist32, int64_t(slots) * D, c->stream);
-        launch_cast_f64_to_f32(c->w64, c->w32, int64_t(slots), c->stream);
-        launch_cast_f64_to_f32(c->dw64, c->dw32, int64_t(slots) * D, c->stream);
+        if (m.linear) HCC_TRY(c->alloc(c->gw32, slots * D, "gradient weights f32"));
+        m.dist32 = c->dist32; m.w32 = c->w32; m.dw32 = c->dw32; m.gw32 = c->gw32;
+    }
+    if ((st = mls_prepare(m, c->stream, c->err)) != HCC_OK) return st;
+    if (c->f32) {
         launch_cast_f64_to_f32(c->inv_r64, c->inv_r32, c->npad * c->Br * c->Br, c->stream);
-        if (c->rdeg == 1 && !c->no_recon()) {
-            HCC_TRY(c->alloc(c->gw32, slots * D, "gradient weights f32"));
-            launch_grad_weights(c->n, c->npad, D, std::max(c->kmax, 1), c->cnt, c->dist64, c->w64, c->inv_r64, c->ok_r,
-                                c->invL, c->gw32, c->stream);
+        if (!m.linear) {                           // (k_mls_linear writes its own)
+            launch_cast_f64_to_f32(c->dist64, c->dist32, int64_t(slots) * D, c->stream);
+            launch_cast_f64_to_f32(c->w64, c->w32, int64_t(slots), c->stream);
+            launch_cast_f64_to_f32(c->dw64, c->dw32, int64_t(slots) * D, c->stream);
         }
         if (c->need_dw1) {
             HCC_TRY(c->alloc(c->dw1_32, slots * D, "degree-1 weights f32"));
@@ -1729,32 +1701,15 @@ hcc_status hcc_prepare_geometry(hcc_ctx *c) {
         c->ops->weno_geom(wg, c->stream);
         HCC_TRY(launch_check(c, "WENO factors"));
     }
-    // outflow donor roots, then the boundary list (tag -> condition)
+    // outflow donor roots and the sources of the boundary list
     DonorArgs da{};
     da.n = c->n; da.npad = c->npad; da.D = D; da.cnt = c->cnt; da.nidx = c->nidx; da.dist = c->dist64;
-    da.bnd = c->bnd; da.tags = c->tags; da.status = c->status; da.status_prev = c->status2; da.root = c->root;
-    if ((st = donor_map(da, -1, c->stream, c->err)) != HCC_OK) return st;
+    da.bnd = c->bnd; da.tags = c->tags; da.status = c->status; da.root = c->root;
+    da.nb = c->nbnd; da.blist = c->blist; da.bsrc = c->bsrc;
     for (int tag = 1; tag <= HCC_MAX_TAGS; ++tag)
-        if (c->cfg.bc_by_tag[tag - 1] == HCC_BC_OUTFLOW)
-            if ((st = donor_map(da, tag, c->stream, c->err)) != HCC_OK) return st;
-    std::vector<int32_t> root(c->n);
+        if (c->cfg.bc_by_tag[tag - 1] == HCC_BC_OUTFLOW) da.outflow_tags |= 1u << (tag - 1);
+    if ((st = donor_map(da, c->stream, c->err)) != HCC_OK) return st;
     HCC_TRY(c->sync("geometry kernels"));
-    if (c->n) HCC_TRY(c->cuda(cudaMemcpy(root.data(), c->root, c->n * sizeof(int32_t), cudaMemcpyDeviceToHost), "donor roots"));
-    std::vector<int32_t> bl, bs;
-    for (int64_t i = 0; i < c->n; ++i) {
-        if (!c->h_bnd[i]) continue;
-        int tag = c->h_tags[i];
-        int kind = (tag >= 1 && tag <= HCC_MAX_TAGS) ? c->cfg.bc_by_tag[tag - 1] : HCC_BC_KEEP;
-        bl.push_back(int32_t(i));
-        bs.push_back(kind == HCC_BC_OUTFLOW ? root[i] : -1);
-    }
-    c->nbnd = int64_t(bl.size());
-    HCC_TRY(c->alloc(c->blist, std::max<size_t>(bl.size(), 1), "boundary list"));
-    HCC_TRY(c->alloc(c->bsrc, std::max<size_t>(bs.size(), 1), "boundary sources"));
-    if (!bl.empty()) {
-        HCC_TRY(c->cuda(cudaMemcpy(c->blist, bl.data(), bl.size() * 4, cudaMemcpyHostToDevice), "boundary list"));
-        HCC_TRY(c->cuda(cudaMemcpy(c->bsrc, bs.data(), bs.size() * 4, cudaMemcpyHostToDevice), "boundary sources"));
-    }
     c->have_geom = true;
     return HCC_OK;
 }

@@ -455,7 +455,8 @@ struct SearchArgs {
     int dims[3];
     int64_t nbins;
     int noff;
-    const int64_t *binnb;             // [nbins * noff]
+    int64_t *binnb;                   // [nbins * noff]
+    const uint8_t *bnd;               // for the smallest interior count
     int32_t *bin_of;                  // [n]
     int32_t *cell_count;              // [nbins + 1]
     int64_t *cell_start;              // [nbins + 2]
@@ -495,22 +496,30 @@ struct MlsArgs {
     int central_qmax;                 // > 0: CentralDivergence weight sets of degree 1..central_qmax
     double *dwc[3];
     uint8_t *okc[3];
+    int linear;                       // every fit is linear (order <= 2, degree-1 divergence, MUSCL): k_mls_linear,
+    float *dw32, *w32, *dist32, *gw32;   // which in FP32 contexts (gw32 set) also writes the FP32 streams
     double *mw;                       // != nullptr: moment-correction weights of a first-order scheme (from dw)
     int aligned;                      // AlignedRusanovFlux (the dissipation direction of the moment weights)
 };
 hcc_status mls_prepare(MlsArgs &a, cudaStream_t s, std::string &err);
 
-// Outflow donor map (BoundaryConditions.jl:82-130 with the state-free part precomputed per geometry).
+// Outflow donor map (BoundaryConditions.jl:82-130 with the state-free part precomputed per geometry) and the sources of
+// the boundary list.
 struct DonorArgs {
-    int64_t n, npad;
+    int64_t n, npad, nb;
     int D;
     const int32_t *cnt, *nidx;
     const double *dist;
     const uint8_t *bnd;
     const int32_t *tags;
-    int32_t *status, *status_prev, *root;
+    const int32_t *blist;             // [nb] boundary particles
+    uint32_t outflow_tags;            // bit t - 1: tag t is an outflow tag
+    int32_t *status, *root, *bsrc;
+    __device__ __forceinline__ bool outflow(int32_t tag) const {
+        return tag >= 1 && tag <= HCC_MAX_TAGS && ((outflow_tags >> (tag - 1)) & 1u);
+    }
 };
-hcc_status donor_map(DonorArgs &a, int tag, cudaStream_t s, std::string &err);
+hcc_status donor_map(DonorArgs &a, cudaStream_t s, std::string &err);
 
 // Small utility kernels (hcc_util.cu).
 void launch_cast_f64_to_f32(const double *src, float *dst, int64_t n, cudaStream_t s);
@@ -550,11 +559,6 @@ void launch_force(const int32_t *ctiles, uint32_t *cmask, ListCounts *counts, in
                   uint32_t *fmask, int32_t *ftiles, int blocks, cudaStream_t s);
 void launch_count_inadmissible(const uint8_t *inadm, const uint8_t *bnd, int64_t n, unsigned long long *out,
                                cudaStream_t s);
-// Gradient weights of the cached degree-1 fit (FP64 sums, FP32 store): gw[(k*D + b) * npad + i] =
-// invL Σ_c inv_r[b][c] w_k (dist_k[c] invL) for particles with ok_r, 0 elsewhere.
-void launch_grad_weights(int64_t n, int64_t npad, int D, int kmax, const int32_t *cnt, const double *dist,
-                         const double *w, const double *inv_r, const uint8_t *ok_r, double invL, float *gw,
-                         cudaStream_t s);
 void launch_shepard(const int32_t *cnt, const int32_t *nidx, const double *w, int64_t n, int64_t npad, double w0,
                     int sweeps, double *S, double *V, double *Vt, double *partial, cudaStream_t s);
 void launch_scale(double *V, int64_t n, double f, cudaStream_t s);

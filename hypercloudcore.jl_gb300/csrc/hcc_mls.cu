@@ -13,6 +13,7 @@
 #include <algorithm>
 #include <array>
 #include <mutex>
+#include <type_traits>
 
 namespace hcc {
 namespace {
@@ -291,6 +292,158 @@ __global__ void k_mls(MlsArgs a) {
     }
 }
 
+// Cholesky factor and inverse of a B x B moment matrix held in registers, the operations of cholesky_moment and
+// chol_solve in their order. In the column j of the inverse the forward solution is zero above row j (0 - u 0 = 0,
+// 0 / u = 0 for the positive pivots), so those steps are left out.
+template <int B>
+__device__ __forceinline__ bool chol_fixed(const double (&N)[B][B], double (&U)[B][B]) {
+    bool ok = true;
+#pragma unroll
+    for (int i = 0; i < B; ++i)
+#pragma unroll
+        for (int j = i; j < B; ++j) {
+            double s = N[i][j];
+#pragma unroll
+            for (int k = 0; k < i; ++k) s = s - U[k][i] * U[k][j];
+            if (i == j) {
+                ok = ok && s > 0.0;
+                U[i][i] = sqrt(s);
+            } else {
+                U[i][j] = s / U[i][i];
+            }
+        }
+    return ok;
+}
+template <int B> __device__ __forceinline__ bool invert_fixed(double (&N)[B][B], double (&inv)[B][B]) {
+    double U[B][B];
+    bool ok = chol_fixed<B>(N, U);
+    if (ok) {
+        const double tol = 10.0 * 2.220446049250313e-16;
+#pragma unroll
+        for (int k = 0; k < B; ++k) ok = ok && (U[k][k] * U[k][k] > tol * N[k][k]);
+    }
+    if (!ok) {
+        double tr = 0.0;
+#pragma unroll
+        for (int k = 0; k < B; ++k) tr = tr + N[k][k];
+        const double eps_reg = 1.4901161193847656e-08 * tr / double(B);
+#pragma unroll
+        for (int k = 0; k < B; ++k) N[k][k] = N[k][k] + eps_reg;
+        ok = chol_fixed<B>(N, U);
+    }
+#pragma unroll
+    for (int j = 0; j < B; ++j) {
+        double y[B], x[B];
+        y[j] = 1.0 / U[j][j];
+#pragma unroll
+        for (int r = j + 1; r < B; ++r) {
+            double t = 0.0 - U[j][r] * y[j];
+#pragma unroll
+            for (int k = j + 1; k < r; ++k) t = t - U[k][r] * y[k];
+            y[r] = t / U[r][r];
+        }
+#pragma unroll
+        for (int r = B - 1; r >= 0; --r) {
+            double t = r >= j ? y[r >= j ? r : j] : 0.0;
+#pragma unroll
+            for (int k = r + 1; k < B; ++k) t = t - U[r][k] * x[k];
+            x[r] = t / U[r][r];
+        }
+#pragma unroll
+        for (int r = 0; r < B; ++r) inv[r][j] = ok ? x[r] : 0.0;
+    }
+    return ok;
+}
+
+// The MUSCL caches of contexts whose fits are all linear (order <= 2, degree-1 divergence): what k_mls computes, by the
+// same operations in the same order, with the fit's size known at compile time. FP32 contexts also get the FP32
+// copies of the slot streams and the gradient weights of the cached fit,
+//   gw_k[b] = invL w_k sum_c inv_r[b][c] x_k[c] / h  (FP64 sums, FP32 store),
+// in the second sweep. Bound by the FP64 unit (two lanes a clock and SM): 28 operations a slot for the moments
+// (products with the constant basis term are the other factor), 30 for the divergence weights, 12 for the gradient
+// weights in 3-D, and about 700 for the two inverses. The generic kernel kept its matrices in local memory, and the
+// copies and gradient weights were passes of their own over the FP64 streams: 25.7 ms on 1.59M particles with 66
+// neighbours for the three, 19.8 ms here (2-D, 1.01M particles with 20 neighbours: 3.64 ms, now 2.42).
+template <int D, bool F32>
+__global__ void __launch_bounds__(128) k_mls_linear(MlsArgs a) {
+    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i >= a.n) return;
+    constexpr int B = D + 1;
+    const int cnt = a.cnt[i];
+    const int64_t np = a.npad;
+    double N[B][B], inv[B][B];
+#pragma unroll
+    for (int r = 0; r < B; ++r)
+#pragma unroll
+        for (int c = 0; c < B; ++c) N[r][c] = 0.0;
+#pragma unroll 2
+    for (int k = 0; k < cnt; ++k) {
+        double x[D];
+#pragma unroll
+        for (int d = 0; d < D; ++d) x[d] = a.dist[(int64_t(k) * D + d) * np + i] * a.invL;
+        const double w = a.w[int64_t(k) * np + i];
+        N[0][0] = N[0][0] + w;
+#pragma unroll
+        for (int r = 0; r < D; ++r) {
+            N[0][r + 1] = N[0][r + 1] + w * x[r];
+#pragma unroll
+            for (int c = r; c < D; ++c) N[r + 1][c + 1] = N[r + 1][c + 1] + w * (x[r] * x[c]);
+        }
+    }
+    double R[D][D], invr[D][D];
+#pragma unroll
+    for (int r = 0; r < D; ++r)
+#pragma unroll
+        for (int c = 0; c < D; ++c) R[r][c] = N[(r < c ? r : c) + 1][(r < c ? c : r) + 1];
+    const bool okr = invert_fixed<D>(R, invr);
+    a.ok_r[i] = okr;
+#pragma unroll
+    for (int r = 0; r < D; ++r)
+#pragma unroll
+        for (int c = 0; c < D; ++c) a.inv_r[i * (D * D) + r * D + c] = invr[r][c];
+    const bool okd = invert_fixed<B>(N, inv);
+    a.ok_d[i] = okd;
+#pragma unroll
+    for (int r = 0; r < B; ++r)
+#pragma unroll
+        for (int c = 0; c < B; ++c) a.inv_d[i * (B * B) + r * B + c] = inv[r][c];
+#pragma unroll 2
+    for (int k = 0; k < cnt; ++k) {
+        const int64_t s = int64_t(k) * np + i;
+        double xd[D], x[D], v[B];
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+            xd[d] = a.dist[(int64_t(k) * D + d) * np + i];
+            x[d] = xd[d] * a.invL;
+        }
+        const double w = a.w[s];
+        v[0] = w;
+#pragma unroll
+        for (int d = 0; d < D; ++d) v[d + 1] = w * x[d];
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+            double acc = inv[d + 1][0] * v[0];
+#pragma unroll
+            for (int b = 1; b < B; ++b) acc = acc + inv[d + 1][b] * v[b];
+            acc = okd ? acc * a.invL : 0.0;
+            a.dw[(int64_t(k) * D + d) * np + i] = acc;
+            if constexpr (F32) a.dw32[(int64_t(k) * D + d) * np + i] = float(acc);
+        }
+        if constexpr (F32) {
+            a.w32[s] = float(w);
+#pragma unroll
+            for (int d = 0; d < D; ++d) a.dist32[(int64_t(k) * D + d) * np + i] = float(xd[d]);
+#pragma unroll
+            for (int b = 0; b < D; ++b) {
+                double acc = invr[b][0] * x[0];
+#pragma unroll
+                for (int c = 1; c < D; ++c) acc = __fma_rn(invr[b][c], x[c], acc);
+                a.gw32[(int64_t(k) * D + b) * np + i] = float(a.invL * (w * acc));
+            }
+        }
+    }
+}
+
 // CentralDivergence weight set of degree q (Central.jl:45-88 with compute_dynamic_divergence,
 // Interpolators.jl:290-334, per slot as _slot_weight(::DynamicWeights), MUSCL.jl:442-445): C \ (w p~), rows 2..D+1,
 // times invL, for the particles with basis_count(D, q) + 1 neighbours (the others never use degree q).
@@ -454,25 +607,34 @@ __global__ void k_mweights(MlsArgs a) {
 }
 
 // ---- outflow donor map
-__global__ void k_donor_init(DonorArgs a, int tag, int first) {
-    int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+__global__ void k_donor_init(DonorArgs a) {
+    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= a.n) return;
-    a.status[i] = !a.bnd[i] ? 1 : (a.tags[i] == tag ? 0 : -1);
-    if (first) a.root[i] = a.bnd[i] ? -1 : int32_t(i);
+    const bool b = a.bnd[i];
+    a.status[i] = !b ? 1 : (a.outflow(a.tags[i]) ? 0 : -1);
+    a.root[i] = b ? -1 : int32_t(i);
 }
 
-// _outflow_pass! (BoundaryConditions.jl:106-126), propagating the donor's root instead of its state. A particle
-// resolved in this pass gets status pass+1, which no other particle accepts in the same pass.
+// _outflow_pass! (BoundaryConditions.jl:106-126), propagating the donor's root instead of its state, over the boundary
+// list and for every outflow tag at once: a tag's particles take interior donors or resolved ones of their own tag, so
+// the tags do not meet. A particle resolved in this pass gets status pass+1, which no other particle accepts in the
+// same pass. Each entry walks its neighbours (a dependent chain of loads, which bounds the pass); one pass over the list
+// per hop took the place of one over the whole cloud per hop and tag: 1.67 -> 0.57 ms for the 262k ghosts of six walls
+// around 1.33M particles.
 __global__ void k_donor_pass(DonorArgs a, int pass) {
-    int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= a.n || a.status[i] != 0) return;
+    const int64_t q = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (q >= a.nb) return;
+    const int64_t i = a.blist[q];
+    if (a.status[i] != 0) return;
+    const int32_t tag = a.tags[i];
     int32_t closest = -1;
     double mind = INFINITY;
     const int cnt = a.cnt[i];
+#pragma unroll 4
     for (int k = 0; k < cnt; ++k) {
-        int32_t j = a.nidx[int64_t(k) * a.npad + i];
-        int32_t sj = a.status[j];
-        if (0 < sj && sj <= pass) {
+        const int32_t j = a.nidx[int64_t(k) * a.npad + i];
+        const int32_t sj = a.status[j];
+        if (0 < sj && sj <= pass && (!a.bnd[j] || a.tags[j] == tag)) {
             double d2 = 0.0;
             for (int d = 0; d < a.D; ++d) {
                 double x = a.dist[(int64_t(k) * a.D + d) * a.npad + i];
@@ -487,6 +649,14 @@ __global__ void k_donor_pass(DonorArgs a, int pass) {
     }
 }
 
+// The source of every boundary particle's state: its donor's root under an outflow tag, else none.
+__global__ void k_boundary_sources(DonorArgs a) {
+    const int64_t q = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (q >= a.nb) return;
+    const int32_t i = a.blist[q];
+    a.bsrc[q] = a.outflow(a.tags[i]) ? a.root[i] : -1;
+}
+
 inline unsigned grid_for(int64_t n, int bs = HCC_BLOCK) { return unsigned((n + bs - 1) / bs); }
 
 }  // namespace
@@ -499,7 +669,17 @@ hcc_status mls_prepare(MlsArgs &a, cudaStream_t s, std::string &err) {
                                      : std::max(std::max(a.Bd, a.Br), a.D + 1);
     if (a.central_qmax > 0) need = std::max(need, basis_count(a.D, a.central_qmax) + 1);
     if (need > kMaxB) { err = "basis too large for the MLS kernel"; return HCC_ERR_UNSUPPORTED; }
-    if (need <= 4) k_mls<4><<<grid_for(a.n, 128), 128, 0, s>>>(a);
+    if (a.linear) {
+        const unsigned g = grid_for(a.n, 128);
+        auto run = [&](auto dim) {
+            constexpr int D = decltype(dim)::value;
+            if (a.gw32) k_mls_linear<D, true><<<g, 128, 0, s>>>(a);
+            else k_mls_linear<D, false><<<g, 128, 0, s>>>(a);
+        };
+        if (a.D == 1) run(std::integral_constant<int, 1>{});
+        else if (a.D == 2) run(std::integral_constant<int, 2>{});
+        else run(std::integral_constant<int, 3>{});
+    } else if (need <= 4) k_mls<4><<<grid_for(a.n, 128), 128, 0, s>>>(a);
     else if (need <= 10) k_mls<10><<<grid_for(a.n, 128), 128, 0, s>>>(a);
     else k_mls<kMaxB><<<grid_for(a.n, 64), 64, 0, s>>>(a);
     if (a.mw) k_mweights<<<grid_for(a.n, 128), 128, 0, s>>>(a);
@@ -514,12 +694,12 @@ hcc_status mls_prepare(MlsArgs &a, cudaStream_t s, std::string &err) {
     return HCC_OK;
 }
 
-hcc_status donor_map(DonorArgs &a, int tag, cudaStream_t s, std::string &err) {
-    if (a.n == 0) return HCC_OK;
-    // tag < 0: first call, roots of interior particles point at themselves, boundary roots are unresolved
-    k_donor_init<<<grid_for(a.n), HCC_BLOCK, 0, s>>>(a, tag, tag < 0 ? 1 : 0);
-    if (tag >= 0)
-        for (int pass = 1; pass <= 5; ++pass) k_donor_pass<<<grid_for(a.n), HCC_BLOCK, 0, s>>>(a, pass);
+hcc_status donor_map(DonorArgs &a, cudaStream_t s, std::string &err) {
+    if (a.n == 0 || a.nb == 0) return HCC_OK;
+    k_donor_init<<<grid_for(a.n), HCC_BLOCK, 0, s>>>(a);
+    if (a.outflow_tags)
+        for (int pass = 1; pass <= 5; ++pass) k_donor_pass<<<grid_for(a.nb, 64), 64, 0, s>>>(a, pass);
+    k_boundary_sources<<<grid_for(a.nb), HCC_BLOCK, 0, s>>>(a);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) { err = std::string("donor map: ") + cudaGetErrorString(e); return HCC_ERR_CUDA; }
     return HCC_OK;
