@@ -689,7 +689,6 @@ hcc_status mls_prepare(MlsArgs &a, cudaStream_t s, std::string &err) {
         else k_mls_central<kMaxB><<<grid_for(a.n, 64), 64, 0, s>>>(a, q);
     }
     cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) { err = std::string("mls kernel: ") + cudaGetErrorString(e); return HCC_ERR_CUDA; }
     return HCC_OK;
 }
