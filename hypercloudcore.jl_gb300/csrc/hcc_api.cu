@@ -1320,7 +1320,8 @@ hcc_status hcc_upload_cloud(hcc_ctx *c, int64_t n, const double *pos, const uint
     const size_t sb = size_t(np) * M * c->esz();
     HCC_TRY(c->reserve_bytes(c->rhos, sb, "rhos"));
     HCC_TRY(c->reserve_bytes(c->cand, sb, "candidate"));
-    HCC_TRY(c->reserve_bytes(c->grad, size_t(np) * c->Br * M * c->esz(), "gradients"));
+    const size_t gb = size_t(np) * grad_row_elements(c->Br * M, int(c->esz())) * c->esz();
+    HCC_TRY(c->reserve_bytes(c->grad, gb, "gradients"));
     HCC_TRY(c->reserve_bytes(c->xfer, size_t(np) * M * sizeof(double), "conversion buffer"));
     for (int s = 0; s < c->tab.s; ++s) {
         HCC_TRY(c->reserve_bytes(c->Y[s], sb, "stage states"));
@@ -1329,7 +1330,7 @@ hcc_status hcc_upload_cloud(hcc_ctx *c, int64_t n, const double *pos, const uint
         cudaMemsetAsync(c->KE[s], 0, sb, c->stream);
         cudaMemsetAsync(c->KI[s], 0, sb, c->stream);
     }
-    cudaMemsetAsync(c->grad, 0, size_t(np) * c->Br * M * c->esz(), c->stream);
+    cudaMemsetAsync(c->grad, 0, gb, c->stream);
     cudaMemsetAsync(c->rhos, 0, sb, c->stream);
     HCC_TRY(c->reserve(c->orders, np, "orders"));
     HCC_TRY(c->reserve(c->nbmin, np, "nbmin"));

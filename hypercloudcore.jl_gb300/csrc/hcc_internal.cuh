@@ -26,6 +26,9 @@
 #define HCC_FP32_PACKED 0          // FP32 stage kernels: 1 = packed FP32x2 instructions for component pairs (measured
                                    // slower than scalar instructions in the tile-staged 3-D flux pass)
 #endif
+#ifndef HCC_SPLIT_WIDE_TILES
+#define HCC_SPLIT_WIDE_TILES 304   // FP32 worklist passes: lists of up to this many tiles take a whole block a tile
+#endif
 #ifndef HCC_TILE_FLUX_PF
 #define HCC_TILE_FLUX_PF 8         // tile-staged flux pass: union places of a thread's slots fetched this many slots ahead
 #endif
@@ -107,6 +110,12 @@ __host__ __device__ __forceinline__ int divergence_index(int DO, int D, int p_or
     if (idx > base && 2 * num_nb < 3 * (basis_count(D, idx - 1) + 1)) idx = base;
     while (idx > 2 && num_nb < basis_count(D, idx - 1) + 1) idx -= 1;
     return idx;
+}
+
+// Elements of a particle's gradient row for n slope components of `bytes` each (padded to whole 16-byte groups from 12
+// components on; shorter rows are read by scalar loads and stay dense).
+__host__ __device__ constexpr int grad_row_elements(int n, int bytes) {
+    return n < 12 ? n : (n + 16 / bytes - 1) / (16 / bytes) * (16 / bytes);
 }
 
 // Compile-time exponent table of the MLS basis of degree Q in D variables (_generate_exponents,

@@ -125,15 +125,24 @@ template <> __device__ __forceinline__ double floatmin_of<double>() { return 2.2
 template <> __device__ __forceinline__ float floatmin_of<float>() { return 1.17549435e-38f; }
 
 // Arithmetic kernels of the two paths. FP64 (plain path): IEEE division and square root — the oracle's exact
-// sequence. FP32 (bulk path, compiled with denormals flushed to zero): the fast reciprocal and reciprocal square
-// root of the special-function unit (≤ 2 ulp; sqrt(x) = x rsqrt(x), 0 at 0, NaN below); its results are compared
+// sequence. FP32 (bulk path, compiled with denormals flushed to zero): the reciprocal (1 ulp) and square root (relative
+// error 2^-23; NaN below zero) of the special-function unit, one instruction each, where __fdividef and x rsqrt(x) took
+// several (a slot of the Euler flux pass takes three and two of them); its results are compared
 // with the FP64 oracle to tolerance. Both keep Julia's NaN-propagating min/max:
 // a reconstruction with negative pressure has a NaN sound speed, and the NaN must reach the candidate so that the
 // admissibility check flags it (fmaxf would drop it and keep the high order).
 template <typename T> __device__ __forceinline__ T recip(T x) { return T(1) / x; }
-template <> __device__ __forceinline__ float recip<float>(float x) { return __fdividef(1.0f, x); }
+template <> __device__ __forceinline__ float recip<float>(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
 template <typename T> __device__ __forceinline__ T root(T x) { return sqrt(x); }
-template <> __device__ __forceinline__ float root<float>(float x) { return x == 0.0f ? 0.0f : x * rsqrtf(x); }
+template <> __device__ __forceinline__ float root<float>(float x) {
+    float r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
 template <typename T> __device__ __forceinline__ T vmin(T x, T y) { return jmin(x, y); }
 template <typename T> __device__ __forceinline__ T vmax(T x, T y) { return jmax(x, y); }
 // FP32: the NaN-propagating forms of the min/max instructions (one instruction each)
@@ -203,6 +212,32 @@ template <> __device__ __forceinline__ bool positive<double>(double x) {
 // x or -x by the sign bit
 __device__ __forceinline__ double negate_if(double x, bool neg) {
     return __longlong_as_double(__double_as_longlong(x) ^ (neg ? (long long)0x8000000000000000ull : 0ll));
+}
+
+// Elements of a particle's gradient row for N slope components: rows of 12 or more that are not whole 16-byte groups
+// (3-D Euler: 15) are padded to them, so that a neighbour's row comes in 16-byte loads (four instead of fifteen).
+// hcc_internal.cuh's grad_row_elements is the host's form.
+template <typename T, int N> constexpr int grad_row() { return grad_row_elements(N, int(sizeof(T))); }
+// N elements of a 16-byte-aligned row of S >= N elements (S a multiple of the group, or S = N).
+template <typename T, int N, int S> __device__ __forceinline__ void load_row(const T *__restrict__ p, T *out) {
+    if constexpr (S == N) {
+        load_vec<T, N>(p, out);
+    } else {
+        T v[S];
+        load_vec<T, S>(p, v);
+#pragma unroll
+        for (int q = 0; q < N; ++q) out[q] = v[q];
+    }
+}
+template <typename T, int N, int S> __device__ __forceinline__ void store_row(T *__restrict__ p, const T *v) {
+    if constexpr (S == N) {
+        store_vec<T, N>(p, v);
+    } else {
+        T w[S];
+#pragma unroll
+        for (int q = 0; q < S; ++q) w[q] = q < N ? v[q < N ? q : 0] : T(0);
+        store_vec<T, S>(p, w);
+    }
 }
 
 // Euler primitives: inv_rho = 1/rho, u_d = m_d inv_rho, p = (gamma-1)(E - 0.5 (rho |u|^2)), c = sqrt(gamma p inv_rho).
@@ -483,7 +518,7 @@ __device__ __forceinline__ void gather_one(const StageArgs<T> &a, const int64_t 
     const int p0 = p;
     while (p > 1 && cnt < basis_count(D, p - 1)) --p;
     if (p < p0) a.orders[i] = int8_t(p);
-    T *g = a.grad + i * (BR * M);
+    T *g = a.grad + i * grad_row<T, BR * M>();
     T fi[M];
 #pragma unroll
     for (int m = 0; m < M; ++m) fi[m] = a.U[i * M + m];
@@ -670,24 +705,39 @@ __device__ __forceinline__ void gather_one(const StageArgs<T> &a, const int64_t 
         }
     }
     if (a.sc.limiter != HCC_LIMITER_NONE && p > 1) limit_slopes<T, D, M, RDEG>(a, i, cnt, fi, out);
-    store_vec<T, BR * M>(g, &out[0][0]);
+    store_row<T, BR * M, grad_row<T, BR * M>()>(g, &out[0][0]);
 }
 
-// FP32 degree-1 worklist pass of the reconstruction with four warps per tile: warp 0 lowers starved orders and picks
-// the path; on the cached gradient-weight path warp w sums the slots k = w, w + 4, ... and marks their neighbours'
-// reach, warp 0 adds the four partial sums in a fixed order, applies the limiter and stores the gradients; any
-// other particle is reconstructed whole by warp 0.
+// Warps of a block of the FP32 worklist passes, and how many of them share a tile of nt listed tiles. A tile's slots
+// are dealt to its warps, so a warp's serial chain (a dependent index -> state -> gradient load a slot, about 1.4 us
+// each at 66 slots in 3-D) is the slots over the warps. Short lists leave most SMs idle and take the whole block a
+// tile; longer ones keep four warps a tile, whose partial sums cost less to combine. The line depends on the list
+// alone, so results do not depend on the launch shape. States of 8 and more components keep blocks of four warps
+// (shared memory of their partial sums).
+template <int M> constexpr int split_warps() { return M >= 8 ? 4 : 16; }
+template <int M> __device__ __forceinline__ int split_share(unsigned nt) {
+    return split_warps<M>() > 4 && nt <= HCC_SPLIT_WIDE_TILES ? split_warps<M>() : 4;
+}
+
+// FP32 degree-1 worklist pass of the reconstruction with several warps per tile: the tile's first warp lowers starved
+// orders and picks the path; on the cached gradient-weight path warp w of W sums the slots k = w, w + W, ... and marks
+// their neighbours' reach, the first warp adds the partial sums in a fixed order, applies the limiter and stores the
+// gradients; any other particle is reconstructed whole by the first warp.
 template <typename T, int D, int M, int PDE, int RDEG>
-__global__ void __launch_bounds__(128) k_gather_tiles(const StageArgs<T> a) {
-    constexpr int BR = RBasis<D, RDEG>::B;
-    __shared__ T parts[4][32][BR * M];
-    __shared__ int path[32];
-    const int lane = int(threadIdx.x & 31), w = int(threadIdx.x >> 5);
+__global__ void __launch_bounds__(32 * split_warps<M>()) k_gather_tiles(const StageArgs<T> a) {
+    constexpr int BR = RBasis<D, RDEG>::B, NW = split_warps<M>();
+    __shared__ T parts[NW][32][BR * M];
+    __shared__ int path[NW / 4][32];
+    const int lane = int(threadIdx.x & 31), wb = int(threadIdx.x >> 5);
     const unsigned nt = *a.wcount;
+    const int W = split_share<M>(nt);              // warps per tile
+    const int group = wb / W, w = wb % W, first = group * W;
+    const unsigned step = unsigned(NW / W) * gridDim.x;
     const int64_t np = a.g.npad;
-    for (unsigned q = blockIdx.x; q < nt; q += gridDim.x) {
-        const int32_t tile = a.wtiles[q];
-        const uint32_t word = a.wmask[tile];
+    for (unsigned q0 = blockIdx.x * unsigned(NW / W); q0 < nt; q0 += step) {
+        const unsigned q = q0 + unsigned(group);
+        const int32_t tile = q < nt ? a.wtiles[q] : 0;
+        const uint32_t word = q < nt ? a.wmask[tile] : 0u;
         const int64_t i = int64_t(tile) * 32 + lane;
         const bool live = ((word >> lane) & 1u) && !a.g.bnd[i];
         const int cnt = live ? a.g.cnt[i] : 0;
@@ -700,10 +750,10 @@ __global__ void __launch_bounds__(128) k_gather_tiles(const StageArgs<T> a) {
                 if (p < p0) a.orders[i] = int8_t(p);
                 gp = (p == a.sc.max_order && p > 1 && a.g.ok_r[i] && a.g.gw) ? 1 : 0;
             }
-            path[lane] = gp;
+            path[group][lane] = gp;
         }
         __syncthreads();
-        const int gp = path[lane];
+        const int gp = path[group][lane];
         {
             // warp-uniform slot loop over every live member (the reach marks, combined across the warp); the
             // cached-fit members also accumulate their gradients here
@@ -714,7 +764,7 @@ __global__ void __launch_bounds__(128) k_gather_tiles(const StageArgs<T> a) {
             if (myc > 0) load_vec<T, M>(a.U + i * M, fi);
 #pragma unroll
             for (int b = 0; b < BR * M; ++b) out[b] = T(0);
-            for (int k = w; k < kw; k += 4) {
+            for (int k = w; k < kw; k += W) {
                 const int32_t j = k < myr ? a.g.nidx[int64_t(k) * np + i] : -1;
                 if (k < myc) {
                     T gk[D], df[M];
@@ -732,7 +782,7 @@ __global__ void __launch_bounds__(128) k_gather_tiles(const StageArgs<T> a) {
             }
             if (myc > 0 || (live && gp))
 #pragma unroll
-                for (int b = 0; b < BR * M; ++b) parts[w][lane][b] = out[b];
+                for (int b = 0; b < BR * M; ++b) parts[wb][lane][b] = out[b];
         }
         __syncthreads();
         if (w == 0 && a.rmask) reach_mark_warp(a.rmask, a.rtiles, a.rcount, live ? int32_t(i) : -1);
@@ -743,16 +793,18 @@ __global__ void __launch_bounds__(128) k_gather_tiles(const StageArgs<T> a) {
 #pragma unroll
                 for (int b = 0; b < BR; ++b)
 #pragma unroll
-                    for (int m = 0; m < M; ++m)
-                        out[b][m] = ((parts[0][lane][b * M + m] + parts[1][lane][b * M + m]) + parts[2][lane][b * M + m]) +
-                                    parts[3][lane][b * M + m];
+                    for (int m = 0; m < M; ++m) {
+                        T sm = parts[first][lane][b * M + m];
+                        for (int v = 1; v < W; ++v) sm = sm + parts[first + v][lane][b * M + m];
+                        out[b][m] = sm;
+                    }
                 if (a.sc.limiter != HCC_LIMITER_NONE) limit_slopes<T, D, M, RDEG>(a, i, cnt, fi, out);
-                store_vec<T, BR * M>(a.grad + i * (BR * M), &out[0][0]);
+                store_row<T, BR * M, grad_row<T, BR * M>()>(a.grad + i * grad_row<T, BR * M>(), &out[0][0]);
             } else {
                 gather_one<T, D, M, PDE, RDEG>(a, i);
             }
         }
-        if (threadIdx.x == 0 && a.clear_wmask) a.wmask[tile] = 0u;   // every lane read the word before the barrier
+        if (w == 0 && lane == 0 && q < nt && a.clear_wmask) a.wmask[tile] = 0u;   // every lane read the word before the barrier
         __syncthreads();
     }
 }
@@ -797,7 +849,7 @@ __global__ void __launch_bounds__(128) k_gather(const StageArgs<T> a) {
 // 1.5h comparable magnitudes, or are negligible; otherwise the candidate is flagged. A rare path (DMP violators only).
 template <typename T, int D, int M, int RDEG>
 __device__ __noinline__ bool u2_curvature_fails(const StageArgs<T> &a, int64_t i, const bool *viol) {
-    constexpr int BR = RBasis<D, RDEG>::B;
+    constexpr int GS = grad_row<T, RBasis<D, RDEG>::B * M>();
     const int cnt = a.g.cnt[i];
     const int64_t np = a.g.npad;
     const T h = a.u2_h, h2 = h * h, r15 = T(1.5) * h, near_sq = r15 * r15, dl = a.delta;
@@ -806,7 +858,7 @@ __device__ __noinline__ bool u2_curvature_fails(const StageArgs<T> &a, int64_t i
         T mini[M], maxi[M], minA[M], maxA[M];
 #pragma unroll
         for (int m = 0; m < M; ++m) {
-            const T ci = a.grad[(i * BR + b) * M + m];
+            const T ci = a.grad[i * GS + b * M + m];
             mini[m] = maxi[m] = ci;
             minA[m] = maxA[m] = fabs(ci);
         }
@@ -821,7 +873,7 @@ __device__ __noinline__ bool u2_curvature_fails(const StageArgs<T> &a, int64_t i
             const bool near = r2 <= near_sq;
 #pragma unroll
             for (int m = 0; m < M; ++m) {
-                const T cj = a.grad[(j * BR + b) * M + m];
+                const T cj = a.grad[j * GS + b * M + m];
                 mini[m] = vmin(mini[m], cj);
                 maxi[m] = vmax(maxi[m], cj);
                 if (near) { minA[m] = vmin(minA[m], fabs(cj)); maxA[m] = vmax(maxA[m], fabs(cj)); }
@@ -1183,11 +1235,13 @@ __device__ __forceinline__ void flux_slot(const StageArgs<T> &a, const T *fi, co
     }
 }
 
-// The flux pass of particle i over its slots k0, k0 + KSTEP, ... With KSTEP = 1 the whole pass and its epilogue;
-// with KSTEP > 1 (FP32) the partial sums and extrema go to `part` for the caller to combine.
-template <typename T, int D, int M, int PDE, int RDEG, bool ALE, int KSTEP = 1, bool MOM = false>
-__device__ __forceinline__ bool flux_one(const StageArgs<T> &a, const int64_t i, const int k0 = 0,
-                                         FluxPart<T, M> *part = nullptr, bool *rough = nullptr) {
+// The flux pass of particle i over its slots: the whole pass and its epilogue, or with SPLIT (FP32) the slots
+// k0, k0 + kstep, ..., whose partial sums and extrema go to `part` for the caller to combine.
+template <typename T, int D, int M, int PDE, int RDEG, bool ALE, bool SPLIT = false, bool MOM = false>
+__device__ __forceinline__ bool flux_one(const StageArgs<T> &a, const int64_t i, const int first_slot = 0,
+                                         const int split_step = 1, FluxPart<T, M> *part = nullptr,
+                                         bool *rough = nullptr) {
+    const int k0 = SPLIT ? first_slot : 0, kstep = SPLIT ? split_step : 1;
     constexpr int BR = RBasis<D, RDEG>::B;
     if (a.g.bnd[i]) {
         if (a.full) {
@@ -1205,7 +1259,8 @@ __device__ __forceinline__ bool flux_one(const StageArgs<T> &a, const int64_t i,
     (void)invL;
     T fi[M], gi[BR][M], Fi[D][M];
     load_vec<T, M>(a.U + i * M, fi);
-    load_vec<T, BR * M>(a.grad + i * (BR * M), &gi[0][0]);
+    constexpr int GS = grad_row<T, BR * M>();
+    load_row<T, BR * M, GS>(a.grad + i * GS, &gi[0][0]);
     // moving grid: this particle's grid velocity (K_X of the stage) and every flux in its frame
     T wv[D];
     const T *wp = nullptr;
@@ -1235,7 +1290,7 @@ __device__ __forceinline__ bool flux_one(const StageArgs<T> &a, const int64_t i,
         T fj[M];
         load_vec<T, M>(a.U + int64_t(j) * M, fj);
         T gj[BR * M];
-        load_vec<T, BR * M>(a.grad + int64_t(j) * (BR * M), gj);
+        load_row<T, BR * M, GS>(a.grad + int64_t(j) * GS, gj);
         if (need_ext) {
 #pragma unroll
             for (int m = 0; m < M; ++m) { mn[m] = vmin(mn[m], fj[m]); mx[m] = vmax(mx[m], fj[m]); }
@@ -1253,7 +1308,7 @@ __device__ __forceinline__ bool flux_one(const StageArgs<T> &a, const int64_t i,
     };
     // FP32 full passes: the slots in groups of UF, the next group's slot data in flight while this group is
     // computed (the slot body unrolled over the group); otherwise a one-deep software pipeline
-    constexpr int UF = (kFast && KSTEP == 1) ? HCC_FLUX_STREAM_GROUP : 1;
+    constexpr int UF = (kFast && !SPLIT) ? HCC_FLUX_STREAM_GROUP : 1;
     if (UF > 1 && wok && k0 < cnt) {
         int32_t jb[UF];
         T dkb[UF][D], wkb[UF][D];
@@ -1301,23 +1356,23 @@ __device__ __forceinline__ bool flux_one(const StageArgs<T> &a, const int64_t i,
             dkn[d] = a.g.dist[(int64_t(k0) * D + d) * np + i];
             wkn[d] = wsl[(int64_t(k0) * D + d) * np + i];
         }
-        for (int k = k0; k < cnt; k += KSTEP) {
+        for (int k = k0; k < cnt; k += kstep) {
             const int32_t j = jn;
             T dk[D], wk[D];
 #pragma unroll
             for (int d = 0; d < D; ++d) { dk[d] = dkn[d]; wk[d] = wkn[d]; }
-            if (k + KSTEP < cnt) {
-                jn = a.g.nidx[int64_t(k + KSTEP) * np + i];
+            if (k + kstep < cnt) {
+                jn = a.g.nidx[int64_t(k + kstep) * np + i];
 #pragma unroll
                 for (int d = 0; d < D; ++d) {
-                    dkn[d] = a.g.dist[(int64_t(k + KSTEP) * D + d) * np + i];
-                    wkn[d] = wsl[(int64_t(k + KSTEP) * D + d) * np + i];
+                    dkn[d] = a.g.dist[(int64_t(k + kstep) * D + d) * np + i];
+                    wkn[d] = wsl[(int64_t(k + kstep) * D + d) * np + i];
                 }
             }
             slot(j, dk, wk, k);
         }
     } else if (need_ext) {
-        for (int k = k0; k < cnt; k += KSTEP) {
+        for (int k = k0; k < cnt; k += kstep) {
             const int32_t j = a.g.nidx[int64_t(k) * np + i];
 #pragma unroll
             for (int m = 0; m < M; ++m) {
@@ -1327,7 +1382,7 @@ __device__ __forceinline__ bool flux_one(const StageArgs<T> &a, const int64_t i,
             }
         }
     }
-    if constexpr (KSTEP > 1) {
+    if constexpr (SPLIT) {
         static_assert(sizeof(T) == 4, "split tiles are the FP32 path");
 #pragma unroll
         for (int m = 0; m < M; ++m) {
@@ -1368,8 +1423,8 @@ __global__ void __launch_bounds__(HCC_FLUX_BLOCK, flux_min_blocks<T, D, M>()) k_
     if (a.full) {
         const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
         bool rough = false;
-        const bool f = (i < a.g.n) ? flux_one<T, D, M, PDE, RDEG, ALE, 1, MOM>(a, i, 0, nullptr,
-                                                                               a.rough_words ? &rough : nullptr)
+        const bool f = (i < a.g.n) ? flux_one<T, D, M, PDE, RDEG, ALE, false, MOM>(a, i, 0, 1, nullptr,
+                                                                                   a.rough_words ? &rough : nullptr)
                                    : false;
         if (a.check) tile_failures(a, i >> 5, f);
         if (a.rough_words) {
@@ -1384,46 +1439,50 @@ __global__ void __launch_bounds__(HCC_FLUX_BLOCK, flux_min_blocks<T, D, M>()) k_
         const int32_t tile = a.wtiles[q];
         const uint32_t word = a.wmask[tile];
         const int64_t i = int64_t(tile) * 32 + lane;
-        const bool f = ((word >> lane) & 1u) ? flux_one<T, D, M, PDE, RDEG, ALE, 1, MOM>(a, i) : false;
+        const bool f = ((word >> lane) & 1u) ? flux_one<T, D, M, PDE, RDEG, ALE, false, MOM>(a, i) : false;
         if (a.check) tile_failures(a, tile, f);
         if (lane == 0 && a.clear_wmask) a.wmask[tile] = 0u;
     }
 }
 
-// FP32 worklist pass with four warps per tile: warp w takes the slots k = w, w + 4, ... of every member of the tile
-// (a quarter of the serial slot chain, the latency that bounds the short worklist passes), warp 0 combines the four
-// compensated partial sums (Kahan over the partials, minus their compensations) and the extrema, and runs the
-// epilogue. One block per tile, block-stride over the list.
+// FP32 worklist pass with several warps per tile (split_share): warp w of W takes the slots k = w, w + W, ... of every
+// member of the tile (a share of the serial slot chain, the latency that bounds the short worklist passes), the tile's
+// first warp combines the compensated partial sums (Kahan over the partials, minus their compensations) and the
+// extrema, and runs the epilogue. Block-stride over the list.
 template <typename T, int D, int M, int PDE, int RDEG, bool ALE, bool MOM = false>
-__global__ void __launch_bounds__(128) k_flux_tiles(const StageArgs<T> a) {
-    __shared__ FluxPart<T, M> parts[4][32];
-    const int lane = int(threadIdx.x & 31), w = int(threadIdx.x >> 5);
+__global__ void __launch_bounds__(32 * split_warps<M>()) k_flux_tiles(const StageArgs<T> a) {
+    constexpr int NW = split_warps<M>();
+    __shared__ FluxPart<T, M> parts[NW][32];
+    const int lane = int(threadIdx.x & 31), wb = int(threadIdx.x >> 5);
     const unsigned nt = *a.wcount;
-    for (unsigned q = blockIdx.x; q < nt; q += gridDim.x) {
-        const int32_t tile = a.wtiles[q];
-        const uint32_t word = a.wmask[tile];
+    const int W = split_share<M>(nt);              // warps per tile
+    const int group = wb / W, w = wb % W, first = group * W;
+    const unsigned step = unsigned(NW / W) * gridDim.x;
+    for (unsigned q0 = blockIdx.x * unsigned(NW / W); q0 < nt; q0 += step) {
+        const unsigned q = q0 + unsigned(group);
+        const int32_t tile = q < nt ? a.wtiles[q] : 0;
+        const uint32_t word = q < nt ? a.wmask[tile] : 0u;
         const int64_t i = int64_t(tile) * 32 + lane;
         const bool live = ((word >> lane) & 1u) && !a.g.bnd[i];
-        if (live) flux_one<T, D, M, PDE, RDEG, ALE, 4, MOM>(a, i, w, &parts[w][lane]);
+        if (live) flux_one<T, D, M, PDE, RDEG, ALE, true, MOM>(a, i, w, W, &parts[wb][lane]);
         __syncthreads();
-        if (w == 0) {
+        if (w == 0 && q < nt) {
             bool f = false;
             if (live) {
                 T Kv[M], mn[M], mx[M], fi[M];
 #pragma unroll
                 for (int m = 0; m < M; ++m) {
                     T sm = T(0), cm = T(0), comp = T(0);
-                    mn[m] = parts[0][lane].mn[m];
-                    mx[m] = parts[0][lane].mx[m];
-#pragma unroll
-                    for (int v = 0; v < 4; ++v) {
-                        const T y = parts[v][lane].s[m] - cm;
+                    mn[m] = parts[first][lane].mn[m];
+                    mx[m] = parts[first][lane].mx[m];
+                    for (int v = 0; v < W; ++v) {
+                        const T y = parts[first + v][lane].s[m] - cm;
                         const T u = sm + y;
                         cm = (u - sm) - y;
                         sm = u;
-                        comp = comp + parts[v][lane].c[m];
-                        mn[m] = vmin(mn[m], parts[v][lane].mn[m]);
-                        mx[m] = vmax(mx[m], parts[v][lane].mx[m]);
+                        comp = comp + parts[first + v][lane].c[m];
+                        mn[m] = vmin(mn[m], parts[first + v][lane].mn[m]);
+                        mx[m] = vmax(mx[m], parts[first + v][lane].mx[m]);
                     }
                     Kv[m] = -(sm - comp);
                 }
@@ -1508,10 +1567,12 @@ template <int RW> constexpr int tile_stage_unroll() {
 
 template <int D, int M> constexpr int tile_gather_min_blocks() { return M >= 8 ? 1 : 3; }
 
-template <int D, int M, int PDE>
+// LIM: slope limiters, which go through gather_one. Without one, a particle off the cached fit (an order below the full
+// one, a failed fit) has zero slopes, and the kernel does without gather_one's registers.
+template <int D, int M, int PDE, bool LIM>
 __global__ void __launch_bounds__(2 * HCC_TILE, tile_gather_min_blocks<D, M>()) k_gather_tile(const StageArgs<float> a) {
     extern __shared__ __align__(16) float sm[];
-    constexpr int W = tile_gather_row<D, M>();
+    constexpr int W = tile_gather_row<D, M>(), GS = grad_row<float, D * M>();
     const int64_t t = blockIdx.x;
     {
         const int64_t u0 = a.tv.ustart[t];
@@ -1551,7 +1612,8 @@ __global__ void __launch_bounds__(2 * HCC_TILE, tile_gather_min_blocks<D, M>()) 
         cnt = a.g.cnt[i];
         int q = a.orders[i];
         while (q > 1 && cnt < basis_count(D, q - 1)) --q;
-        mode = (q == a.sc.max_order && q > 1 && a.g.ok_r[i] && a.sc.limiter == HCC_LIMITER_NONE) ? 1 : 2;
+        if (!LIM && h == 0 && q < a.orders[i]) a.orders[i] = int8_t(q);   // starved (gather_one lowers it itself)
+        mode = (q == a.sc.max_order && q > 1 && a.g.ok_r[i] && !LIM) ? 1 : 2;
     }
     float out[D][M];
 #pragma unroll
@@ -1565,12 +1627,6 @@ __global__ void __launch_bounds__(2 * HCC_TILE, tile_gather_min_blocks<D, M>()) 
         int qi[D];
 #pragma unroll
         for (int d = 0; d < D; ++d) qi[d] = __float_as_int(own[d]);
-        float G[D][D];
-        const float *cf = a.tv.coef + i * a.tv.cw + D + D * D;
-#pragma unroll
-        for (int b = 0; b < D; ++b)
-#pragma unroll
-            for (int c = 0; c < D; ++c) G[b][c] = cf[b * D + c];
         const float qt = a.tv.quantum[t], ws = a.tv.wscale;
         // this thread's slots h, h + 2, ...: their union places in groups of PF, the next group's loads in flight
         // while this group is summed
@@ -1599,19 +1655,14 @@ __global__ void __launch_bounds__(2 * HCC_TILE, tile_gather_min_blocks<D, M>()) 
 #pragma unroll
                 for (int d = 1; d < D; ++d) r2 = r2 + x[d] * x[d];
                 const float w = tile_weight(r2, ws);
-                float gk[D];
+                // the right-hand side of the fit, sum_k w_k x_k (f_j - f_i); the fit's rows are applied once at the end
 #pragma unroll
-                for (int b = 0; b < D; ++b) {
-                    float v = G[b][0] * x[0];
-#pragma unroll
-                    for (int c = 1; c < D; ++c) v = v + G[b][c] * x[c];
-                    gk[b] = w * v;
-                }
+                for (int d = 0; d < D; ++d) x[d] = w * x[d];
 #pragma unroll
                 for (int m = 0; m < M; ++m) {
                     const float dm = r[D + m] - own[D + m];
 #pragma unroll
-                    for (int b = 0; b < D; ++b) out[b][m] = out[b][m] + gk[b] * dm;
+                    for (int b = 0; b < D; ++b) out[b][m] = out[b][m] + x[b] * dm;
                 }
             }
 #pragma unroll
@@ -1626,13 +1677,21 @@ __global__ void __launch_bounds__(2 * HCC_TILE, tile_gather_min_blocks<D, M>()) 
     __syncthreads();
     if (h == 1) return;
     if (mode == 2) {
-        gather_one<float, D, M, PDE, 1>(a, i);
+        if constexpr (LIM) gather_one<float, D, M, PDE, 1>(a, i);
+        else store_row<float, D * M, GS>(a.grad + i * GS, &out[0][0]);
     } else if (mode == 1) {
+        const float *cf = a.tv.coef + i * a.tv.cw + D + D * D;
+        float g[D][M];
 #pragma unroll
         for (int b = 0; b < D; ++b)
 #pragma unroll
-            for (int m = 0; m < M; ++m) out[b][m] = out[b][m] + parts[pl * (D * M) + b * M + m];
-        store_vec<float, D * M>(a.grad + i * (D * M), &out[0][0]);
+            for (int m = 0; m < M; ++m) {
+                float v = 0.0f;
+#pragma unroll
+                for (int c = 0; c < D; ++c) v = v + cf[b * D + c] * (out[c][m] + parts[pl * (D * M) + c * M + m]);
+                g[b][m] = v;
+            }
+        store_row<float, D * M, GS>(a.grad + i * GS, &g[0][0]);
     }
 }
 
@@ -1640,11 +1699,13 @@ __global__ void __launch_bounds__(2 * HCC_TILE, tile_gather_min_blocks<D, M>()) 
 // compensated partial sums and extrema to shared memory, the first combines them and runs the epilogue.
 template <int D, int M> constexpr int tile_flux_min_blocks() { return M >= 8 ? 1 : 2; }
 
-template <int D, int M, int PDE>
+// PLAIN: EPD1 interface orders and the plain Rusanov flux (the usual configuration), known at compile time.
+template <int D, int M, int PDE, bool PLAIN>
 __global__ void __launch_bounds__(2 * HCC_TILE, tile_flux_min_blocks<D, M>()) k_flux_tile(const StageArgs<float> a) {
     extern __shared__ __align__(16) float sm[];
     constexpr int W = tile_flux_row<D, M>();
     constexpr int RW = M + D * M;                 // used words of a row: the state, then the gradient
+    constexpr int GS = grad_row<float, D * M>();
     const int64_t t = blockIdx.x;
     const int64_t u0 = a.tv.ustart[t];
     const int nu = int(a.tv.ustart[t + 1] - u0);
@@ -1702,8 +1763,7 @@ __global__ void __launch_bounds__(2 * HCC_TILE, tile_flux_min_blocks<D, M>()) k_
                 qq[u].w = a.orders[j];
 #pragma unroll
                 for (int m = 0; m < M; ++m) v[u][m] = a.U[j * M + m];
-#pragma unroll
-                for (int c = 0; c < D * M; ++c) v[u][M + c] = a.grad[j * (D * M) + c];
+                load_row<float, D * M, GS>(a.grad + j * GS, v[u] + M);
             }
 #pragma unroll
             for (int u = 0; u < SU; ++u) {
@@ -1760,10 +1820,10 @@ __global__ void __launch_bounds__(2 * HCC_TILE, tile_flux_min_blocks<D, M>()) k_
                 }
                 const int oj_own = qj4.w;
                 int oi, oj;
-                if (a.sc.strategy == HCC_EPD1) { oi = oj = (oi_own < oj_own ? oi_own : oj_own); }
+                if (PLAIN || a.sc.strategy == HCC_EPD1) { oi = oj = (oi_own < oj_own ? oi_own : oj_own); }
                 else { oi = oi_own; oj = oj_own; }
-                const bool below = a.sc.aligned && (a.sc.max_order == 1 || oi_own < a.sc.max_order ||
-                                                    oj_own < a.sc.max_order);
+                const bool below = !PLAIN && a.sc.aligned && (a.sc.max_order == 1 || oi_own < a.sc.max_order ||
+                                                              oj_own < a.sc.max_order);
                 flux_slot<float, D, M, PDE, 1, false, false>(a, fi, gi, Fi, nullptr, r, r + M, oi, oj, below, dk,
                                                              wk, blk, i, k);
             };
@@ -2521,16 +2581,13 @@ __global__ void k_stage1(const StageArgs<T> a) {
     const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= a.g.n) return;
     T Y[M];
-#pragma unroll
-    for (int m = 0; m < M; ++m) Y[m] = a.Un[i * M + m];
+    load_vec<T, M>(a.Un + i * M, Y);
     if (!a.g.bnd[i] && a.implicit_mode) {
         T KIo[M];
         implicit_part<T, D, M, PDE>(a, i, Y, KIo);
-#pragma unroll
-        for (int m = 0; m < M; ++m) a.KInext[i * M + m] = KIo[m];
+        store_vec<T, M>(a.KInext + i * M, KIo);
     }
-#pragma unroll
-    for (int m = 0; m < M; ++m) a.Ynext[i * M + m] = Y[m];
+    store_vec<T, M>(a.Ynext + i * M, Y);
 }
 
 // Spacing of the speed table's rows: whole vectors.
@@ -3119,6 +3176,10 @@ struct StageInst {
         const unsigned g = grid(n, bs);
         return a.full ? g : std::max(1u, std::min(g, unsigned(a.list_blocks)));
     }
+    // blocks of an FP32 split worklist pass (list_blocks counts blocks of four warps)
+    static unsigned split_grid(const StageArgs<T> &a) {
+        return std::max(1u, unsigned(a.list_blocks) * 4u / unsigned(split_warps<M>()));
+    }
     // block of a full pass of the other flux-like schemes (the tuned flux block); worklist passes keep 128
     static int fbs(const StageArgs<T> &a) { return a.full ? a.flux_block : 128; }
     static void gather(const void *args, int64_t n, cudaStream_t s) {
@@ -3127,15 +3188,21 @@ struct StageInst {
             if (a.full && a.tile) {   // FP32 full pass with tile tables: neighbours staged in shared memory
                 static bool attr = false;
                 if (!attr) {
-                    cudaFuncSetAttribute(k_gather_tile<D, M, PDE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         tile_smem_optin());
+                    cudaFuncSetAttribute(k_gather_tile<D, M, PDE, true>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, tile_smem_optin());
+                    cudaFuncSetAttribute(k_gather_tile<D, M, PDE, false>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, tile_smem_optin());
                     attr = true;
                 }
-                k_gather_tile<D, M, PDE><<<unsigned(a.tv.ntiles), 2 * HCC_TILE, tile_gather_smem<D, M>(a.tv.umax), s>>>(a);
+                const size_t smem = tile_gather_smem<D, M>(a.tv.umax);
+                if (a.sc.limiter != HCC_LIMITER_NONE)
+                    k_gather_tile<D, M, PDE, true><<<unsigned(a.tv.ntiles), 2 * HCC_TILE, smem, s>>>(a);
+                else
+                    k_gather_tile<D, M, PDE, false><<<unsigned(a.tv.ntiles), 2 * HCC_TILE, smem, s>>>(a);
                 return;
             }
-            if (!a.full) {   // FP32 degree-1 worklist pass: split tiles (four warps a tile)
-                k_gather_tiles<T, D, M, PDE, RDEG><<<std::max(1u, unsigned(a.list_blocks)), 128, 0, s>>>(a);
+            if (!a.full) {   // FP32 degree-1 worklist pass: split tiles
+                k_gather_tiles<T, D, M, PDE, RDEG><<<split_grid(a), 32 * split_warps<M>(), 0, s>>>(a);
                 return;
             }
         }
@@ -3145,9 +3212,9 @@ struct StageInst {
     template <bool MOM> static void flux_mom(const StageArgs<T> &a, int64_t n, cudaStream_t s) {
         if constexpr (sizeof(T) == 4) {
             if (!a.full) {
-                const unsigned g = std::max(1u, unsigned(a.list_blocks));
-                if (a.mover) k_flux_tiles<T, D, M, PDE, RDEG, true, MOM><<<g, 128, 0, s>>>(a);
-                else k_flux_tiles<T, D, M, PDE, RDEG, false, MOM><<<g, 128, 0, s>>>(a);
+                const unsigned g = split_grid(a), nth = 32 * split_warps<M>();
+                if (a.mover) k_flux_tiles<T, D, M, PDE, RDEG, true, MOM><<<g, nth, 0, s>>>(a);
+                else k_flux_tiles<T, D, M, PDE, RDEG, false, MOM><<<g, nth, 0, s>>>(a);
                 return;
             }
         }
@@ -3169,18 +3236,25 @@ struct StageInst {
                 if (a.full && a.tile) {   // full pass with tile tables: neighbours staged in shared memory
                     static bool attr = false;
                     if (!attr) {
-                        cudaFuncSetAttribute(k_flux_tile<D, M, PDE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             tile_smem_optin());
-                        attr = true;
+                        cudaFuncSetAttribute(k_flux_tile<D, M, PDE, true>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, tile_smem_optin());
+                        cudaFuncSetAttribute(k_flux_tile<D, M, PDE, false>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, tile_smem_optin());
                     }
-                    k_flux_tile<D, M, PDE><<<unsigned(a.tv.ntiles), 2 * HCC_TILE, tile_flux_smem<D, M>(a.tv.umax), s>>>(a);
+                    const bool plain = a.sc.strategy == HCC_EPD1 && !a.sc.aligned;
+                    const size_t smem = tile_flux_smem<D, M>(a.tv.umax);
+                    if (plain)
+                        k_flux_tile<D, M, PDE, true><<<unsigned(a.tv.ntiles), 2 * HCC_TILE, smem, s>>>(a);
+                    else
+                        k_flux_tile<D, M, PDE, false><<<unsigned(a.tv.ntiles), 2 * HCC_TILE, smem, s>>>(a);
+                    attr = true;
                     return;
                 }
             }
-            if (!a.full) {   // FP32 worklist pass: split tiles (four warps a tile)
-                const unsigned g = std::max(1u, unsigned(a.list_blocks));
-                if (a.mover) k_flux_tiles<T, D, M, PDE, RDEG, true><<<g, 128, 0, s>>>(a);
-                else k_flux_tiles<T, D, M, PDE, RDEG, false><<<g, 128, 0, s>>>(a);
+            if (!a.full) {   // FP32 worklist pass: split tiles
+                const unsigned g = split_grid(a), nth = 32 * split_warps<M>();
+                if (a.mover) k_flux_tiles<T, D, M, PDE, RDEG, true><<<g, nth, 0, s>>>(a);
+                else k_flux_tiles<T, D, M, PDE, RDEG, false><<<g, nth, 0, s>>>(a);
                 return;
             }
         }
