@@ -221,6 +221,7 @@ struct hcc_ctx {
     uint8_t *trig_step = nullptr, *inadm = nullptr;
     // MOOD tile worklists (failed candidates, changed orders, their reach): tile lists and member words
     int32_t *ttiles = nullptr, *ctiles = nullptr, *dtiles = nullptr, *ftiles = nullptr;
+    int32_t *dlist = nullptr;                    // the particles of the reach
     uint32_t *tmask = nullptr, *cmask = nullptr, *dmask = nullptr, *words1 = nullptr, *fmask = nullptr;
     int32_t *forced = nullptr;                    // StrictEPD0 order offers (0x7f7f7f7f: none)
     ListCounts *lcounts = nullptr, *h_lcounts = nullptr;
@@ -403,7 +404,7 @@ struct hcc_ctx {
             for (void **p : {&Y[s], &KE[s], &KI[s]}) { if (*p) cudaFree(*p); *p = nullptr; }
         dfree(orders); dfree(nbmin); dfree(trig_step); dfree(inadm);
         dfree(ttiles); dfree(ctiles); dfree(dtiles); dfree(tmask); dfree(cmask); dfree(dmask); dfree(words1);
-        dfree(ftiles); dfree(fmask); dfree(forced);
+        dfree(ftiles); dfree(fmask); dfree(forced); dfree(dlist);
         dfree(shep_S); dfree(shep_V); dfree(shep_part);
     }
     void free_slots() {
@@ -734,14 +735,16 @@ template <typename T> int enqueue_recompute(hcc_ctx *c, const StageArgs<T> &a, c
         ga.rmask = c->dmask;
         ga.rtiles = c->dtiles;
         ga.rcount = &c->lcounts->d;
+        ga.rlist = c->f32 ? nullptr : c->dlist;
+        ga.rlcount = &c->lcounts->dp;
         if (prof) c->prof_begin(2);
         c->ops->gather(&ga, n, st);
         if (prof) c->prof_end();
         ++k;
     }
     if (hops == 2) {
-        launch_reach_hop2(c->lcounts, c->dtiles, c->dtiles, c->dmask, c->words1, c->cnt, c->nidx, c->npad,
-                          c->list_blocks, st);
+        launch_reach_hop2(c->lcounts, c->dtiles, c->dtiles, c->dmask, c->words1, c->f32 ? nullptr : c->dlist, c->cnt, c->nidx,
+                          c->npad, c->list_blocks, st);
         launch_nbmin(c->orders, c->nbmin, c->cnt, c->nidx, n, c->npad, c->dtiles, c->words1, &c->lcounts->d1,
                      c->list_blocks, st);
         k += 3;
@@ -749,7 +752,8 @@ template <typename T> int enqueue_recompute(hcc_ctx *c, const StageArgs<T> &a, c
     StageArgs<T> fa = a;
     fa.full = 0;
     fa.wtiles = hops > 0 ? c->dtiles : c->ctiles;
-    fa.wcount = hops > 0 ? &c->lcounts->d : &c->lcounts->c;
+    fa.wlist = c->dlist;
+    fa.wcount = hops == 0 ? &c->lcounts->c : c->f32 ? &c->lcounts->d : &c->lcounts->dp;
     fa.wmask = hops > 0 ? c->dmask : c->cmask;
     fa.clear_wmask = 1;
     if (prof) c->prof_begin(2);
@@ -1340,6 +1344,7 @@ hcc_status hcc_upload_cloud(hcc_ctx *c, int64_t n, const double *pos, const uint
     }
     const int64_t ntiles = np / 32;
     for (int32_t **p : {&c->ttiles, &c->ctiles, &c->dtiles, &c->ftiles}) HCC_TRY(c->reserve(*p, ntiles, "MOOD tile lists"));
+    if (!c->f32) HCC_TRY(c->reserve(c->dlist, np, "MOOD reach"));
     HCC_TRY(c->reserve(c->forced, np, "StrictEPD0 offers"));
     cudaMemsetAsync(c->forced, 0x7f, size_t(np) * sizeof(int32_t), c->stream);
     for (uint32_t **p : {&c->tmask, &c->cmask, &c->dmask, &c->words1, &c->fmask}) {

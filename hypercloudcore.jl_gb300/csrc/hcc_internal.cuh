@@ -29,6 +29,15 @@
 #ifndef HCC_SPLIT_WIDE_TILES
 #define HCC_SPLIT_WIDE_TILES 304   // FP32 worklist passes: lists of up to this many tiles take a whole block a tile
 #endif
+#ifndef HCC_SPLIT64_FLUX
+#define HCC_SPLIT64_FLUX 24000     // FP64 full flux passes of clouds up to this size: eight lanes a particle
+#endif
+#ifndef HCC_SPLIT64_GATHER
+#define HCC_SPLIT64_GATHER 24000   // FP64 full reconstruction passes likewise
+#endif
+#ifndef HCC_SPLIT64_LIST
+#define HCC_SPLIT64_LIST 400000    // FP64 worklist flux passes of clouds up to this size (their reach is a fraction of it)
+#endif
 #ifndef HCC_TILE_FLUX_PF
 #define HCC_TILE_FLUX_PF 8         // tile-staged flux pass: union places of a thread's slots fetched this many slots ahead
 #endif
@@ -324,8 +333,11 @@ template <typename T> struct StageArgs {
     uint32_t *wmask;
     int clear_wmask;                  // flux pass over the reach: clear each tile's word once read
     uint32_t *rmask;                  // gather pass over the changed orders: the reach of its members (the member
-    int32_t *rtiles;                  // and its neighbours) is marked here, each tile listed once
+    int32_t *rtiles;                  // and its neighbours) is marked here, each tile listed once ...
     unsigned *rcount;
+    int32_t *rlist;                   // ... and each particle (FP64)
+    unsigned *rlcount;
+    const int32_t *wlist;             // FP64 flux worklist pass over the reach: its particles
     int list_blocks;                  // grid of a worklist pass (warp-stride over the tiles)
     int flux_block, gather_block;     // block sizes of the full flux / gather passes (multiples of 32, <= 128)
     // epilogue: next candidate (Y_{s+1} or the final state) and the MOOD check of checkpoint s+1
@@ -379,7 +391,8 @@ __device__ __forceinline__ const StageCoeffs<T> *coef_of(const StageArgs<T> &a, 
 // changed orders (one or two hops), d1 = its one-hop part; done = blocks finished in the decrement launch; f = tiles
 // offered a lower order by StrictEPD0 forcing.
 struct ListCounts {
-    unsigned t, c, cn, d, d1, done, f, pad1;
+    unsigned t, c, cn, d, d1, done, f;
+    unsigned dp;                      // particles of the reach (FP64)
 };
 
 // Append v to a device list; warp-aggregated: one atomic per group of converged lanes.
@@ -402,20 +415,34 @@ __device__ __forceinline__ void reach_mark(uint32_t *mask, int32_t *tiles, unsig
 }
 
 // reach_mark for a whole warp (all 32 lanes call it; j < 0: no mark): lanes whose particles share a tile combine their
-// bits first, one atomic per distinct tile word, and the newly listed tiles are appended together.
-__device__ __forceinline__ void reach_mark_warp(uint32_t *mask, int32_t *tiles, unsigned *count, int32_t j) {
+// bits first, one atomic per distinct tile word; the newly listed tiles are appended together, and so are the newly
+// marked particles where a list of them is kept (FP64 contexts).
+__device__ __forceinline__ void reach_mark_warp(uint32_t *mask, int32_t *tiles, unsigned *count, int32_t *list,
+                                                unsigned *lcount, int32_t j) {
     const int lane = int(threadIdx.x & 31);
     const int32_t t = j >= 0 ? (j >> 5) : -1;
     const unsigned grp = __match_any_sync(0xffffffffu, t);
     const unsigned bits = __reduce_or_sync(grp, j >= 0 ? (1u << (j & 31)) : 0u);
-    bool fresh = false;
-    if (lane == __ffs(grp) - 1 && t >= 0) fresh = atomicOr(&mask[t], bits) == 0u;
-    const unsigned nb = __ballot_sync(0xffffffffu, fresh);
+    unsigned old = 0xffffffffu;
+    if (lane == __ffs(grp) - 1 && t >= 0) old = atomicOr(&mask[t], bits);
+    const unsigned nb = __ballot_sync(0xffffffffu, old == 0u);
     if (nb) {
         unsigned base = 0;
         if (lane == 0) base = atomicAdd(count, unsigned(__popc(nb)));
         base = __shfl_sync(0xffffffffu, base, 0);
-        if (fresh) tiles[base + unsigned(__popc(nb & ((1u << lane) - 1u)))] = t;
+        if (old == 0u) tiles[base + unsigned(__popc(nb & ((1u << lane) - 1u)))] = t;
+    }
+    if (!list) return;
+    // a particle is new when its bit was clear in its tile's old word and no lower lane of the warp names it
+    const unsigned was = __shfl_sync(0xffffffffu, old, __ffs(grp) - 1);
+    const unsigned same = __match_any_sync(0xffffffffu, j);
+    const bool add = j >= 0 && !((was >> (j & 31)) & 1u) && lane == __ffs(same) - 1;
+    const unsigned na = __ballot_sync(0xffffffffu, add);
+    if (na) {
+        unsigned base = 0;
+        if (lane == 0) base = atomicAdd(lcount, unsigned(__popc(na)));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (add) list[base + unsigned(__popc(na & ((1u << lane) - 1u)))] = j;
     }
 }
 
@@ -539,7 +566,7 @@ void launch_bc_apply(void *Y, const void *rhos, const int32_t *blist, const int3
 // Second hop of the reach (EPD2): d1 = the one-hop tiles and their words (copied to words1), then the neighbours
 // of their members are marked; the neighbourhood minimum of the orders over the one-hop members.
 void launch_reach_hop2(ListCounts *counts, const int32_t *dtiles, int32_t *dtiles_out, uint32_t *dmask,
-                       uint32_t *words1, const int32_t *cnt, const int32_t *nidx, int64_t npad, int blocks,
+                       uint32_t *words1, int32_t *dlist, const int32_t *cnt, const int32_t *nidx, int64_t npad, int blocks,
                        cudaStream_t s);
 // Neighbourhood minimum of the orders: every particle (tiles == nullptr) or the members of the tiles.
 void launch_nbmin(const int8_t *orders, int8_t *nbmin, const int32_t *cnt, const int32_t *nidx, int64_t n,
@@ -596,7 +623,7 @@ struct DropArgs {
     int8_t *orders;
     uint8_t *trig_step;
     const int32_t *ttiles;
-    const uint32_t *tmask;
+    uint32_t *tmask;
     int32_t *ctiles;
     uint32_t *cmask;
     ListCounts *counts;

@@ -778,14 +778,14 @@ __global__ void __launch_bounds__(32 * split_warps<M>()) k_gather_tiles(const St
                         for (int b = 0; b < BR; ++b) out[b * M + m] = out[b * M + m] + gk[b] * dm;
                     }
                 }
-                if (a.rmask) reach_mark_warp(a.rmask, a.rtiles, a.rcount, j);
+                if (a.rmask) reach_mark_warp(a.rmask, a.rtiles, a.rcount, a.rlist, a.rlcount, j);
             }
             if (myc > 0 || (live && gp))
 #pragma unroll
                 for (int b = 0; b < BR * M; ++b) parts[wb][lane][b] = out[b];
         }
         __syncthreads();
-        if (w == 0 && a.rmask) reach_mark_warp(a.rmask, a.rtiles, a.rcount, live ? int32_t(i) : -1);
+        if (w == 0 && a.rmask) reach_mark_warp(a.rmask, a.rtiles, a.rcount, a.rlist, a.rlcount, live ? int32_t(i) : -1);
         if (w == 0 && live) {
             if (gp) {
                 T fi[M], out[BR][M];
@@ -832,11 +832,11 @@ __global__ void __launch_bounds__(128) k_gather(const StageArgs<T> a) {
         if (mem) gather_one<T, D, M, PDE, RDEG>(a, i);
         if (a.rmask) {
             // the reach (members and their neighbours), slot by slot across the warp with combined atomics
-            reach_mark_warp(a.rmask, a.rtiles, a.rcount, mem ? i : -1);
+            reach_mark_warp(a.rmask, a.rtiles, a.rcount, a.rlist, a.rlcount, mem ? i : -1);
             const int c = mem ? a.g.cnt[i] : 0;
             const int kw = __reduce_max_sync(0xffffffffu, c);
             for (int k = 0; k < kw; ++k)
-                reach_mark_warp(a.rmask, a.rtiles, a.rcount, k < c ? a.g.nidx[int64_t(k) * np + i] : -1);
+                reach_mark_warp(a.rmask, a.rtiles, a.rcount, a.rlist, a.rlcount, k < c ? a.g.nidx[int64_t(k) * np + i] : -1);
         }
     }
 }
@@ -1032,6 +1032,15 @@ template <typename T, int D, int M> constexpr int flux_min_blocks() {
 // Partial sums of a particle's slots handled by one warp of a split tile (FP32 worklist passes).
 template <typename T, int M> struct FluxPart {
     T s[M], c[M], mn[M], mx[M];
+};
+
+// A slot's term on its own (the ordered split adds it later).
+template <int M> struct SlotTerm {
+    double t[M];
+    __device__ __forceinline__ void add(const double *x) {
+#pragma unroll
+        for (int m = 0; m < M; ++m) t[m] = x[m];
+    }
 };
 
 // One slot k of the flux pass of particle i (the MUSCL functor's slot body, MUSCL.jl:463-508): interface orders oi,
@@ -1415,8 +1424,17 @@ template <typename T> __device__ __forceinline__ void tile_failures(const StageA
     }
 }
 
-// A full pass (one thread per particle) or a worklist pass over tiles (one warp per tile, the members of its word;
-// the reach marks are cleared once read). Either way each warp reports the failed candidates of its tile.
+// Failed candidates of a warp of particles from anywhere (i: this lane's particle): their bits, and each tile once. The
+// words are clear between passes (k_drop_decide clears those it reads).
+template <typename T> __device__ __forceinline__ void list_failures(const StageArgs<T> &a, int64_t i, bool f) {
+    if (f && atomicOr(&a.tmask[i >> 5], 1u << (i & 31)) == 0u) list_append(a.ttiles, a.tcount, int32_t(i >> 5));
+}
+
+// A full pass (one thread per particle; each warp reports the failed candidates of its tile) or an FP64 worklist pass over
+// the particles of the reach, 32 to a warp. The members of a listed tile are few of its 32 (7 to 9 around the extrema of
+// a smooth field, 22 around a front), and a warp instruction of the FP64 unit costs the same for any number of them. (The
+// FP32 worklist pass, k_flux_tiles, keeps the tiles: it gains less from full warps than it loses to scattered slot
+// loads.) The reach marks are cleared once read.
 template <typename T, int D, int M, int PDE, int RDEG, bool ALE, bool MOM = false>
 __global__ void __launch_bounds__(HCC_FLUX_BLOCK, flux_min_blocks<T, D, M>()) k_flux(const StageArgs<T> a) {
     const int lane = int(threadIdx.x & 31);
@@ -1433,15 +1451,215 @@ __global__ void __launch_bounds__(HCC_FLUX_BLOCK, flux_min_blocks<T, D, M>()) k_
         }
         return;
     }
-    const unsigned nt = *a.wcount;
-    const unsigned warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (unsigned q = warp; q < nt; q += nwarps) {
-        const int32_t tile = a.wtiles[q];
-        const uint32_t word = a.wmask[tile];
-        const int64_t i = int64_t(tile) * 32 + lane;
-        const bool f = ((word >> lane) & 1u) ? flux_one<T, D, M, PDE, RDEG, ALE, false, MOM>(a, i) : false;
-        if (a.check) tile_failures(a, tile, f);
-        if (lane == 0 && a.clear_wmask) a.wmask[tile] = 0u;
+    const unsigned nm = *a.wcount;
+    const unsigned first = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+    for (unsigned q = first; q < nm; q += step) {
+        const int64_t i = a.wlist[q];
+        if (a.clear_wmask) a.wmask[i >> 5] = 0u;
+        const bool f = flux_one<T, D, M, PDE, RDEG, ALE, false, MOM>(a, i);
+        if (a.check) list_failures(a, i, f);
+    }
+}
+
+// ----------------------------------------------------------------------------------- ordered slot split (FP64)
+// FP64 passes of small clouds and short worklists: eight lanes share a particle. Lane h computes the terms of the slots
+// h, h + 8, ... and leaves them in shared memory, and the lanes then add the round's terms in slot order, one component
+// each, so every sum has the order of the one-thread pass and the result its bits. A warp instruction occupies the FP64
+// unit for 16 cycles and its result is some 40 cycles away, so the one-thread pass wants about four warps an SM
+// (20,000 particles on 152 SMs) before the unit is busy rather than the chain of one slot after another.
+constexpr int kSplit64 = 8;
+
+// Adds the round's terms (term[lane * E + e] of the slots k0 ... k0 + 7 of the warp's four particles) to this lane's
+// share of the sums: entry h + 8 j in sum[j].
+template <int E>
+__device__ __forceinline__ void ordered_round(const double *term, int lane, int k0, int cnt, double *sum) {
+    const int h = lane % kSplit64, g = lane - h;
+#pragma unroll
+    for (int j = 0; j < (E + kSplit64 - 1) / kSplit64; ++j) {
+        const int e = h + kSplit64 * j;
+        if (e < E) {
+#pragma unroll
+            for (int q = 0; q < kSplit64; ++q)
+                if (k0 + q < cnt) sum[j] = sum[j] + term[(g + q) * E + e];
+        }
+    }
+}
+// The particle of this lane's group in entry `g` of a full pass (every particle) or a worklist pass, or -1.
+template <typename T> __device__ __forceinline__ int64_t split_particle(const StageArgs<T> &a, unsigned g, unsigned count) {
+    return g < count ? (a.full ? int64_t(g) : int64_t(a.wlist[g])) : -1;
+}
+
+// flux_one with the slots shared by eight lanes (no moment correction, no marks for the predictor).
+template <int D, int M, int PDE, int RDEG, bool ALE>
+__global__ void __launch_bounds__(128) k_flux_split(const StageArgs<double> a) {
+    constexpr int BR = RBasis<D, RDEG>::B, GS = grad_row<double, BR * M>();
+    __shared__ double terms[4][32 * M];
+    double *term = terms[threadIdx.x >> 5];
+    const int lane = int(threadIdx.x & 31), h = lane % kSplit64;
+    const int64_t np = a.g.npad;
+    const unsigned count = a.full ? unsigned(a.g.n) : *a.wcount;
+    const unsigned step = gridDim.x * blockDim.x / kSplit64;
+    const bool need_ext = a.check && (a.sc.criterion == HCC_MOOD_U1 || a.sc.criterion == HCC_MOOD_U2);
+    for (unsigned g0 = (blockIdx.x * blockDim.x + threadIdx.x - lane) / kSplit64; g0 < count; g0 += step) {
+        const int64_t i = split_particle(a, g0 + unsigned(lane / kSplit64), count);
+        const bool bnd = i >= 0 && a.g.bnd[i];
+        const bool live = i >= 0 && !bnd;
+        if (bnd && a.full && h == 0) {
+#pragma unroll
+            for (int m = 0; m < M; ++m) a.K[i * M + m] = 0.0;
+            if (ALE)
+#pragma unroll
+                for (int d = 0; d < D; ++d) a.KXout[int64_t(d) * np + i] = 0.0;
+        }
+        const int cnt = live ? a.g.cnt[i] : 0;
+        double fi[M], gi[BR][M], Fi[D][M], wv[D], mn[M], mx[M], sum[1] = {0.0};
+        const double *wp = nullptr, *wsl = nullptr;
+        bool wok = false;
+        int oi_own = 1, nbmin_i = 0;
+        if (live) {
+            load_vec<double, M>(a.U + i * M, fi);
+            load_row<double, BR * M, GS>(a.grad + i * GS, &gi[0][0]);
+            if constexpr (ALE) {
+                grid_velocity<double, D, M, PDE>(a, i, fi, wv);
+                wp = wv;
+                if (h == 0)
+#pragma unroll
+                    for (int d = 0; d < D; ++d) a.KXout[int64_t(d) * np + i] = wv[d];
+            }
+            own_flux<double, D, M, PDE, ALE, false>(a.ph, fi, Fi, wp);
+            oi_own = a.orders[i];
+            const int didx = divergence_index(a.sc.DO, D, oi_own, cnt);
+            const bool cached = a.g.ok_d[i] && didx == divergence_index(a.sc.DO, D, a.sc.max_order, cnt);
+            wsl = cached ? a.g.dw : a.g.dw1;
+            wok = cnt > 0 && (cached || (a.g.dw1 != nullptr && didx == 2 && a.g.ok_1[i]));
+            if (a.sc.strategy == HCC_EPD2) nbmin_i = a.nbmin[i];
+#pragma unroll
+            for (int m = 0; m < M; ++m) { mn[m] = fi[m]; mx[m] = fi[m]; }
+        }
+        const int kw = __reduce_max_sync(0xffffffffu, cnt);
+        for (int k0 = 0; k0 < kw; k0 += kSplit64) {
+            const int k = k0 + h;
+            if (k < cnt) {
+                const int64_t j = a.g.nidx[int64_t(k) * np + i];
+                double fj[M];
+                load_vec<double, M>(a.U + j * M, fj);
+                if (need_ext) {
+#pragma unroll
+                    for (int m = 0; m < M; ++m) { mn[m] = vmin(mn[m], fj[m]); mx[m] = vmax(mx[m], fj[m]); }
+                }
+                if (wok) {
+                    double gj[BR * M], dk[D], wk[D];
+                    load_row<double, BR * M, GS>(a.grad + j * GS, gj);
+#pragma unroll
+                    for (int d = 0; d < D; ++d) {
+                        dk[d] = a.g.dist[(int64_t(k) * D + d) * np + i];
+                        wk[d] = wsl[(int64_t(k) * D + d) * np + i];
+                    }
+                    const int oj_own = a.orders[j];
+                    int oi = oi_own, oj = oj_own;
+                    if (a.sc.strategy == HCC_EPD1) oi = oj = (oi_own < oj_own ? oi_own : oj_own);
+                    else if (a.sc.strategy == HCC_EPD2) { const int nj = a.nbmin[j]; oi = oj = (nbmin_i < nj ? nbmin_i : nj); }
+                    const bool below = a.sc.aligned && (a.sc.max_order == 1 || oi_own < a.sc.max_order ||
+                                                        oj_own < a.sc.max_order);
+                    SlotTerm<M> t;
+                    flux_slot<double, D, M, PDE, RDEG, ALE, false>(a, fi, gi, Fi, wp, fj, gj, oi, oj, below, dk, wk, t,
+                                                                   i, k);
+#pragma unroll
+                    for (int m = 0; m < M; ++m) term[lane * M + m] = t.t[m];
+                }
+            }
+            __syncwarp();
+            if constexpr (M <= kSplit64) {
+                if (wok) ordered_round<M>(term, lane, k0, cnt, sum);
+            }
+            __syncwarp();
+        }
+        // the sums to the particle's first lane, the extrema over its lanes (exact in any order)
+        if (live && h < M) term[(lane - h) * M + h] = sum[0];
+        __syncwarp();
+        if (need_ext) {
+#pragma unroll
+            for (int m = 0; m < M; ++m)
+#pragma unroll
+                for (int o = 1; o < kSplit64; o <<= 1) {
+                    mn[m] = vmin(mn[m], __shfl_xor_sync(0xffffffffu, mn[m], o));
+                    mx[m] = vmax(mx[m], __shfl_xor_sync(0xffffffffu, mx[m], o));
+                }
+        }
+        if (live && h == 0) {
+            double Kv[M];
+#pragma unroll
+            for (int m = 0; m < M; ++m) Kv[m] = -(2.0 * term[lane * M + m]);
+            const bool f = stage_epilogue<double, D, M, PDE, RDEG>(a, i, fi, Kv, mn, mx);
+            if (a.check) list_failures(a, i, f);
+        }
+        if (i >= 0 && h == 0 && !a.full && a.clear_wmask) a.wmask[i >> 5] = 0u;
+        __syncwarp();
+    }
+}
+
+// gather_one's cached fit with the slots shared by eight lanes; the other cases (no cached fit) go through gather_one
+// in the particle's first lane. Full passes without a limiter.
+template <int D, int M, int PDE, int RDEG>
+__global__ void __launch_bounds__(128) k_gather_split(const StageArgs<double> a) {
+    constexpr int BR = RBasis<D, RDEG>::B, E = BR * M, GS = grad_row<double, E>(), NE = (E + kSplit64 - 1) / kSplit64;
+    __shared__ double terms[4][32 * E];
+    double *term = terms[threadIdx.x >> 5];
+    const int lane = int(threadIdx.x & 31), h = lane % kSplit64;
+    const int64_t np = a.g.npad;
+    const int64_t i = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) / kSplit64;
+    const bool live = i < a.g.n && !a.g.bnd[i];
+    int cnt = 0;
+    bool cached = false;
+    double fi[M], sum[NE];
+#pragma unroll
+    for (int q = 0; q < NE; ++q) sum[q] = 0.0;
+    if (live) {
+        cnt = a.g.cnt[i];
+        int p = a.orders[i];
+        while (p > 1 && cnt < basis_count(D, p - 1)) --p;
+        cached = p == a.sc.max_order && p > 1 && a.g.ok_r[i];
+        load_vec<double, M>(a.U + i * M, fi);
+    }
+    if (!cached) cnt = 0;
+    const int kw = __reduce_max_sync(0xffffffffu, cnt);
+    for (int k0 = 0; k0 < kw; k0 += kSplit64) {
+        const int k = k0 + h;
+        if (k < cnt) {
+            const int64_t s = int64_t(k) * np + i;
+            double x[D], pb[BR], df[M];
+            load_vec<double, M>(a.U + int64_t(a.g.nidx[s]) * M, df);
+#pragma unroll
+            for (int d = 0; d < D; ++d) x[d] = a.g.dist[(int64_t(k) * D + d) * np + i] * a.g.invL;
+            const double w = a.g.wt[s];
+            recon_basis<D, RDEG, double>(x, pb);
+#pragma unroll
+            for (int m = 0; m < M; ++m) df[m] = df[m] - fi[m];
+#pragma unroll
+            for (int b = 0; b < BR; ++b)
+#pragma unroll
+                for (int m = 0; m < M; ++m) term[lane * E + b * M + m] = w * (pb[b] * df[m]);
+        }
+        __syncwarp();
+        ordered_round<E>(term, lane, k0, cnt, sum);
+        __syncwarp();
+    }
+#pragma unroll
+    for (int q = 0; q < NE; ++q)
+        if (h + kSplit64 * q < E) term[(lane - h) * E + h + kSplit64 * q] = sum[q];
+    __syncwarp();
+    if (!live) return;
+    if (!cached) {
+        if (h == 0) gather_one<double, D, M, PDE, RDEG>(a, i);
+        return;
+    }
+    // the inverse moments applied entry by entry: g_bm = (sum_c inv_bc bs_cm) scale_b, in gather_one's order
+    const double *inv = a.g.inv_r + i * (BR * BR), *bs = term + (lane - h) * E;
+    for (int e = h; e < E; e += kSplit64) {
+        const int b = e / M, m = e % M;
+        double acc = inv[b * BR] * bs[m];
+        for (int c = 1; c < BR; ++c) acc = acc + inv[b * BR + c] * bs[c * M + m];
+        a.grad[i * GS + e] = acc * recon_scale<D, RDEG, double>(b, a.g.invL);
     }
 }
 
@@ -3206,6 +3424,12 @@ struct StageInst {
                 return;
             }
         }
+        if constexpr (sizeof(T) == 8 && M <= kSplit64) {
+            if (a.full && a.sc.limiter == HCC_LIMITER_NONE && n <= HCC_SPLIT64_GATHER) {
+                k_gather_split<D, M, PDE, RDEG><<<grid(n * kSplit64, 128), 128, 0, s>>>(a);
+                return;
+            }
+        }
         const int bs = a.full ? a.gather_block : 128;
         k_gather<T, D, M, PDE, RDEG><<<pass_grid(a, n, bs), bs, 0, s>>>(a);
     }
@@ -3255,6 +3479,14 @@ struct StageInst {
                 const unsigned g = split_grid(a), nth = 32 * split_warps<M>();
                 if (a.mover) k_flux_tiles<T, D, M, PDE, RDEG, true><<<g, nth, 0, s>>>(a);
                 else k_flux_tiles<T, D, M, PDE, RDEG, false><<<g, nth, 0, s>>>(a);
+                return;
+            }
+        }
+        if constexpr (sizeof(T) == 8 && M <= kSplit64) {
+            if (n <= (a.full ? HCC_SPLIT64_FLUX : HCC_SPLIT64_LIST) && !(a.full && a.rough_words)) {
+                const unsigned g = a.full ? grid(n * kSplit64, 128) : std::max(1u, unsigned(a.list_blocks));
+                if (a.mover) k_flux_split<D, M, PDE, RDEG, true><<<g, 128, 0, s>>>(a);
+                else k_flux_split<D, M, PDE, RDEG, false><<<g, 128, 0, s>>>(a);
                 return;
             }
         }

@@ -59,6 +59,8 @@ __global__ void k_drop_decide(const DropArgs a) {
         for (unsigned q = warp; q < nt; q += nwarps) {
             const int32_t tile = a.ttiles[q];
             const uint32_t word = a.tmask[tile];
+            __syncwarp();
+            if (lane == 0) a.tmask[tile] = 0u;         // the failures are consumed here
             const int64_t i = int64_t(tile) * 32 + lane;
             bool ch = false;
             if ((word >> lane) & 1u) {
@@ -92,6 +94,7 @@ __global__ void k_drop_decide(const DropArgs a) {
     ct->cn = 0;
     ct->t = 0;
     ct->d = 0;
+    ct->dp = 0;
     ct->f = 0;
     ct->done = 0;
     unsigned go = 0;
@@ -171,7 +174,7 @@ __global__ void k_reach_fix(ListCounts *counts, const int32_t *dtiles, const uin
         words1[q] = dmask[dtiles[q]];
 }
 __global__ void k_reach_hop2(ListCounts *counts, int32_t *dtiles, uint32_t *dmask, const uint32_t *words1,
-                             const int32_t *cnt, const int32_t *nidx, int64_t npad) {
+                             int32_t *dlist, const int32_t *cnt, const int32_t *nidx, int64_t npad) {
     const unsigned n1 = counts->d1;
     const int lane = int(threadIdx.x & 31);
     const unsigned warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -181,7 +184,7 @@ __global__ void k_reach_hop2(ListCounts *counts, int32_t *dtiles, uint32_t *dmas
         const int c = mem ? cnt[i] : 0;
         const int kw = __reduce_max_sync(0xffffffffu, c);
         for (int k = 0; k < kw; ++k)     // slot by slot across the warp, combined atomics
-            reach_mark_warp(dmask, dtiles, &counts->d, k < c ? nidx[int64_t(k) * npad + i] : -1);
+            reach_mark_warp(dmask, dtiles, &counts->d, dlist, &counts->dp, k < c ? nidx[int64_t(k) * npad + i] : -1);
     }
 }
 
@@ -359,10 +362,10 @@ void launch_drop_decide(const DropArgs &a, int is_f32, int drop_blocks, cudaStre
     else k_drop_decide<double><<<blocks, HCC_BLOCK, 0, s>>>(a);
 }
 void launch_reach_hop2(ListCounts *counts, const int32_t *dtiles, int32_t *dtiles_out, uint32_t *dmask,
-                       uint32_t *words1, const int32_t *cnt, const int32_t *nidx, int64_t npad, int blocks,
-                       cudaStream_t s) {
+                       uint32_t *words1, int32_t *dlist, const int32_t *cnt, const int32_t *nidx, int64_t npad,
+                       int blocks, cudaStream_t s) {
     k_reach_fix<<<blocks, HCC_BLOCK, 0, s>>>(counts, dtiles, dmask, words1);
-    k_reach_hop2<<<blocks, HCC_BLOCK, 0, s>>>(counts, dtiles_out, dmask, words1, cnt, nidx, npad);
+    k_reach_hop2<<<blocks, HCC_BLOCK, 0, s>>>(counts, dtiles_out, dmask, words1, dlist, cnt, nidx, npad);
 }
 void launch_nbmin(const int8_t *orders, int8_t *nbmin, const int32_t *cnt, const int32_t *nidx, int64_t n,
                   int64_t npad, const int32_t *tiles, const uint32_t *words, const unsigned *count, int blocks,

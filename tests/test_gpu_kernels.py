@@ -145,3 +145,37 @@ def test_tile_unions(hcc, oracle, cuda_lib, n, shuffled):
         assert got["union_entries"] == sum(sizes) and got["largest_union"] == max(sizes)
     inner = cloud.is_boundary == 0
     assert _rel_l1(g.compute_rhs()[inner], o.compute_rhs()[inner]) < 1e-4
+
+
+@pytest.mark.parametrize("n", [6, 150, 160])
+@pytest.mark.parametrize("kind", ["euler", "order3", "limited", "moving", "strict"])
+def test_fp64_passes_on_both_sides_of_the_split(hcc, oracle, cuda_lib, kind, n):
+    """FP64 clouds below and above the size up to which eight lanes share a particle, with jumps that keep the worklists
+    busy: states, orders and flags bit for bit."""
+    h = 1.0 / n
+    cloud = hcc.rectangular_cloud((0.0, 0.0), (1.0, 1.0), h, 2.5 * h, jitter=0.2 * h, seed=n, periodic=kind == "moving")
+    x, y = cloud.pos[:, 0], cloud.pos[:, 1]
+    inside = (x - 0.5) ** 2 + (y - 0.45) ** 2 < 0.06
+    mood = hcc.MOOD(hcc.STRICT_EPD0 if kind == "strict" else hcc.EPD1, hcc.MOODu1(1e-4 * h * h))
+    bc = {} if kind == "moving" else OUTFLOW
+    if kind in ("order3", "limited"):
+        cfg = hcc.make_config(hcc.LinearAdvection(((1.0,), (0.5,))), cloud, mood=mood, bc_map=bc,
+                              scheme=hcc.MUSCL(3, 0, "vk_hard" if kind == "limited" else "none"))
+        U = (np.where(inside, 1.0, 0.0) + 0.3 * np.sin(6 * x))[:, None]
+    else:
+        cfg = hcc.make_config(hcc.Euler(2), cloud, mood=mood, bc_map=bc, scheme=hcc.MUSCL(2, 2))
+        rho, p = np.where(inside, 1.0, 0.3), np.where(inside, 1.0, 0.2)
+        U = np.column_stack([rho, 0.2 * rho, -0.1 * rho, p / 0.4 + 0.025 * rho])
+    g, o = _pair(hcc, oracle, cfg, cloud, U)
+    if kind == "moving":
+        for c in (g, o):
+            c.set_mover(hcc.mover("lagrangian"))
+    dt = 0.3 * o.time_step()
+    assert g.time_step() == o.time_step()
+    for s in range(2):
+        g.step(s * dt, dt)
+        o.step(s * dt, dt)
+    assert _same_bits(g.download_state(), o.download_state())
+    assert np.array_equal(g.orders(), o.orders()) and np.array_equal(g.mood_flags(), o.mood_flags())
+    if kind == "moving":
+        assert _same_bits(g.positions(), o.positions())
