@@ -26,9 +26,13 @@ UNITS = {
     "hcc_search.cu": ["-fmad=false"],
     "hcc_mls.cu": ["-fmad=false"],
     "hcc_stage_f64_r1.cu": ["-fmad=false"],
+    "hcc_stage_f64_r1_linear.cu": ["-fmad=false"],
     "hcc_stage_f64_r2.cu": ["-fmad=false"],
+    "hcc_stage_f64_r2_linear.cu": ["-fmad=false"],
     "hcc_stage_f32_r1.cu": ["-ftz=true"],
+    "hcc_stage_f32_r1_linear.cu": ["-ftz=true"],
     "hcc_stage_f32_r2.cu": ["-ftz=true"],
+    "hcc_stage_f32_r2_linear.cu": ["-ftz=true"],
     "hcc_noalloc.cu": ["-fmad=false"],
     "hcc_tiles.cu": [],
     "hcc_learn.cu": ["-fmad=false"],
@@ -77,7 +81,7 @@ def build(verbose: bool = False, jobs: int | None = None, extra_flags=None, lib_
             print(r.stdout + r.stderr, flush=True)
         return r
 
-    with ThreadPoolExecutor(max_workers=jobs or min(8, os.cpu_count() or 4)) as ex:
+    with ThreadPoolExecutor(max_workers=jobs or min(16, os.cpu_count() or 4)) as ex:
         list(ex.map(run, cmds))
     if cmds or not LIB.exists() or any(o.stat().st_mtime > LIB.stat().st_mtime for o in objs):
         link = [nvcc(), *ARCH, "-shared", "-o", str(LIB), *map(str, objs)]

@@ -480,6 +480,10 @@ const StageOps *stage_ops_f64_r1(int D, int M, int pde);
 const StageOps *stage_ops_f64_r2(int D, int M, int pde);
 const StageOps *stage_ops_f32_r1(int D, int M, int pde);
 const StageOps *stage_ops_f32_r2(int D, int M, int pde);
+const StageOps *stage_ops_f64_r1_linear(int D, int M, int pde);
+const StageOps *stage_ops_f64_r2_linear(int D, int M, int pde);
+const StageOps *stage_ops_f32_r1_linear(int D, int M, int pde);
+const StageOps *stage_ops_f32_r2_linear(int D, int M, int pde);
 
 // ----------------------------------------------------------------------------------- search / geometry
 struct SearchArgs {

@@ -1,5 +1,7 @@
-// hcc_stage_f32_r2.cu — stage kernels, float arithmetic, reconstruction degree 2.
+// hcc_stage_f32_r2.cu — stage kernels of the Euler modules, float arithmetic, reconstruction degree 2.
 #include "hcc_stage_impl.cuh"
 namespace hcc {
-const StageOps *stage_ops_f32_r2(int D, int M, int pde) { return lookup_rdeg<float, 2>(D, M, pde); }
+const StageOps *stage_ops_f32_r2(int D, int M, int pde) {
+    return pde == HCC_PDE_EULER ? lookup_euler<float, 2>(D, M) : stage_ops_f32_r2_linear(D, M, pde);
+}
 }  // namespace hcc

@@ -1,6 +1,7 @@
 // hcc_stage_impl.cuh — the per-stage kernels, templated on the arithmetic type T (double: plain FP64 path,
 // float: FP32 bulk path), the dimension D, the number of state components M, the physics module PDE and the
-// reconstruction degree RDEG. Included once per precision by hcc_stage_f64.cu / hcc_stage_f32.cu.
+// reconstruction degree RDEG. Included per precision, degree and physics by hcc_stage_f{64,32}_r{1,2}[_linear].cu (the
+// Euler modules and the linear ones compile side by side).
 //
 // Thread per particle over slot-major neighbour arrays: the 32 threads of a warp read slot k of 32 consecutive
 // particles from consecutive addresses; neighbour states, gradients and orders are gathered through L1/L2
@@ -452,35 +453,41 @@ template <typename T>
 __device__ __forceinline__ T limiter_phi(int lim, T r) {
     if (lim == HCC_LIMITER_BJ_SOFT || lim == HCC_LIMITER_BJ_HARD) return vmin(T(1), r);
     const T rp = vmax(T(0), r);
-    const T sv = T(1) / vmax(T(1), rp);
-    const T small = (rp * rp + T(2) * rp) / (rp * rp + rp + T(2));
-    const T large = (T(1) + T(2) * sv) / (T(1) + sv + T(2) * (sv * sv));
-    return rp > T(1) ? large : small;
+    if (rp > T(1)) {
+        const T sv = T(1) / rp;
+        return (T(1) + T(2) * sv) / (T(1) + sv + T(2) * (sv * sv));
+    }
+    return (rp * rp + T(2) * rp) / (rp * rp + rp + T(2));
 }
 
 template <typename T> __device__ __forceinline__ T eps16();
 template <> __device__ __forceinline__ double eps16<double>() { return 16.0 * 2.220446049250313e-16; }
 template <> __device__ __forceinline__ float eps16<float>() { return 16.0f * 1.1920929e-7f; }
 
-// _limit_slopes for BJ / VK (Limiter.jl:120-143): local extrema over {i} ∪ N(i) (_local_extrema, :61-69), the
+// Local extrema over {i} u N(i) (_local_extrema, Limiter.jl:61-69), one neighbour at a time.
+template <typename T, int M> __device__ __forceinline__ void extend_extrema(const T *f, T *umin, T *umax) {
+#pragma unroll
+    for (int m = 0; m < M; ++m) { umax[m] = vmax(umax[m], f[m]); umin[m] = vmin(umin[m], f[m]); }
+}
+
+// _limit_slopes for BJ / VK (Limiter.jl:120-143): with the local extrema of the reconstruction's own neighbour loop, the
 // bounding coefficient over the interface reconstructions (_bounding_phi / _update_phi, :76-100), then the
-// gradient terms (hard: every term; soft: the first-degree ones) scaled by it.
+// gradient terms (hard: every term; soft: the first-degree ones) scaled by it. The coefficient only falls below 1
+// where the distance to the bound is under twice the reconstructed step (Venkatakrishnan; (r^2 + 2r) >= (r^2 + r + 2)
+// from r = 2 on, computed as 1 or more) or under the step (Barth-Jespersen), so the divisions of the other slots, most
+// of them in a resolved field, are left out.
 template <typename T, int D, int M, int RDEG>
-__device__ __forceinline__ void limit_slopes(const StageArgs<T> &a, int64_t i, int cnt, const T *fi,
-                                             T (*out)[M]) {
+__device__ __forceinline__ void limit_slopes(const StageArgs<T> &a, int64_t i, int cnt, const T *fi, const T *umin,
+                                             const T *umax, T (*out)[M]) {
     constexpr int BR = RBasis<D, RDEG>::B;
     const int64_t np = a.g.npad;
-    T umax[M], umin[M], phi[M];
+    T phi[M];
 #pragma unroll
-    for (int m = 0; m < M; ++m) { umax[m] = fi[m]; umin[m] = fi[m]; phi[m] = T(1); }
-    for (int k = 0; k < cnt; ++k) {
-        const int32_t j = a.g.nidx[int64_t(k) * np + i];
-        T fj[M];
-        load_vec<T, M>(a.U + int64_t(j) * M, fj);
-#pragma unroll
-        for (int m = 0; m < M; ++m) { umax[m] = vmax(umax[m], fj[m]); umin[m] = vmin(umin[m], fj[m]); }
-    }
+    for (int m = 0; m < M; ++m) phi[m] = T(1);
     const T tol16 = eps16<T>();
+    const bool bj = a.sc.limiter == HCC_LIMITER_BJ_SOFT || a.sc.limiter == HCC_LIMITER_BJ_HARD;
+    const T reach = bj ? T(1) : T(2.01);
+#pragma unroll 2
     for (int k = 0; k < cnt; ++k) {
         T hx[D], p[BR];
 #pragma unroll
@@ -491,9 +498,11 @@ __device__ __forceinline__ void limit_slopes(const StageArgs<T> &a, int64_t i, i
             T recon = out[0][m] * p[0];
 #pragma unroll
             for (int b = 1; b < BR; ++b) recon = recon + out[b][m] * p[b];
-            const T bound = recon > T(0) ? umax[m] : umin[m];
+            const T bound = positive(recon) ? umax[m] : umin[m];
+            const T room = bound - fi[m];
+            if (fabs(room) >= fabs(reach * recon)) continue;      // (a NaN goes on)
             const T tol = tol16 * vmax(fabs(fi[m]), fabs(bound));
-            if (fabs(recon) > tol) phi[m] = vmin(phi[m], limiter_phi<T>(a.sc.limiter, (bound - fi[m]) / recon));
+            if (fabs(recon) > tol) phi[m] = vmin(phi[m], limiter_phi<T>(a.sc.limiter, room / recon));
         }
     }
     const bool hard = a.sc.limiter == HCC_LIMITER_BJ_HARD || a.sc.limiter == HCC_LIMITER_VK_HARD;
@@ -508,7 +517,8 @@ __device__ __forceinline__ void limit_slopes(const StageArgs<T> &a, int64_t i, i
 // ----------------------------------------------------------------------------------- gather pass
 // update_content! of MUSCL (MUSCL.jl:351-384) with NoLimiter: starved-order lowering, cached full-order fit
 // (apply_weights, Interpolators.jl:585-602), dynamic lower-degree fit, or zero (order 1).
-template <typename T, int D, int M, int PDE, int RDEG>
+// LIM: a slope limiter is on (its extrema are kept in the neighbour loop; without it they cost no registers).
+template <typename T, int D, int M, int PDE, int RDEG, bool LIM>
 __device__ __forceinline__ void gather_one(const StageArgs<T> &a, const int64_t i) {
     constexpr int BR = RBasis<D, RDEG>::B;
     if (a.g.bnd[i]) return;
@@ -529,6 +539,10 @@ __device__ __forceinline__ void gather_one(const StageArgs<T> &a, const int64_t 
         for (int m = 0; m < M; ++m) out[b][m] = T(0);
     const T invL = a.g.invL;
     bool done = false;
+    const bool lim = LIM && p > 1;
+    T umin[M], umax[M];                               // of the neighbour loop below (limiter only)
+#pragma unroll
+    for (int m = 0; m < M; ++m) umin[m] = umax[m] = fi[m];
     if constexpr (sizeof(T) == 4 && RDEG == 1) {
         // FP32, degree 1: the cached fit as one weight vector per slot (nidx + D floats per slot)
         if (p == a.sc.max_order && p > 1 && a.g.ok_r[i] && a.g.gw) {
@@ -546,14 +560,17 @@ __device__ __forceinline__ void gather_one(const StageArgs<T> &a, const int64_t 
                 }
 #pragma unroll
                 for (int q = 0; q < G; ++q) load_vec<T, M>(a.U + int64_t(j[q]) * M, df[q]);
+                asm volatile("" ::: "memory");        // the compiler keeps the group's loads ahead of its sums
 #pragma unroll
-                for (int q = 0; q < G; ++q)
+                for (int q = 0; q < G; ++q) {
+                    if (lim) extend_extrema<T, M>(df[q], umin, umax);
 #pragma unroll
                     for (int m = 0; m < M; ++m) {
                         const T dm = df[q][m] - fi[m];
 #pragma unroll
                         for (int b = 0; b < BR; ++b) out[b][m] = out[b][m] + gk[q][b] * dm;
                     }
+                }
             }
             for (; k < cnt; ++k) {
                 const int32_t j = a.g.nidx[int64_t(k) * np + i];
@@ -561,6 +578,7 @@ __device__ __forceinline__ void gather_one(const StageArgs<T> &a, const int64_t 
 #pragma unroll
                 for (int d = 0; d < D; ++d) gk[d] = a.g.gw[(int64_t(k) * D + d) * np + i];
                 load_vec<T, M>(a.U + int64_t(j) * M, df);
+                if (lim) extend_extrema<T, M>(df, umin, umax);
 #pragma unroll
                 for (int m = 0; m < M; ++m) {
                     const T dm = df[m] - fi[m];
@@ -598,6 +616,7 @@ __device__ __forceinline__ void gather_one(const StageArgs<T> &a, const int64_t 
             recon_basis<D, RDEG, T>(x, pb);
             T df[M];
             load_vec<T, M>(a.U + int64_t(j) * M, df);
+            if (lim) extend_extrema<T, M>(df, umin, umax);
 #pragma unroll
             for (int m = 0; m < M; ++m) df[m] = df[m] - fi[m];
 #pragma unroll
@@ -704,7 +723,15 @@ __device__ __forceinline__ void gather_one(const StageArgs<T> &a, const int64_t 
             }
         }
     }
-    if (a.sc.limiter != HCC_LIMITER_NONE && p > 1) limit_slopes<T, D, M, RDEG>(a, i, cnt, fi, out);
+    if (lim) {
+        if (!done && !(p == a.sc.max_order && a.g.ok_r[i]))       // a lowered order's fit (or none): its own loop
+            for (int k = 0; k < cnt; ++k) {
+                T f[M];
+                load_vec<T, M>(a.U + int64_t(a.g.nidx[int64_t(k) * np + i]) * M, f);
+                extend_extrema<T, M>(f, umin, umax);
+            }
+        limit_slopes<T, D, M, RDEG>(a, i, cnt, fi, umin, umax, out);
+    }
     store_row<T, BR * M, grad_row<T, BR * M>()>(g, &out[0][0]);
 }
 
@@ -713,24 +740,26 @@ __device__ __forceinline__ void gather_one(const StageArgs<T> &a, const int64_t 
 // each at 66 slots in 3-D) is the slots over the warps. Short lists leave most SMs idle and take the whole block a
 // tile; longer ones keep four warps a tile, whose partial sums cost less to combine. The line depends on the list
 // alone, so results do not depend on the launch shape. States of 8 and more components keep blocks of four warps
-// (shared memory of their partial sums).
+// (shared memory of their partial sums), and so does the flux pass in 1-D and 2-D: about 20 slots are few for 16 warps
+// (15.7 us a pass with 16 warps, 12.9 with four; the reconstruction pass 8.8 against 12.5).
 template <int M> constexpr int split_warps() { return M >= 8 ? 4 : 16; }
-template <int M> __device__ __forceinline__ int split_share(unsigned nt) {
-    return split_warps<M>() > 4 && nt <= HCC_SPLIT_WIDE_TILES ? split_warps<M>() : 4;
+template <int D, int M> constexpr int flux_split_warps() { return M >= 8 || D < 3 ? 4 : 16; }
+template <int NW> __device__ __forceinline__ int split_share(unsigned nt) {
+    return NW > 4 && nt <= HCC_SPLIT_WIDE_TILES ? NW : 4;
 }
 
 // FP32 degree-1 worklist pass of the reconstruction with several warps per tile: the tile's first warp lowers starved
 // orders and picks the path; on the cached gradient-weight path warp w of W sums the slots k = w, w + W, ... and marks
 // their neighbours' reach, the first warp adds the partial sums in a fixed order, applies the limiter and stores the
-// gradients; any other particle is reconstructed whole by the first warp.
-template <typename T, int D, int M, int PDE, int RDEG>
+// gradients; any other particle has zero slopes (with a limiter: is reconstructed whole by the first warp).
+template <typename T, int D, int M, int PDE, int RDEG, bool LIM>
 __global__ void __launch_bounds__(32 * split_warps<M>()) k_gather_tiles(const StageArgs<T> a) {
     constexpr int BR = RBasis<D, RDEG>::B, NW = split_warps<M>();
     __shared__ T parts[NW][32][BR * M];
     __shared__ int path[NW / 4][32];
     const int lane = int(threadIdx.x & 31), wb = int(threadIdx.x >> 5);
     const unsigned nt = *a.wcount;
-    const int W = split_share<M>(nt);              // warps per tile
+    const int W = split_share<NW>(nt);             // warps per tile
     const int group = wb / W, w = wb % W, first = group * W;
     const unsigned step = unsigned(NW / W) * gridDim.x;
     const int64_t np = a.g.npad;
@@ -798,10 +827,27 @@ __global__ void __launch_bounds__(32 * split_warps<M>()) k_gather_tiles(const St
                         for (int v = 1; v < W; ++v) sm = sm + parts[first + v][lane][b * M + m];
                         out[b][m] = sm;
                     }
-                if (a.sc.limiter != HCC_LIMITER_NONE) limit_slopes<T, D, M, RDEG>(a, i, cnt, fi, out);
+                if constexpr (LIM) {
+                    T umin[M], umax[M];
+#pragma unroll
+                    for (int m = 0; m < M; ++m) umin[m] = umax[m] = fi[m];
+                    for (int k = 0; k < cnt; ++k) {
+                        T f[M];
+                        load_vec<T, M>(a.U + int64_t(a.g.nidx[int64_t(k) * np + i]) * M, f);
+                        extend_extrema<T, M>(f, umin, umax);
+                    }
+                    limit_slopes<T, D, M, RDEG>(a, i, cnt, fi, umin, umax, out);
+                }
                 store_row<T, BR * M, grad_row<T, BR * M>()>(a.grad + i * grad_row<T, BR * M>(), &out[0][0]);
             } else {
-                gather_one<T, D, M, PDE, RDEG>(a, i);
+                if constexpr (LIM) {
+                    gather_one<T, D, M, PDE, RDEG, true>(a, i);
+                } else {                           // off the cached fit: zero slopes
+                    T z[BR * M];
+#pragma unroll
+                    for (int b = 0; b < BR * M; ++b) z[b] = T(0);
+                    store_row<T, BR * M, grad_row<T, BR * M>()>(a.grad + i * grad_row<T, BR * M>(), z);
+                }
             }
         }
         if (w == 0 && lane == 0 && q < nt && a.clear_wmask) a.wmask[tile] = 0u;   // every lane read the word before the barrier
@@ -811,11 +857,11 @@ __global__ void __launch_bounds__(32 * split_warps<M>()) k_gather_tiles(const St
 
 // A full pass (one thread per particle) or a worklist pass over tiles (one warp per tile, the members of its word)
 // that also marks the one-hop reach of each member in rmask / rtiles.
-template <typename T, int D, int M, int PDE, int RDEG>
+template <typename T, int D, int M, int PDE, int RDEG, bool LIM>
 __global__ void __launch_bounds__(128) k_gather(const StageArgs<T> a) {
     if (a.full) {
         const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-        if (i < a.g.n) gather_one<T, D, M, PDE, RDEG>(a, i);
+        if (i < a.g.n) gather_one<T, D, M, PDE, RDEG, LIM>(a, i);
         return;
     }
     const unsigned nt = *a.wcount;
@@ -829,7 +875,7 @@ __global__ void __launch_bounds__(128) k_gather(const StageArgs<T> a) {
         if (a.clear_wmask && lane == 0) a.wmask[tile] = 0u;     // the changed list is consumed here
         const bool mem = (word >> lane) & 1u;
         const int32_t i = tile * 32 + lane;
-        if (mem) gather_one<T, D, M, PDE, RDEG>(a, i);
+        if (mem) gather_one<T, D, M, PDE, RDEG, LIM>(a, i);
         if (a.rmask) {
             // the reach (members and their neighbours), slot by slot across the warp with combined atomics
             reach_mark_warp(a.rmask, a.rtiles, a.rcount, a.rlist, a.rlcount, mem ? i : -1);
@@ -1650,7 +1696,7 @@ __global__ void __launch_bounds__(128) k_gather_split(const StageArgs<double> a)
     __syncwarp();
     if (!live) return;
     if (!cached) {
-        if (h == 0) gather_one<double, D, M, PDE, RDEG>(a, i);
+        if (h == 0) gather_one<double, D, M, PDE, RDEG, false>(a, i);
         return;
     }
     // the inverse moments applied entry by entry: g_bm = (sum_c inv_bc bs_cm) scale_b, in gather_one's order
@@ -1668,12 +1714,12 @@ __global__ void __launch_bounds__(128) k_gather_split(const StageArgs<double> a)
 // first warp combines the compensated partial sums (Kahan over the partials, minus their compensations) and the
 // extrema, and runs the epilogue. Block-stride over the list.
 template <typename T, int D, int M, int PDE, int RDEG, bool ALE, bool MOM = false>
-__global__ void __launch_bounds__(32 * split_warps<M>()) k_flux_tiles(const StageArgs<T> a) {
-    constexpr int NW = split_warps<M>();
+__global__ void __launch_bounds__(32 * flux_split_warps<D, M>()) k_flux_tiles(const StageArgs<T> a) {
+    constexpr int NW = flux_split_warps<D, M>();
     __shared__ FluxPart<T, M> parts[NW][32];
     const int lane = int(threadIdx.x & 31), wb = int(threadIdx.x >> 5);
     const unsigned nt = *a.wcount;
-    const int W = split_share<M>(nt);              // warps per tile
+    const int W = split_share<NW>(nt);             // warps per tile
     const int group = wb / W, w = wb % W, first = group * W;
     const unsigned step = unsigned(NW / W) * gridDim.x;
     for (unsigned q0 = blockIdx.x * unsigned(NW / W); q0 < nt; q0 += step) {
@@ -1895,7 +1941,7 @@ __global__ void __launch_bounds__(2 * HCC_TILE, tile_gather_min_blocks<D, M>()) 
     __syncthreads();
     if (h == 1) return;
     if (mode == 2) {
-        if constexpr (LIM) gather_one<float, D, M, PDE, 1>(a, i);
+        if constexpr (LIM) gather_one<float, D, M, PDE, 1, true>(a, i);
         else store_row<float, D * M, GS>(a.grad + i * GS, &out[0][0]);
     } else if (mode == 1) {
         const float *cf = a.tv.coef + i * a.tv.cw + D + D * D;
@@ -3395,8 +3441,8 @@ struct StageInst {
         return a.full ? g : std::max(1u, std::min(g, unsigned(a.list_blocks)));
     }
     // blocks of an FP32 split worklist pass (list_blocks counts blocks of four warps)
-    static unsigned split_grid(const StageArgs<T> &a) {
-        return std::max(1u, unsigned(a.list_blocks) * 4u / unsigned(split_warps<M>()));
+    static unsigned split_grid(const StageArgs<T> &a, int warps) {
+        return std::max(1u, unsigned(a.list_blocks) * 4u / unsigned(warps));
     }
     // block of a full pass of the other flux-like schemes (the tuned flux block); worklist passes keep 128
     static int fbs(const StageArgs<T> &a) { return a.full ? a.flux_block : 128; }
@@ -3420,7 +3466,10 @@ struct StageInst {
                 return;
             }
             if (!a.full) {   // FP32 degree-1 worklist pass: split tiles
-                k_gather_tiles<T, D, M, PDE, RDEG><<<split_grid(a), 32 * split_warps<M>(), 0, s>>>(a);
+                if (a.sc.limiter != HCC_LIMITER_NONE)
+                    k_gather_tiles<T, D, M, PDE, RDEG, true><<<split_grid(a, split_warps<M>()), 32 * split_warps<M>(), 0, s>>>(a);
+                else
+                    k_gather_tiles<T, D, M, PDE, RDEG, false><<<split_grid(a, split_warps<M>()), 32 * split_warps<M>(), 0, s>>>(a);
                 return;
             }
         }
@@ -3431,12 +3480,15 @@ struct StageInst {
             }
         }
         const int bs = a.full ? a.gather_block : 128;
-        k_gather<T, D, M, PDE, RDEG><<<pass_grid(a, n, bs), bs, 0, s>>>(a);
+        if (a.sc.limiter != HCC_LIMITER_NONE)
+            k_gather<T, D, M, PDE, RDEG, true><<<pass_grid(a, n, bs), bs, 0, s>>>(a);
+        else
+            k_gather<T, D, M, PDE, RDEG, false><<<pass_grid(a, n, bs), bs, 0, s>>>(a);
     }
     template <bool MOM> static void flux_mom(const StageArgs<T> &a, int64_t n, cudaStream_t s) {
         if constexpr (sizeof(T) == 4) {
             if (!a.full) {
-                const unsigned g = split_grid(a), nth = 32 * split_warps<M>();
+                const unsigned g = split_grid(a, flux_split_warps<D, M>()), nth = 32 * flux_split_warps<D, M>();
                 if (a.mover) k_flux_tiles<T, D, M, PDE, RDEG, true, MOM><<<g, nth, 0, s>>>(a);
                 else k_flux_tiles<T, D, M, PDE, RDEG, false, MOM><<<g, nth, 0, s>>>(a);
                 return;
@@ -3476,7 +3528,7 @@ struct StageInst {
                 }
             }
             if (!a.full) {   // FP32 worklist pass: split tiles
-                const unsigned g = split_grid(a), nth = 32 * split_warps<M>();
+                const unsigned g = split_grid(a, flux_split_warps<D, M>()), nth = 32 * flux_split_warps<D, M>();
                 if (a.mover) k_flux_tiles<T, D, M, PDE, RDEG, true><<<g, nth, 0, s>>>(a);
                 else k_flux_tiles<T, D, M, PDE, RDEG, false><<<g, nth, 0, s>>>(a);
                 return;
@@ -3572,13 +3624,14 @@ struct StageInst {
 };
 
 template <typename T, int RDEG>
-const StageOps *lookup_rdeg(int D, int M, int pde) {
-    if (pde == HCC_PDE_EULER) {
-        if (D == 1 && M == 3) return StageInst<T, 1, 3, HCC_PDE_EULER, RDEG>::ops();
-        if (D == 2 && M == 4) return StageInst<T, 2, 4, HCC_PDE_EULER, RDEG>::ops();
-        if (D == 3 && M == 5) return StageInst<T, 3, 5, HCC_PDE_EULER, RDEG>::ops();
-        return nullptr;
-    }
+const StageOps *lookup_euler(int D, int M) {
+    if (D == 1 && M == 3) return StageInst<T, 1, 3, HCC_PDE_EULER, RDEG>::ops();
+    if (D == 2 && M == 4) return StageInst<T, 2, 4, HCC_PDE_EULER, RDEG>::ops();
+    if (D == 3 && M == 5) return StageInst<T, 3, 5, HCC_PDE_EULER, RDEG>::ops();
+    return nullptr;
+}
+template <typename T, int RDEG>
+const StageOps *lookup_linear(int D, int M, int pde) {
     if (pde == HCC_PDE_BGK) {
         if (D == 2 && M == 16) return StageInst<T, 2, 16, HCC_PDE_BGK, RDEG>::ops();
         if (D == 1 && M == 2) return StageInst<T, 1, 2, HCC_PDE_BGK, RDEG>::ops();
@@ -3590,6 +3643,5 @@ const StageOps *lookup_rdeg(int D, int M, int pde) {
     if (D == 2 && M == 2) return StageInst<T, 2, 2, HCC_PDE_ADVECTION, RDEG>::ops();
     return nullptr;
 }
-
 
 }  // namespace hcc
