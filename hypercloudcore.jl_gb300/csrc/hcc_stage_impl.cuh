@@ -2176,6 +2176,259 @@ __global__ void __launch_bounds__(2 * HCC_TILE, tile_flux_min_blocks<D, M>()) k_
     }
 }
 
+// ----------------------------------------------------------------------------------- wide linear systems (FP32)
+// Full flux pass of an FP32 linear system with many components (the 16-velocity kinetic model): a block takes a tile of
+// HCC_TILE particles, stages the rows of its neighbour union in shared memory and gives every particle M / 4 lanes, four
+// components each, half of the tile at a time. A row is 64 bytes of state and 128 of gradient, read about 20 times: with
+// one thread per particle and the rows gathered through the caches, a thread held 112 numbers of state, gradient, sums
+// and extrema (219 registers, two blocks an SM) and waited for the twelve loads of a slot that its index load had to
+// precede. Here a lane holds a quarter of that, the rows come from shared memory, and the slot streams (place in the
+// union, offsets, divergence weights: the FP32 streams of the stream-fed pass) do not depend on one another; the four
+// lanes load one of a slot's four stream words each and exchange them, four slots ahead of the sums.
+// (The reconstruction pass of these systems keeps k_gather: with a quarter of the arithmetic a slot, lanes sharing a
+// particle took 258 us against its 227.)
+template <int M> constexpr int wide_lanes() { return M / 4; }
+template <typename T, int M, int PDE> constexpr bool wide_system() {
+    return sizeof(T) == 4 && PDE != HCC_PDE_EULER && M >= 8 && M % 4 == 0 && 32 % (M / 4) == 0;
+}
+constexpr int kWideThreads = 256;
+// the flux row: state, gradient, the order in the word after them
+template <int D, int M> constexpr int wide_flux_row() { return 4 * tile_odd_groups(M + D * M + 1); }
+
+// stage_epilogue for the four components `off` ... of the lanes of a particle; every lane of the warp calls it (the
+// Maxwellian's sum and the flags cross the lanes), `live` marks those with a particle.
+template <int D, int M, int PDE>
+__device__ __forceinline__ bool wide_epilogue(const StageArgs<float> &a, int64_t i, int off, bool live, const float *fi,
+                                              const float *Kv, const float *mn, const float *mx) {
+    constexpr int L = wide_lanes<M>();
+    const int64_t row = i * M + off;
+    if (live) store_vec<float, 4>(a.K + row, Kv);
+    if (!a.form_next) return false;
+    float Y[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    const StageCoeffs<float> *cf = live ? coef_of(a, i) : a.coef;
+    if (live) {
+        load_vec<float, 4>(a.Un + row, Y);
+        for (int j = 0; j < a.n_prev; ++j) {
+            const float hE = cf->hE[j], hI = cf->hI[j];
+            if (hE != 0.0f) {
+                float kv[4];
+                if (j != a.self_slot) load_vec<float, 4>(a.KE[j] + row, kv);
+#pragma unroll
+                for (int m = 0; m < 4; ++m) Y[m] = Y[m] + hE * (j == a.self_slot ? Kv[m] : kv[m]);
+            }
+            if (hI != 0.0f) {
+                float kv[4];
+                load_vec<float, 4>(a.KI[j] + row, kv);
+#pragma unroll
+                for (int m = 0; m < 4; ++m) Y[m] = Y[m] + hI * kv[m];
+            }
+        }
+    }
+    if (a.implicit_mode) {
+        float KIo[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        if constexpr (PDE == HCC_PDE_BGK) {
+            float u = (Y[0] + Y[1]) + (Y[2] + Y[3]);
+#pragma unroll
+            for (int o = 1; o < L; o <<= 1) u = u + __shfl_xor_sync(0xffffffffu, u, o);
+            const float dto = cf->dt_ii * a.ph.inv_eps, denom = 1.0f / (1.0f + dto), inv_dt_ii = cf->inv_dt_ii;
+#pragma unroll
+            for (int m = 0; m < 4; ++m) {
+                float fd = (a.ph.a_macro[0] * u) * a.ph.sinv[off + m][0];
+#pragma unroll
+                for (int d = 1; d < D; ++d) fd = fd + (a.ph.a_macro[d] * u) * a.ph.sinv[off + m][d];
+                const float Mk = a.ph.coeff * (u + fd);
+                if (a.implicit_mode == 1) {
+                    const float o = (Y[m] + dto * Mk) * denom;
+                    KIo[m] = (o - Y[m]) * inv_dt_ii;
+                    Y[m] = o;
+                } else {
+                    KIo[m] = (Mk - Y[m]) * a.ph.inv_eps;
+                }
+            }
+        }
+        if (live) store_vec<float, 4>(a.KInext + row, KIo);
+    }
+    if (live) store_vec<float, 4>(a.Ynext + row, Y);
+    if (!a.check) return false;
+    float cand[4];
+    if (a.check_substep) {
+        float ki[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        if (a.KIs && live) load_vec<float, 4>(a.KIs + row, ki);
+#pragma unroll
+        for (int m = 0; m < 4; ++m) cand[m] = fi[m] + cf->h_sub * (a.KIs ? Kv[m] + ki[m] : Kv[m]);
+    } else {
+#pragma unroll
+        for (int m = 0; m < 4; ++m) cand[m] = Y[m];
+    }
+    bool adm = true, flag = false;
+    const float dl = a.delta, d3 = dl * dl * dl;
+    constexpr float kPad = 16.0f * 1.1920928955078125e-7f;
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+        adm = adm && isfinite(cand[m]);
+        const float pad = dl + kPad * vmax(fabsf(mn[m]), fabsf(mx[m]));
+        bool v = fabsf(mx[m] - mn[m]) >= d3 && (cand[m] < mn[m] - pad || cand[m] > mx[m] + pad);
+        if (a.sc.criterion == HCC_MOOD_U2 && v && a.u2_range) {
+            const unsigned long long nanbits = a.u2_range[2 * M];
+            const float range = ((nanbits >> (off + m)) & 1ull)
+                                    ? float(NAN)
+                                    : float(order_value(a.u2_range[M + off + m])) - float(order_value(a.u2_range[off + m]));
+            v = !(mx[m] - mn[m] < a.u2_plateau * range);
+        }
+        flag = flag || v;
+    }
+    // over the particle's lanes
+    const unsigned lanes = ((1u << L) - 1u) << ((threadIdx.x & 31u) / L * L);
+    adm = (__ballot_sync(0xffffffffu, !adm) & lanes) == 0u;
+    flag = (__ballot_sync(0xffffffffu, flag) & lanes) != 0u;
+    if (live && off == 0) a.inadm[i] = !adm;
+    if (!live) return false;
+    if (a.sc.criterion == HCC_MOOD_ONLY || !adm) return true;
+    return (a.sc.criterion == HCC_MOOD_U1 || a.sc.criterion == HCC_MOOD_U2) && flag;
+}
+
+// flux_one for a linear system on a fixed grid, degree-1 reconstruction. With A = f_ij - f_i and B = f_ji - f_i the flux
+// difference of a slot contracted with its divergence weights is
+//   cw (f_ij + f_ji - 2 f_i) - S (f_ji - f_ij) = (cw + S) A + (cw - S) B,   cw = sum_d w_d c_dm,
+// S = sum_d w_d s_d max lambda_d common to the components: formed from differences of the states, no flux cancels.
+template <int D, int M, int PDE>
+__global__ void __launch_bounds__(kWideThreads, 3) k_flux_wide(const StageArgs<float> a) {
+    extern __shared__ __align__(16) float sm[];
+    constexpr int L = wide_lanes<M>(), W = wide_flux_row<D, M>(), RG = (D + 1) * L;   // 16-byte groups of a row
+    constexpr int G = 4, P = kWideThreads / L;     // slots a group, particles at a time
+    static_assert(L == 2 * D, "one of a slot's 2 D offsets and weights a lane");
+    __shared__ unsigned failed[HCC_TILE / 32], rough[HCC_TILE / 32];
+    const int64_t t = blockIdx.x, u0 = a.tv.ustart[t], np = a.g.npad;
+    const int nu = int(a.tv.ustart[t + 1] - u0);
+    if (threadIdx.x < HCC_TILE / 32) { failed[threadIdx.x] = 0u; rough[threadIdx.x] = 0u; }
+    for (int e = threadIdx.x; e < nu * RG; e += kWideThreads) {
+        const int64_t j = a.tv.uid[u0 + e / RG];
+        const int g = e % RG;
+        float v[4];
+        load_vec<float, 4>(g < L ? a.U + j * M + 4 * g : a.grad + j * (D * M) + 4 * (g - L), v);
+        store_vec<float, 4>(sm + (e / RG) * W + 4 * g, v);
+    }
+    for (int e = threadIdx.x; e < nu; e += kWideThreads)
+        sm[e * W + (D + 1) * M] = __int_as_float(int(a.orders[a.tv.uid[u0 + e]]));
+    const int c = int(threadIdx.x) % L, off = 4 * c, lane0 = int(threadIdx.x & 31) - c;
+    const bool need_ext = a.check && (a.sc.criterion == HCC_MOOD_U1 || a.sc.criterion == HCC_MOOD_U2);
+    float cm[D][4];
+#pragma unroll
+    for (int d = 0; d < D; ++d)
+#pragma unroll
+        for (int m = 0; m < 4; ++m) cm[d][m] = a.ph.c[d][off + m];
+    __syncthreads();
+    for (int pl = int(threadIdx.x) / L; pl < HCC_TILE; pl += P) {
+        const int64_t i = t * HCC_TILE + pl;
+        const bool bnd = i < a.g.n && a.g.bnd[i];
+        const bool live = i < a.g.n && !bnd;
+        float fi[4] = {0.0f, 0.0f, 0.0f, 0.0f}, mn[4], mx[4], Kv[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        if (bnd) store_vec<float, 4>(a.K + i * M + off, Kv);
+        const int cnt = live ? a.g.cnt[i] : 0;
+        const bool wok = cnt > 0 && a.g.ok_d[i];
+        // this lane's stream word of each slot, and the neighbour's place: the next group's in flight
+        const float *sp = (c < D ? a.g.dist + int64_t(c) * np : a.g.dw + int64_t(c - D) * np) + i;
+        const uint16_t *lp = a.tv.lidx + i;
+        float v[G];
+        int l[G];
+#pragma unroll
+        for (int q = 0; q < G; ++q) {
+            v[q] = q < cnt ? sp[int64_t(q) * (D * np)] : 0.0f;
+            l[q] = q < cnt ? int(lp[int64_t(q) * np]) : 0;
+        }
+        float gi[D][4] = {};
+        int oi_own = 1;
+        if (live) {
+            const float *own = sm + int(a.tv.lself[i]) * W;
+            oi_own = __float_as_int(own[(D + 1) * M]);
+            load_vec<float, 4>(own + off, fi);
+#pragma unroll
+            for (int d = 0; d < D; ++d) load_vec<float, 4>(own + (d + 1) * M + off, gi[d]);
+        }
+        AccumV<float, 4> acc;
+#pragma unroll
+        for (int m = 0; m < 4; ++m) { mn[m] = fi[m]; mx[m] = fi[m]; }
+        const int kw = __reduce_max_sync(0xffffffffu, cnt);
+        for (int k0 = 0; k0 < kw; k0 += G) {
+            sp += int64_t(G) * (D * np);
+            lp += int64_t(G) * np;
+            float vn[G], part[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            int ln[G];
+#pragma unroll
+            for (int q = 0; q < G; ++q) {
+                vn[q] = k0 + G + q < cnt ? sp[int64_t(q) * (D * np)] : 0.0f;
+                ln[q] = k0 + G + q < cnt ? int(lp[int64_t(q) * np]) : 0;
+            }
+#pragma unroll
+            for (int q = 0; q < G; ++q) {
+                float dk[D], wk[D];
+#pragma unroll
+                for (int d = 0; d < D; ++d) {
+                    dk[d] = __shfl_sync(0xffffffffu, v[q], lane0 + d);
+                    wk[d] = __shfl_sync(0xffffffffu, v[q], lane0 + D + d);
+                }
+                if (k0 + q >= cnt) continue;
+                const float *row = sm + l[q] * W;
+                float fj[4];
+                load_vec<float, 4>(row + off, fj);
+                if (need_ext) {
+#pragma unroll
+                    for (int m = 0; m < 4; ++m) { mn[m] = vmin(mn[m], fj[m]); mx[m] = vmax(mx[m], fj[m]); }
+                }
+                if (!wok) continue;
+                const int oj_own = __float_as_int(row[(D + 1) * M]);
+                float gj[D][4];
+#pragma unroll
+                for (int d = 0; d < D; ++d) load_vec<float, 4>(row + (d + 1) * M + off, gj[d]);
+                const bool epd1 = a.sc.strategy == HCC_EPD1;       // (EPD2 has no tile tables)
+                const int lo = oi_own < oj_own ? oi_own : oj_own;
+                const float si = (epd1 ? lo : oi_own) >= 2 ? 0.5f : 0.0f, sj = (epd1 ? lo : oj_own) >= 2 ? -0.5f : 0.0f;
+                const bool below = a.sc.aligned && (a.sc.max_order == 1 || lo < a.sc.max_order);
+                float S = 0.0f, pi[D], pj[D];
+#pragma unroll
+                for (int d = 0; d < D; ++d) {
+                    const float sw = (below ? wk[d] : dk[d]) > 0.0f ? a.ph.amax[d] : -a.ph.amax[d];
+                    S = (d == 0) ? wk[0] * sw : S + wk[d] * sw;
+                    pi[d] = si * dk[d];
+                    pj[d] = sj * dk[d];
+                }
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                    float A = gi[0][m] * pi[0], B = fj[m] - fi[m], cw = wk[0] * cm[0][m];
+#pragma unroll
+                    for (int d = 0; d < D; ++d) {
+                        if (d > 0) { A = A + gi[d][m] * pi[d]; cw = cw + wk[d] * cm[d][m]; }
+                        B = B + gj[d][m] * pj[d];
+                    }
+                    part[m] = part[m] + ((cw + S) * A + (cw - S) * B);
+                }
+            }
+            acc.add(part);
+#pragma unroll
+            for (int q = 0; q < G; ++q) { v[q] = vn[q]; l[q] = ln[q]; }
+        }
+#pragma unroll
+        for (int m = 0; m < 4; ++m) Kv[m] = -acc.s[m];
+        if (live && a.rough_words) {
+            bool r = !need_ext;
+#pragma unroll
+            for (int m = 0; m < 4; ++m) r = r || (mx[m] - mn[m]) > 1e-6f * (fabsf(mx[m]) + fabsf(mn[m]));
+            if (r) atomicOr(&rough[pl >> 5], 1u << (pl & 31));
+        }
+        if (wide_epilogue<D, M, PDE>(a, i, off, live, fi, Kv, mn, mx) && c == 0)
+            atomicOr(&failed[pl >> 5], 1u << (pl & 31));
+    }
+    if (!a.check && !a.rough_words) return;
+    __syncthreads();
+    const int64_t w32 = t * (HCC_TILE / 32) + threadIdx.x;
+    if (threadIdx.x >= HCC_TILE / 32 || w32 * 32 >= a.g.n) return;
+    if (a.check && failed[threadIdx.x]) {
+        a.tmask[w32] = failed[threadIdx.x];
+        a.ttiles[atomicAdd(a.tcount, 1u)] = int32_t(w32);
+    }
+    if (a.rough_words) a.rough_words[w32] = rough[threadIdx.x];
+}
+
 // The opt-in shared-memory limit of a block on the current device (the tile passes' dynamic allocation may go up
 // to it).
 inline int tile_smem_optin() {
@@ -3449,21 +3702,23 @@ struct StageInst {
     static void gather(const void *args, int64_t n, cudaStream_t s) {
         const StageArgs<T> &a = *static_cast<const StageArgs<T> *>(args);
         if constexpr (sizeof(T) == 4 && RDEG == 1) {
-            if (a.full && a.tile) {   // FP32 full pass with tile tables: neighbours staged in shared memory
-                static bool attr = false;
-                if (!attr) {
-                    cudaFuncSetAttribute(k_gather_tile<D, M, PDE, true>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, tile_smem_optin());
-                    cudaFuncSetAttribute(k_gather_tile<D, M, PDE, false>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, tile_smem_optin());
-                    attr = true;
+            if (a.full && a.tile) {   // FP32 full pass with tile tables: neighbours staged in shared memory (not wide systems)
+                if constexpr (!wide_system<T, M, PDE>()) {
+                    static bool attr = false;
+                    if (!attr) {
+                        cudaFuncSetAttribute(k_gather_tile<D, M, PDE, true>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, tile_smem_optin());
+                        cudaFuncSetAttribute(k_gather_tile<D, M, PDE, false>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, tile_smem_optin());
+                        attr = true;
+                    }
+                    const size_t smem = tile_gather_smem<D, M>(a.tv.umax);
+                    if (a.sc.limiter != HCC_LIMITER_NONE)
+                        k_gather_tile<D, M, PDE, true><<<unsigned(a.tv.ntiles), 2 * HCC_TILE, smem, s>>>(a);
+                    else
+                        k_gather_tile<D, M, PDE, false><<<unsigned(a.tv.ntiles), 2 * HCC_TILE, smem, s>>>(a);
+                    return;
                 }
-                const size_t smem = tile_gather_smem<D, M>(a.tv.umax);
-                if (a.sc.limiter != HCC_LIMITER_NONE)
-                    k_gather_tile<D, M, PDE, true><<<unsigned(a.tv.ntiles), 2 * HCC_TILE, smem, s>>>(a);
-                else
-                    k_gather_tile<D, M, PDE, false><<<unsigned(a.tv.ntiles), 2 * HCC_TILE, smem, s>>>(a);
-                return;
             }
             if (!a.full) {   // FP32 degree-1 worklist pass: split tiles
                 if (a.sc.limiter != HCC_LIMITER_NONE)
@@ -3511,18 +3766,26 @@ struct StageInst {
             if constexpr (RDEG == 1) {
                 if (a.full && a.tile) {   // full pass with tile tables: neighbours staged in shared memory
                     static bool attr = false;
-                    if (!attr) {
-                        cudaFuncSetAttribute(k_flux_tile<D, M, PDE, true>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, tile_smem_optin());
-                        cudaFuncSetAttribute(k_flux_tile<D, M, PDE, false>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, tile_smem_optin());
+                    if constexpr (wide_system<T, M, PDE>()) {
+                        if (!attr)
+                            cudaFuncSetAttribute(k_flux_wide<D, M, PDE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 tile_smem_optin() - 1024);
+                        const size_t smem = size_t(a.tv.umax) * wide_flux_row<D, M>() * sizeof(float);
+                        k_flux_wide<D, M, PDE><<<unsigned(a.tv.ntiles), kWideThreads, smem, s>>>(a);
+                    } else {
+                        if (!attr) {
+                            cudaFuncSetAttribute(k_flux_tile<D, M, PDE, true>,
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, tile_smem_optin());
+                            cudaFuncSetAttribute(k_flux_tile<D, M, PDE, false>,
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, tile_smem_optin());
+                        }
+                        const bool plain = a.sc.strategy == HCC_EPD1 && !a.sc.aligned;
+                        const size_t smem = tile_flux_smem<D, M>(a.tv.umax);
+                        if (plain)
+                            k_flux_tile<D, M, PDE, true><<<unsigned(a.tv.ntiles), 2 * HCC_TILE, smem, s>>>(a);
+                        else
+                            k_flux_tile<D, M, PDE, false><<<unsigned(a.tv.ntiles), 2 * HCC_TILE, smem, s>>>(a);
                     }
-                    const bool plain = a.sc.strategy == HCC_EPD1 && !a.sc.aligned;
-                    const size_t smem = tile_flux_smem<D, M>(a.tv.umax);
-                    if (plain)
-                        k_flux_tile<D, M, PDE, true><<<unsigned(a.tv.ntiles), 2 * HCC_TILE, smem, s>>>(a);
-                    else
-                        k_flux_tile<D, M, PDE, false><<<unsigned(a.tv.ntiles), 2 * HCC_TILE, smem, s>>>(a);
                     attr = true;
                     return;
                 }
