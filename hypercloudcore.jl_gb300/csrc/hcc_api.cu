@@ -501,6 +501,7 @@ template <typename T> StageArgs<T> base_args(hcc_ctx *c) {
     a.tcount = &c->lcounts->t;
     a.inadm = c->inadm;
     a.list_blocks = c->list_blocks;
+    a.sms = c->sms;
     a.flux_block = c->tune.flux_block;
     a.gather_block = c->tune.gather_block;
     a.delta = T(c->cfg.mood_delta);
@@ -620,6 +621,10 @@ template <typename T> StageArgs<T> stage_args(hcc_ctx *c, int s) {
         a.KInext = static_cast<T *>(c->KI[0]);
         a.implicit_mode = implicit_mode(c, 0);
         a.coef = coef;
+        a.trig_step = c->trig_step;
+        a.root = c->root;
+        a.lists = c->lcounts;
+        a.stats = c->mood_stats;
         return a;
     }
     const bool fin = (s + 1 == S);
@@ -653,7 +658,7 @@ PassFn pass_op(const hcc_ctx *c) {
 
 // Full pass of stage s: reconstruction, (EPD2 neighbourhood orders), flux with its fused epilogue (the failed
 // candidates go to the t list), and — without the MOOD check — the boundary conditions of the new candidate (with
-// the check they are part of the decrement launch). Returns the kernels launched.
+// the check they follow the fixed point). Returns the kernels launched.
 template <typename T> int enqueue_full(hcc_ctx *c, const StageArgs<T> &a, cudaStream_t st, bool prof) {
     const int64_t n = c->n;
     int k = 0;
@@ -682,20 +687,10 @@ template <typename T> int enqueue_full(hcc_ctx *c, const StageArgs<T> &a, cudaSt
     return k;
 }
 
-// Boundary conditions of the candidate Y + MOOD decrement + decision (one launch). Returns the kernels launched.
-int enqueue_drop(hcc_ctx *c, void *Y, cudaStream_t st, const cudaGraphConditionalHandle *h) {
+// MOOD decrement + decision (one launch). Returns the kernels launched.
+int enqueue_drop(hcc_ctx *c, cudaStream_t st, const cudaGraphConditionalHandle *h) {
     const int cap = c->cfg.max_mood_iterations > 0 ? c->cfg.max_mood_iterations : 64;
     DropArgs d{};
-    d.Y = Y;
-    d.rhos = c->rhos;
-    d.blist = c->blist;
-    d.bsrc = c->bsrc;
-    d.nb = c->nbnd;
-    d.M = c->M;
-    // boundary conditions of the candidate: up to eight blocks per SM (a few boundary particles a thread; every
-    // copy is a dependent load chain, so the pass is latency-bound and wants the whole GPU)
-    d.bc_blocks = c->nbnd > 0 ? int(std::min<int64_t>((c->nbnd + HCC_BLOCK - 1) / HCC_BLOCK,
-                                                      int64_t(8) * std::max(1, c->sms))) : 0;
     d.orders = c->orders;
     d.trig_step = c->trig_step;
     d.ttiles = c->ttiles;
@@ -707,14 +702,20 @@ int enqueue_drop(hcc_ctx *c, void *Y, cudaStream_t st, const cudaGraphConditiona
     d.has_handle = h != nullptr;
     if (h) d.h = *h;
     d.cap = cap;
-    launch_drop_decide(d, c->f32, c->drop_blocks, st);
+    launch_drop_decide(d, c->drop_blocks, st);
+    return 1;
+}
+
+// Boundary conditions of the converged candidate Y and its inadmissible count (one launch).
+int enqueue_stage_end(hcc_ctx *c, void *Y, cudaStream_t st) {
+    launch_stage_end(Y, c->rhos, c->blist, c->bsrc, c->nbnd, c->M, c->f32, c->sms, c->inadm, c->bnd, c->n,
+                     &c->mood_stats->inadmissible, st);
     return 1;
 }
 
 // One MOOD recompute (mood_checkpoint!, TimeSteppers.jl:471-475) over worklists: reconstruction of the changed
 // particles, which also pushes their reach (one hop; a second for EPD2; expand_mask!, MOOD.jl:343-351; none for
-// WENO, which reads no neighbour orders), then the flux and candidate of the reach. Its boundary conditions come
-// with the decrement launch that follows. Schemes without a reconstruction (WENO, CentralDivergence,
+// WENO, which reads no neighbour orders), then the flux and candidate of the reach. Schemes without a reconstruction (WENO, CentralDivergence,
 // UpwindDivergence) read no neighbour orders: no gather and no reach. Returns the kernels launched.
 template <typename T> int enqueue_recompute(hcc_ctx *c, const StageArgs<T> &a, cudaStream_t st, bool prof) {
     const int64_t n = c->n;
@@ -797,11 +798,12 @@ hcc_status ensure_learn_buffers(hcc_ctx *c) {
 }
 
 int enqueue_prologue(hcc_ctx *c, const void *args, cudaStream_t st) {
-    cudaMemsetAsync(c->lcounts, 0, sizeof(ListCounts), st);
-    cudaMemsetAsync(c->mood_stats, 0, sizeof(MoodStats), st);
-    launch_fill_i8(c->orders, int8_t(c->max_order), c->n, st);
-    cudaMemsetAsync(c->trig_step, 0, size_t(c->n), st);
-    int k = 0;
+    c->ops->stage1(args, c->n, st);
+    int k = 1;
+    if (implicit_mode(c, 0) == 1) {                // the donors' states after the implicit solve
+        launch_bc_apply(c->Y[0], c->rhos, c->blist, c->bsrc, c->nbnd, c->M, c->f32, st);
+        k += c->nbnd > 0;
+    }
     if (c->capture_feat || c->mlp) {
         const FeatArgs fa = feat_args(c, c->rhos);
         if (c->mlp) {
@@ -828,9 +830,7 @@ int enqueue_prologue(hcc_ctx *c, const void *args, cudaStream_t st) {
             k += 1;
         }
     }
-    c->ops->stage1(args, c->n, st);
-    launch_bc_apply(c->Y[0], c->rhos, c->blist, c->bsrc, c->nbnd, c->M, c->f32, st);
-    return k + 2 + (c->nbnd > 0);
+    return k;
 }
 
 // The step with the MOOD fixed points driven from the host (one counter read per decrement).
@@ -892,7 +892,7 @@ template <typename T> hcc_status run_step_host(hcc_ctx *c, double dt) {
             continue;
         }
         for (;;) {
-            c->launches += enqueue_drop(c, a.Ynext, c->stream, nullptr);
+            c->launches += enqueue_drop(c, c->stream, nullptr);
             if ((st = c->cuda(cudaMemcpyAsync(c->h_lcounts, c->lcounts, sizeof(ListCounts), cudaMemcpyDeviceToHost,
                                               c->stream), "MOOD counts")) != HCC_OK) return st;
             if ((st = read_mood_stats(c, c->stream)) != HCC_OK) return st;
@@ -905,8 +905,7 @@ template <typename T> hcc_status run_step_host(hcc_ctx *c, double dt) {
             c->launches += enqueue_recompute<T>(c, a, c->stream, c->prof != 0);
             if ((st = launch_check(c, "MOOD recompute")) != HCC_OK) return st;
         }
-        launch_count_inadmissible(c->inadm, c->bnd, n, &c->mood_stats->inadmissible, c->stream);
-        c->launches += 1;
+        c->launches += enqueue_stage_end(c, a.Ynext, c->stream);
         if (mv && s + 1 < S && (st = apply_positions(c, c->Xs[s + 1], c->mover.full_search_per_stage != 0)) != HCC_OK)
             return st;
     }
@@ -966,7 +965,7 @@ template <typename T> hcc_status capture_step(hcc_ctx *c, int parity) {
         cudaGraphConditionalHandle h;
         err = cudaGraphConditionalHandleCreate(&h, cg, 0, cudaGraphCondAssignDefault);
         if (err != cudaSuccess) break;
-        launches += enqueue_drop(c, a.Ynext, st, &h);
+        launches += enqueue_drop(c, st, &h);
         err = cudaStreamGetCaptureInfo(st, &cs, nullptr, &cg, &deps, nullptr, &ndeps);
         if (err != cudaSuccess) break;
         cudaGraphNodeParams np = {};
@@ -983,14 +982,12 @@ template <typename T> hcc_status capture_step(hcc_ctx *c, int parity) {
         err = cudaStreamBeginCaptureToGraph(c->stream2, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
         if (err != cudaSuccess) break;
         int bl = enqueue_recompute<T>(c, a, c->stream2, false);
-        bl += enqueue_drop(c, a.Ynext, c->stream2, &h);
+        bl += enqueue_drop(c, c->stream2, &h);
         body_launches += bl;
         cudaGraph_t body_out = nullptr;
         err = cudaStreamEndCapture(c->stream2, &body_out);
         if (err != cudaSuccess) break;
-        // interior candidates that are not admissible once the fixed point has converged
-        launch_count_inadmissible(c->inadm, c->bnd, c->n, &c->mood_stats->inadmissible, st);
-        launches += 1;
+        launches += enqueue_stage_end(c, a.Ynext, st);
     }
     if (err == cudaSuccess) err = cudaMemcpyAsync(c->mood_stats_host, c->mood_stats, sizeof(MoodStats),
                                                   cudaMemcpyDeviceToHost, st);

@@ -313,6 +313,9 @@ template <typename T> struct StageCoeffs {
     T dt_ii, inv_dt_ii;
 };
 
+struct ListCounts;
+struct MoodStats;
+
 // Arguments of the gather (reconstruction) and flux kernels.
 template <typename T> struct StageArgs {
     Geometry<T> g;
@@ -339,6 +342,7 @@ template <typename T> struct StageArgs {
     unsigned *rlcount;
     const int32_t *wlist;             // FP64 flux worklist pass over the reach: its particles
     int list_blocks;                  // grid of a worklist pass (warp-stride over the tiles)
+    int sms;                          // SMs of the device
     int flux_block, gather_block;     // block sizes of the full flux / gather passes (multiples of 32, <= 128)
     // epilogue: next candidate (Y_{s+1} or the final state) and the MOOD check of checkpoint s+1
     int form_next;
@@ -374,6 +378,11 @@ template <typename T> struct StageArgs {
     double *Xnext;
     int tile;                         // 1: full passes of this FP32 context are tile-staged (tv is valid)
     TileView tv;
+    // the step's start (k_stage1): flags, worklist counts and statistics to reset, donor roots of the boundary
+    uint8_t *trig_step;
+    const int32_t *root;
+    ListCounts *lists;
+    MoodStats *stats;
     uint32_t *tmask;                  // MOOD check: failed candidates (a ballot word per tile) ...
     int32_t *ttiles;                  // ... the tiles with a failure ...
     unsigned *tcount;                 // ... and their count
@@ -597,8 +606,11 @@ __host__ __device__ __forceinline__ double order_value(unsigned long long k) {
 void launch_force(const int32_t *ctiles, uint32_t *cmask, ListCounts *counts, int32_t *ctiles_out, int8_t *orders,
                   const uint8_t *bnd, const int32_t *cnt, const int32_t *nidx, int64_t npad, int32_t *forced,
                   uint32_t *fmask, int32_t *ftiles, int blocks, cudaStream_t s);
-void launch_count_inadmissible(const uint8_t *inadm, const uint8_t *bnd, int64_t n, unsigned long long *out,
-                               cudaStream_t s);
+// After a converged fixed point: the boundary conditions of the candidate Y and the count of inadmissible interior
+// candidates (added to *out).
+void launch_stage_end(void *Y, const void *rhos, const int32_t *blist, const int32_t *bsrc, int64_t nb, int M, int is_f32,
+                      int sms, const uint8_t *inadm, const uint8_t *bnd, int64_t n, unsigned long long *out,
+                      cudaStream_t s);
 void launch_shepard(const int32_t *cnt, const int32_t *nidx, const double *w, int64_t n, int64_t npad, double w0,
                     int sweeps, double *S, double *V, double *Vt, double *partial, cudaStream_t s);
 void launch_scale(double *V, int64_t n, double f, cudaStream_t s);
@@ -614,16 +626,10 @@ struct MoodStats {
     unsigned int tc_error, pad2;      // a tensor-core wait of the predictor gave up
 };
 
-// One launch after a flux pass with the MOOD check: boundary conditions of the new candidate (first bc_blocks
-// blocks), the MOOD decrement of the failed candidates into the changed list (the other blocks), and — in the last
-// block to finish — the decision of the fixed point (publish the changed list, reset the other lists, update the
-// statistics, and set the WHILE condition of a step graph when has_handle).
+// One launch after a flux pass with the MOOD check: the MOOD decrement of the failed candidates into the changed list,
+// and — in the last block to finish — the decision of the fixed point (publish the changed list, reset the other lists,
+// update the statistics, and set the WHILE condition of a step graph when has_handle).
 struct DropArgs {
-    void *Y;
-    const void *rhos;
-    const int32_t *blist, *bsrc;
-    int64_t nb;
-    int M, bc_blocks;
     int8_t *orders;
     uint8_t *trig_step;
     const int32_t *ttiles;
@@ -635,7 +641,7 @@ struct DropArgs {
     cudaGraphConditionalHandle h;
     int has_handle, cap;
 };
-void launch_drop_decide(const DropArgs &a, int is_f32, int drop_blocks, cudaStream_t s);
+void launch_drop_decide(const DropArgs &a, int drop_blocks, cudaStream_t s);
 void launch_gather_rows(const void *slotmajor, void *rowmajor, const int32_t *cnt, const int64_t *rowstart,
                         int64_t n, int64_t npad, int width, int elem_bytes, cudaStream_t s);
 // FP64 FMA rate of the current device in TFLOP/s (2 FLOP per FMA), from a timed kernel on every SM.

@@ -3091,15 +3091,26 @@ __global__ void __launch_bounds__(128) k_central(const StageArgs<T> a) {
     }
 }
 
-// form_candidate!(ts, eq, pg, 1, dt, t) (TimeSteppers.jl:365-397) for stage 1: Y_1 = Uⁿ (interior),
-// the start-of-step state (boundary), then the implicit part. Boundary conditions follow in their own kernel.
+// The start of a step: orders, flags, worklist counts and statistics reset, and form_candidate!(ts, eq, pg, 1, dt, t)
+// (TimeSteppers.jl:365-397) for stage 1: Y_1 = Uⁿ (interior; then the implicit part) and the boundary conditions of the
+// boundary (apply_boundary_conditions!, BoundaryConditions.jl:43-130): the donor's start-of-step state or their own.
+// (Stages whose implicit part changes Y_1 take the donors' states from a pass after this one.) One launch: the three
+// resets, the fill, the copy and the boundary pass it replaces were about 2 us each in a step's graph.
 template <typename T, int D, int M, int PDE, int RDEG>
 __global__ void k_stage1(const StageArgs<T> a) {
     const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i == 0) {
+        *a.lists = ListCounts{};
+        *a.stats = MoodStats{};
+    }
     if (i >= a.g.n) return;
+    a.orders[i] = int8_t(a.sc.max_order);
+    a.trig_step[i] = 0;
+    const bool bnd = a.g.bnd[i];
+    const int32_t root = bnd ? a.root[i] : -1;
     T Y[M];
-    load_vec<T, M>(a.Un + i * M, Y);
-    if (!a.g.bnd[i] && a.implicit_mode) {
+    load_vec<T, M>(a.Un + (root >= 0 ? int64_t(root) : i) * M, Y);
+    if (!bnd && a.implicit_mode) {
         T KIo[M];
         implicit_part<T, D, M, PDE>(a, i, Y, KIo);
         store_vec<T, M>(a.KInext + i * M, KIo);

@@ -33,29 +33,20 @@ __global__ void k_bc(T *Y, const T *rhos, const int32_t *blist, const int32_t *b
     for (int m = 0; m < M; ++m) Y[b * M + m] = (src >= 0) ? Y[int64_t(src) * M + m] : rhos[b * M + m];
 }
 
-// After a flux pass with the MOOD check, one launch: the boundary conditions of the new candidate (blocks below
-// bc_blocks; apply_boundary_conditions!, BoundaryConditions.jl:43-130), _mood_drop! (MOOD.jl:299-309) over the
-// failed candidates — an order above 1 drops by one and the particle joins the changed list — and, in the last
-// block to finish, the loop condition of mood_checkpoint! (TimeSteppers.jl:454-477): no changed order ends the loop;
-// otherwise the flagged count grows and the loop repeats, unless the checkpoint already ran `cap` recomputes (the
-// timeout flag ends it). The decision publishes the changed list and clears the other lists for the next pass.
-template <typename T>
+// After a flux pass with the MOOD check: _mood_drop! (MOOD.jl:299-309) over the failed candidates — an order above 1
+// drops by one and the particle joins the changed list — and, in the last block to finish, the loop condition of
+// mood_checkpoint! (TimeSteppers.jl:454-477): no changed order ends the loop; otherwise the flagged count grows and the
+// loop repeats, unless the checkpoint already ran `cap` recomputes (the timeout flag ends it). The decision publishes
+// the changed list and clears the other lists for the next pass. Latency-bound (a chain of dependent loads and the
+// blocks' counter). The boundary conditions of the candidate are not read within the fixed point and follow it
+// (k_stage_end).
 __global__ void k_drop_decide(const DropArgs a) {
-    if (int(blockIdx.x) < a.bc_blocks) {
-        T *Y = static_cast<T *>(a.Y);
-        const T *rhos = static_cast<const T *>(a.rhos);
-        for (int64_t q = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; q < a.nb;
-             q += int64_t(a.bc_blocks) * blockDim.x) {
-            const int64_t b = a.blist[q];
-            const int32_t src = a.bsrc[q];
-            for (int m = 0; m < a.M; ++m) Y[b * a.M + m] = (src >= 0) ? Y[int64_t(src) * a.M + m] : rhos[b * a.M + m];
-        }
-    } else {
+    {
         // one warp per tile of failed candidates; the changed members form the tile's word of the c list
         const unsigned nt = a.counts->t;
         const int lane = int(threadIdx.x & 31);
-        const unsigned warp = ((blockIdx.x - unsigned(a.bc_blocks)) * blockDim.x + threadIdx.x) >> 5;
-        const unsigned nwarps = ((gridDim.x - unsigned(a.bc_blocks)) * blockDim.x) >> 5;
+        const unsigned warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+        const unsigned nwarps = (gridDim.x * blockDim.x) >> 5;
         for (unsigned q = warp; q < nt; q += nwarps) {
             const int32_t tile = a.ttiles[q];
             const uint32_t word = a.tmask[tile];
@@ -241,13 +232,36 @@ __global__ void k_u2_range(const T *U, int64_t n, int M, unsigned long long *key
     }
 }
 
-// Interior candidates that are not admissible once a fixed point has converged (_count_inadmissible,
-// TimeSteppers.jl:481-490).
-__global__ void k_count_inadm(const uint8_t *inadm, const uint8_t *bnd, int64_t n, unsigned long long *out) {
-    int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    const unsigned ia = (i < n && !bnd[i] && inadm[i]) ? 1u : 0u;
-    const unsigned b = __ballot_sync(0xffffffffu, ia);
-    if ((threadIdx.x & 31) == 0 && b) atomicAdd(out, (unsigned long long)__popc(b));
+// Once a fixed point has converged: the boundary conditions of its candidate (apply_boundary_conditions!,
+// BoundaryConditions.jl:43-130; the first bc_blocks blocks, every copy a dependent load chain) and the interior
+// candidates that are not admissible (_count_inadmissible, TimeSteppers.jl:481-490; the other blocks, 16 bytes of each
+// mask a thread).
+template <typename T>
+__global__ void k_stage_end(T *Y, const T *rhos, const int32_t *blist, const int32_t *bsrc, int64_t nb, int M,
+                            int bc_blocks, const uint8_t *inadm, const uint8_t *bnd, int64_t n,
+                            unsigned long long *out) {
+    if (int(blockIdx.x) < bc_blocks) {
+        for (int64_t q = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; q < nb; q += int64_t(bc_blocks) * blockDim.x) {
+            const int64_t b = blist[q];
+            const int32_t src = bsrc[q];
+            for (int m = 0; m < M; ++m) Y[b * M + m] = (src >= 0) ? Y[int64_t(src) * M + m] : rhos[b * M + m];
+        }
+        return;
+    }
+    // (the masks are byte arrays of a multiple of 32 entries)
+    const int64_t q = int64_t(int(blockIdx.x) - bc_blocks) * blockDim.x + threadIdx.x;
+    unsigned bad = 0;
+    if (16 * q < n) {
+        const uint4 f = reinterpret_cast<const uint4 *>(inadm)[q], b = reinterpret_cast<const uint4 *>(bnd)[q];
+        const uint32_t fw[4] = {f.x, f.y, f.z, f.w}, bw[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int w = 0; w < 4; ++w)
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (16 * q + 4 * w + e < n && ((fw[w] >> (8 * e)) & 0xffu) && !((bw[w] >> (8 * e)) & 0xffu)) ++bad;
+    }
+    bad = __reduce_add_sync(0xffffffffu, bad);
+    if ((threadIdx.x & 31) == 0 && bad) atomicAdd(out, (unsigned long long)bad);
 }
 
 // total_mass (Volumes.jl:103-107) in FP64.
@@ -356,10 +370,21 @@ void launch_bc_apply(void *Y, const void *rhos, const int32_t *blist, const int3
         k_bc<double><<<grid_for(nb), HCC_BLOCK, 0, s>>>(static_cast<double *>(Y), static_cast<const double *>(rhos),
                                                          blist, bsrc, nb, M);
 }
-void launch_drop_decide(const DropArgs &a, int is_f32, int drop_blocks, cudaStream_t s) {
-    const unsigned blocks = unsigned(a.bc_blocks + std::max(1, drop_blocks));
-    if (is_f32) k_drop_decide<float><<<blocks, HCC_BLOCK, 0, s>>>(a);
-    else k_drop_decide<double><<<blocks, HCC_BLOCK, 0, s>>>(a);
+void launch_drop_decide(const DropArgs &a, int drop_blocks, cudaStream_t s) {
+    k_drop_decide<<<unsigned(std::max(1, drop_blocks)), HCC_BLOCK, 0, s>>>(a);
+}
+void launch_stage_end(void *Y, const void *rhos, const int32_t *blist, const int32_t *bsrc, int64_t nb, int M, int is_f32,
+                      int sms, const uint8_t *inadm, const uint8_t *bnd, int64_t n, unsigned long long *out,
+                      cudaStream_t s) {
+    if (n <= 0) return;
+    const int bc_blocks = nb > 0 ? int(std::min<int64_t>(grid_for(nb), int64_t(8) * std::max(1, sms))) : 0;
+    const unsigned g = unsigned(bc_blocks) + grid_for((n + 15) / 16);
+    if (is_f32)
+        k_stage_end<float><<<g, HCC_BLOCK, 0, s>>>(static_cast<float *>(Y), static_cast<const float *>(rhos), blist, bsrc,
+                                                   nb, M, bc_blocks, inadm, bnd, n, out);
+    else
+        k_stage_end<double><<<g, HCC_BLOCK, 0, s>>>(static_cast<double *>(Y), static_cast<const double *>(rhos), blist,
+                                                    bsrc, nb, M, bc_blocks, inadm, bnd, n, out);
 }
 void launch_reach_hop2(ListCounts *counts, const int32_t *dtiles, int32_t *dtiles_out, uint32_t *dmask,
                        uint32_t *words1, int32_t *dlist, const int32_t *cnt, const int32_t *nidx, int64_t npad,
@@ -387,10 +412,6 @@ void launch_force(const int32_t *ctiles, uint32_t *cmask, ListCounts *counts, in
                   uint32_t *fmask, int32_t *ftiles, int blocks, cudaStream_t s) {
     k_force_push<<<blocks, HCC_BLOCK, 0, s>>>(ctiles, cmask, counts, orders, bnd, cnt, nidx, npad, forced, fmask, ftiles);
     k_force_apply<<<blocks, HCC_BLOCK, 0, s>>>(counts, ftiles, fmask, forced, orders, cmask, ctiles_out);
-}
-void launch_count_inadmissible(const uint8_t *inadm, const uint8_t *bnd, int64_t n, unsigned long long *out,
-                               cudaStream_t s) {
-    if (n > 0) k_count_inadm<<<grid_for(n), HCC_BLOCK, 0, s>>>(inadm, bnd, n, out);
 }
 // ShepardVolumes (Volumes.jl:183-229): kernel sums and the 1/S start, the partition-of-unity sweeps, and the
 // clamped volumes' block partial sums for the renormalisation.
