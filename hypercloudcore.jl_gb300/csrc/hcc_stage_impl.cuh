@@ -1959,13 +1959,15 @@ __global__ void __launch_bounds__(2 * HCC_TILE, tile_gather_min_blocks<D, M>()) 
     }
 }
 
-// Flux pass, two threads per particle of the tile (slots k = h, h + 2, ... for h = 0, 1); the second writes its
-// compensated partial sums and extrema to shared memory, the first combines them and runs the epilogue.
+// Flux pass, HT threads per particle of the tile (slots k = h, h + HT, ... for h < HT); the others write their
+// compensated partial sums and extrema to shared memory, the first combines them and runs the epilogue. Two threads and
+// two blocks an SM, or (few tiles) four threads and one block, which takes half as long over a tile: the better one is
+// the one whose last wave leaves less of the chip idle (flux_tile_wide).
 template <int D, int M> constexpr int tile_flux_min_blocks() { return M >= 8 ? 1 : 2; }
 
 // PLAIN: EPD1 interface orders and the plain Rusanov flux (the usual configuration), known at compile time.
-template <int D, int M, int PDE, bool PLAIN>
-__global__ void __launch_bounds__(2 * HCC_TILE, tile_flux_min_blocks<D, M>()) k_flux_tile(const StageArgs<float> a) {
+template <int D, int M, int PDE, bool PLAIN, int HT>
+__global__ void __launch_bounds__(HT * HCC_TILE, HT == 2 ? tile_flux_min_blocks<D, M>() : 1) k_flux_tile(const StageArgs<float> a) {
     extern __shared__ __align__(16) float sm[];
     constexpr int W = tile_flux_row<D, M>();
     constexpr int RW = M + D * M;                 // used words of a row: the state, then the gradient
@@ -1982,12 +1984,12 @@ __global__ void __launch_bounds__(2 * HCC_TILE, tile_flux_min_blocks<D, M>()) k_
     const int64_t i = t * HCC_TILE + pl;
     const bool live = i < a.g.n && !a.g.bnd[i];
     const int64_t np = a.g.npad;
-    // this thread's slots h, h + 2, ...: union places PF slots ahead (a rotating window), or in groups of PF with the
+    // this thread's slots h, h + HT, ...: union places PF slots ahead (a rotating window), or in groups of PF with the
     // next group in flight (HCC_TILE_FLUX_GROUP > 0: the slot body unrolled over the group)
     // (wide states, M >= 8, keep the window: the unrolled group spills their registers)
     constexpr int GROUP = M >= 8 ? 0 : HCC_TILE_FLUX_GROUP;
     constexpr int PF = GROUP > 0 ? GROUP : HCC_TILE_FLUX_PF;
-    const int64_t lstep = 2 * np;
+    const int64_t lstep = HT * np;
     const uint16_t *lp = a.tv.lidx + int64_t(h) * np + i;
     int cnt = 0, li = 0, mine = 0;
     bool wok = false;
@@ -2004,7 +2006,7 @@ __global__ void __launch_bounds__(2 * HCC_TILE, tile_flux_min_blocks<D, M>()) k_
 #pragma unroll
             for (int e = 0; e < D; ++e) B[d][e] = cf[D + d * D + e];
         }
-        mine = cnt > h ? (cnt - h + 1) / 2 : 0;
+        mine = cnt > h ? (cnt - h + HT - 1) / HT : 0;
 #pragma unroll
         for (int q = 0; q < PF; ++q) lb[q] = q < mine ? int(lp[int64_t(q) * lstep]) : 0;
         lp += int64_t(PF) * lstep;
@@ -2100,7 +2102,7 @@ __global__ void __launch_bounds__(2 * HCC_TILE, tile_flux_min_blocks<D, M>()) k_
 #pragma unroll
                     for (int q = 0; q < PF; ++q) {
                         if (s0 + q >= mine) break;
-                        slot(lb[q], h + 2 * (s0 + q));
+                        slot(lb[q], h + HT * (s0 + q));
                     }
 #pragma unroll
                     for (int q = 0; q < PF; ++q) lb[q] = ln[q];
@@ -2112,7 +2114,7 @@ __global__ void __launch_bounds__(2 * HCC_TILE, tile_flux_min_blocks<D, M>()) k_
                     for (int q = 0; q + 1 < PF; ++q) lb[q] = lb[q + 1];
                     lb[PF - 1] = s + PF < mine ? int(*lp) : 0;
                     lp += lstep;
-                    slot(l, h + 2 * s);
+                    slot(l, h + HT * s);
                 }
             }
             blk.flush();
@@ -2129,18 +2131,19 @@ __global__ void __launch_bounds__(2 * HCC_TILE, tile_flux_min_blocks<D, M>()) k_
                 for (int m = 0; m < M; ++m) { mn[m] = vmin(mn[m], r[m]); mx[m] = vmax(mx[m], r[m]); }
             }
         }
-        if (h == 1) {
+        if (h > 0) {
+            FluxPart<float, M> &part = parts[(h - 1) * HCC_TILE + pl];
 #pragma unroll
             for (int m = 0; m < M; ++m) {
-                parts[pl].s[m] = acc.s[m];
-                parts[pl].c[m] = acc.c[m];
-                parts[pl].mn[m] = mn[m];
-                parts[pl].mx[m] = mx[m];
+                part.s[m] = acc.s[m];
+                part.c[m] = acc.c[m];
+                part.mn[m] = mn[m];
+                part.mx[m] = mx[m];
             }
         }
     }
     __syncthreads();
-    if (h == 1) return;
+    if (h > 0) return;
     bool f = false, rough = false;
     if (i < a.g.n) {
         if (a.g.bnd[i]) {
@@ -2149,16 +2152,22 @@ __global__ void __launch_bounds__(2 * HCC_TILE, tile_flux_min_blocks<D, M>()) k_
             for (int m = 0; m < M; ++m) z[m] = 0.0f;
             store_vec<float, M>(a.K + i * M, z);
         } else {
-            // the two compensated partials: their sum, minus both compensations and the rounding error of that sum
+            // the compensated partials: their sum, minus their compensations and the rounding errors of that sum
             float Kv[M];
 #pragma unroll
             for (int m = 0; m < M; ++m) {
-                const float s1 = parts[pl].s[m];
-                const float u = acc.s[m] + s1;
-                const float cm = (u - acc.s[m]) - s1;
-                Kv[m] = -(u - ((acc.c[m] + parts[pl].c[m]) + cm));
-                mn[m] = vmin(mn[m], parts[pl].mn[m]);
-                mx[m] = vmax(mx[m], parts[pl].mx[m]);
+                float sum = acc.s[m], comp = acc.c[m];
+#pragma unroll
+                for (int v = 0; v < HT - 1; ++v) {
+                    const FluxPart<float, M> &part = parts[v * HCC_TILE + pl];
+                    const float u = sum + part.s[m];
+                    const float cm = (u - sum) - part.s[m];
+                    comp = (comp + part.c[m]) + cm;
+                    sum = u;
+                    mn[m] = vmin(mn[m], part.mn[m]);
+                    mx[m] = vmax(mx[m], part.mx[m]);
+                }
+                Kv[m] = -(sum - comp);
             }
             if (a.rough_words) {
                 bool r = !need_ext;
@@ -2441,8 +2450,17 @@ inline int tile_smem_optin() {
 template <int D, int M> inline size_t tile_gather_smem(int umax) {
     return (size_t(umax) * tile_gather_row<D, M>() + size_t(HCC_TILE) * D * M) * sizeof(float);
 }
-template <int D, int M> inline size_t tile_flux_smem(int umax) {
-    return size_t(umax) * (4 + tile_flux_row<D, M>()) * sizeof(float) + size_t(HCC_TILE) * sizeof(FluxPart<float, M>);
+template <int D, int M> inline size_t tile_flux_smem(int umax, int threads) {
+    return size_t(umax) * (4 + tile_flux_row<D, M>()) * sizeof(float) +
+           size_t(threads - 1) * HCC_TILE * sizeof(FluxPart<float, M>);
+}
+// Whether a full flux pass of `ntiles` tiles takes four threads a particle: the waves of one block an SM, each half as
+// long, against those of two blocks an SM. Long passes keep two threads (their last wave is a small part).
+template <int D, int M> inline bool flux_tile_wide(const StageArgs<float> &a) {
+    if (M >= 8 || D < 3 || a.tv.ntiles > int64_t(16) * a.sms) return false;
+    if (tile_flux_smem<D, M>(a.tv.umax, 4) > size_t(tile_smem_optin())) return false;
+    const int64_t w4 = (a.tv.ntiles + a.sms - 1) / a.sms, w2 = (a.tv.ntiles + 2 * a.sms - 1) / (2 * a.sms);
+    return w4 < 2 * w2;
 }
 
 // ----------------------------------------------------------------------------------- WENO (scalar)
@@ -3776,28 +3794,27 @@ struct StageInst {
         if constexpr (sizeof(T) == 4) {
             if constexpr (RDEG == 1) {
                 if (a.full && a.tile) {   // full pass with tile tables: neighbours staged in shared memory
-                    static bool attr = false;
                     if constexpr (wide_system<T, M, PDE>()) {
-                        if (!attr)
-                            cudaFuncSetAttribute(k_flux_wide<D, M, PDE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 tile_smem_optin() - 1024);
+                        cudaFuncSetAttribute(k_flux_wide<D, M, PDE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             tile_smem_optin() - 1024);
                         const size_t smem = size_t(a.tv.umax) * wide_flux_row<D, M>() * sizeof(float);
                         k_flux_wide<D, M, PDE><<<unsigned(a.tv.ntiles), kWideThreads, smem, s>>>(a);
                     } else {
-                        if (!attr) {
-                            cudaFuncSetAttribute(k_flux_tile<D, M, PDE, true>,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, tile_smem_optin());
-                            cudaFuncSetAttribute(k_flux_tile<D, M, PDE, false>,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, tile_smem_optin());
-                        }
+                        auto go = [&](auto kernel, int threads) {
+                            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tile_smem_optin());
+                            kernel<<<unsigned(a.tv.ntiles), threads * HCC_TILE, tile_flux_smem<D, M>(a.tv.umax, threads),
+                                     s>>>(a);
+                        };
                         const bool plain = a.sc.strategy == HCC_EPD1 && !a.sc.aligned;
-                        const size_t smem = tile_flux_smem<D, M>(a.tv.umax);
-                        if (plain)
-                            k_flux_tile<D, M, PDE, true><<<unsigned(a.tv.ntiles), 2 * HCC_TILE, smem, s>>>(a);
-                        else
-                            k_flux_tile<D, M, PDE, false><<<unsigned(a.tv.ntiles), 2 * HCC_TILE, smem, s>>>(a);
+                        if constexpr (D == 3 && M < 8) {
+                            if (plain && flux_tile_wide<D, M>(a)) {
+                                go(k_flux_tile<D, M, PDE, true, 4>, 4);
+                                return;
+                            }
+                        }
+                        if (plain) go(k_flux_tile<D, M, PDE, true, 2>, 2);
+                        else go(k_flux_tile<D, M, PDE, false, 2>, 2);
                     }
-                    attr = true;
                     return;
                 }
             }
