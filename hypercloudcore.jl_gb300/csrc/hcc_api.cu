@@ -213,6 +213,10 @@ struct hcc_ctx {
     float *dist32 = nullptr, *w32 = nullptr, *dw32 = nullptr, *dw1_32 = nullptr, *inv_r32 = nullptr, *gw32 = nullptr;
     int32_t *status = nullptr, *root = nullptr;
     int32_t *blist = nullptr, *bsrc = nullptr; int64_t nbnd = 0;
+    int32_t *ilist = nullptr;                    // the interior particles
+    // whether full passes run over the interior list: from one ghost in ten on. (A list costs the slot streams their
+    // alignment to the warps; without ghosts worth skipping it only loses.)
+    bool skip_ghosts() const { return nbnd * 10 >= n; }
     // state (element type double or float)
     void *rhos = nullptr, *cand = nullptr, *grad = nullptr;
     void *xfer = nullptr;                        // n*M doubles: staging of host-precision conversions
@@ -227,6 +231,7 @@ struct hcc_ctx {
     ListCounts *lcounts = nullptr, *h_lcounts = nullptr;
     int list_blocks = 1, drop_blocks = 1;
     int sms = 1;                                 // SM count of the device
+    int half_sm = 0;                             // shared memory of a block that leaves room for a second one on its SM
     hcc_tuning tune{128, 128, 8, 2};             // launch shapes of the step (hcc_set_tuning / hcc_autotune)
     TileTables tiles;                            // tile staging of the FP32 full passes (hcc_tiles.cu)
     int tile_enabled = 1;
@@ -398,7 +403,7 @@ struct hcc_ctx {
         dfree(pos); dfree(bnd); dfree(tags); dfree(vol); dfree(bin_of); dfree(cellp); dfree(cnt);
         dfree(pos32); dfree(pmax32); dfree(wops); dfree(wcnt); dfree(wchol); dfree(wok); dfree(wflux64);
         dfree(ok_r); dfree(ok_d); dfree(ok_1); dfree(inv_r64); dfree(inv_d64); dfree(inv_r32);
-        dfree(status); dfree(root); dfree(blist); dfree(bsrc);
+        dfree(status); dfree(root); dfree(blist); dfree(bsrc); dfree(ilist);
         for (void **p : {&rhos, &cand, &grad, &xfer}) { if (*p) cudaFree(*p); *p = nullptr; }
         for (int s = 0; s < HCC_MAX_STAGES; ++s)
             for (void **p : {&Y[s], &KE[s], &KI[s]}) { if (*p) cudaFree(*p); *p = nullptr; }
@@ -502,6 +507,10 @@ template <typename T> StageArgs<T> base_args(hcc_ctx *c) {
     a.inadm = c->inadm;
     a.list_blocks = c->list_blocks;
     a.sms = c->sms;
+    const bool tiled = sizeof(T) == 4 && c->tiles.ok && c->tile_enabled && !c->moving();
+    const bool listed = tiled ? c->tiles.listed : c->skip_ghosts();
+    a.ilist = listed ? c->ilist : nullptr;
+    a.nfull = listed ? c->n_interior : c->n;
     a.flux_block = c->tune.flux_block;
     a.gather_block = c->tune.gather_block;
     a.delta = T(c->cfg.mood_delta);
@@ -510,7 +519,7 @@ template <typename T> StageArgs<T> base_args(hcc_ctx *c) {
     a.u2_h = T(c->h);
     a.u2_range = c->u2_plateau_on() ? c->u2_keys : nullptr;
     if constexpr (sizeof(T) == 4) {
-        if (c->tiles.ok && c->tile_enabled && !c->moving()) {
+        if (tiled) {
             a.tile = 1;
             TileView &v = a.tv;
             v.ntiles = c->tiles.ntiles; v.ustart = c->tiles.ustart; v.uid = c->tiles.uid; v.upos = c->tiles.upos;
@@ -676,6 +685,8 @@ template <typename T> int enqueue_full(hcc_ctx *c, const StageArgs<T> &a, cudaSt
         launch_u2_range(a.U, n, c->M, c->f32, c->u2_keys, st);
         ++k;
     }
+    // (an interior list's rough marks are set one by one)
+    if (a.rough_words && a.ilist) cudaMemsetAsync(a.rough_words, 0, size_t(c->npad / 32) * sizeof(uint32_t), st);
     if (prof) c->prof_begin(1);
     pass_op(c)(&a, n, st);
     if (prof) c->prof_end();
@@ -1242,6 +1253,13 @@ hcc_status hcc_create(const hcc_config *cfg, int64_t capacity, hcc_ctx **out) {
         if ((st = c->cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count")) != HCC_OK)
             return st;
         c->sms = std::max(1, sms);
+        int sm = 0, own = 0;
+        if ((st = c->cuda(cudaDeviceGetAttribute(&sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev), "shared memory")) !=
+                HCC_OK ||
+            (st = c->cuda(cudaDeviceGetAttribute(&own, cudaDevAttrReservedSharedMemoryPerBlock, dev), "shared memory")) !=
+                HCC_OK)
+            return st;
+        c->half_sm = std::max(0, sm / 2 - own);
         c->apply_tuning();   // worklist passes: a few resident blocks per SM, grid-stride
     }
     if ((st = c->cuda(cudaMallocHost(reinterpret_cast<void **>(&c->mood_stats_host), sizeof(MoodStats)),
@@ -1353,15 +1371,18 @@ hcc_status hcc_upload_cloud(hcc_ctx *c, int64_t n, const double *pos, const uint
     HCC_TRY(c->cuda(cudaMemcpyAsync(c->bnd, is_boundary, n, cudaMemcpyHostToDevice, c->stream), "upload is_boundary"));
     HCC_TRY(c->cuda(cudaMemcpyAsync(c->tags, tags, n * sizeof(int32_t), cudaMemcpyHostToDevice, c->stream), "upload tags"));
     HCC_TRY(c->cuda(cudaMemcpyAsync(c->vol, v.data(), n * sizeof(double), cudaMemcpyHostToDevice, c->stream), "upload volumes"));
-    std::vector<int32_t> bl;
-    for (int64_t i = 0; i < n; ++i)
-        if (is_boundary[i]) bl.push_back(int32_t(i));
+    std::vector<int32_t> bl, il;
+    for (int64_t i = 0; i < n; ++i) (is_boundary[i] ? bl : il).push_back(int32_t(i));
     c->nbnd = int64_t(bl.size());
     HCC_TRY(c->reserve(c->blist, bl.size(), "boundary list"));
     HCC_TRY(c->reserve(c->bsrc, bl.size(), "boundary sources"));
     if (!bl.empty())
         HCC_TRY(c->cuda(cudaMemcpyAsync(c->blist, bl.data(), bl.size() * sizeof(int32_t), cudaMemcpyHostToDevice,
                                         c->stream), "boundary list"));
+    HCC_TRY(c->reserve(c->ilist, il.size(), "interior list"));
+    if (!il.empty())
+        HCC_TRY(c->cuda(cudaMemcpyAsync(c->ilist, il.data(), il.size() * sizeof(int32_t), cudaMemcpyHostToDevice,
+                                        c->stream), "interior list"));
     HCC_TRY(c->sync("upload cloud"));
     c->have_cloud = true;
     return HCC_OK;
@@ -1636,8 +1657,9 @@ hcc_status build_tiles(hcc_ctx *c) {
     const int W = 4 + 4 * (groups % 2 == 1 ? groups : groups + 1);
     const long budget = 200L * 1024 - long(HCC_TILE) * 4 * M * long(sizeof(float));
     TileBuild b{};
-    b.n = c->n; b.npad = c->npad; b.D = D; b.kmax = std::max(c->kmax, 1);
-    b.cnt = c->cnt; b.nidx = c->nidx; b.pos = c->pos;
+    b.n = c->n; b.npad = c->npad; b.D = D;
+    b.kmax = std::max(c->kmax, 1);
+    b.bnd = c->bnd; b.cnt = c->cnt; b.nidx = c->nidx; b.pos = c->pos;
     for (int d = 0; d < D; ++d) {
         b.periodic[d] = c->cfg.periodic[d];
         const double L = c->cfg.domain_max[d] - c->cfg.domain_min[d];
@@ -1648,7 +1670,20 @@ hcc_status build_tiles(hcc_ctx *c) {
     b.inv_r = c->inv_r64; b.inv_d = c->inv_d64; b.ok_r = c->ok_r; b.ok_d = c->ok_d;
     b.invL = c->invL;
     b.wscale = c->cfg.weight_alpha / (c->cfg.radius * c->cfg.radius);
-    b.max_union = int(std::max(0L, budget / (4L * W)));
+    const int most = int(std::max(0L, budget / (4L * W)));
+    // Tiles of the interior list, where there is one, unless their unions cost the flux pass its second block on an SM:
+    // 128 interior particles spread wider than 128 consecutive ones (in 3-D at most 1162 against 963 entries on 64^3).
+    if (c->skip_ghosts()) {
+        b.members = c->ilist;
+        b.nmem = c->n_interior;
+        b.max_union = M >= 8 ? most : std::min(most, c->half_sm / (4 * W));
+        const hcc_status st = build_tile_tables(b, c->tiles, c->stream, c->err);
+        c->tiles.listed = c->tiles.ok;
+        if (st != HCC_OK || c->tiles.ok) return st;
+    }
+    b.members = nullptr;
+    b.nmem = c->n;
+    b.max_union = most;
     return build_tile_tables(b, c->tiles, c->stream, c->err);
 }
 

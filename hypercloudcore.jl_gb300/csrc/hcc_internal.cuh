@@ -277,7 +277,8 @@ template <typename T> struct Geometry {
 };
 
 // Tile staging of the FP32 full passes (MUSCL of order <= 2 with the degree-1 divergence fit, fixed grids): the
-// particles in tiles of HCC_TILE consecutive (Morton-numbered) particles; per tile the sorted union of its particles
+// particles of a full pass (every one, or the interior list) in tiles of HCC_TILE consecutive (Morton-numbered)
+// entries; per tile the sorted union of its particles
 // and of all their neighbours, which one thread block stages in shared memory; per slot the neighbour's place in its
 // particle's tile union (16 bits); per union entry the position relative to the tile's first particle as int32
 // multiples of the tile's power-of-two quantum (so x_j - x_i is an exact integer difference, rounded once when
@@ -295,7 +296,7 @@ struct TileView {
     const int4 *upos;                 // [utotal] quantised offsets from the tile's first particle (x, y, z, 0)
     const float *quantum;             // [ntiles] length of one unit of upos (a power of two)
     const uint16_t *lidx;             // [kmax * npad] slot k of particle i: place of its neighbour in the union
-    const uint16_t *lself;            // [n] place of the particle itself in its tile's union
+    const uint16_t *lself;            // [n] place of the particle itself in its tile's union (members)
     const float *coef;                // [n * cw] A (D), B (D*D), G (D*D), zero-padded to cw floats
     int cw;                           // a multiple of 4
     int umax;                         // largest union of any tile
@@ -329,6 +330,10 @@ template <typename T> struct StageArgs {
     double *wflux64;                  // FP64 Euler WENO: per particle F_d(U)_m and lambda_d of the stage state
     T *K;                             // K_E[s]
     int full;                         // 1: every particle; 0: the members of a tile worklist
+    // Particles of a full pass: entry q < nfull is ilist[q] (the interior ones, where ghosts are many: they have nothing
+    // to compute, yet share warps and tiles with those that do) or particle q (ilist == nullptr, nfull == n)
+    const int32_t *ilist;
+    int64_t nfull;
     // Worklist pass: tiles of 32 consecutive particles (one warp each, coalesced slot-major loads), the tiles to
     // visit, their count (device) and one member bit per particle (a word per tile).
     const int32_t *wtiles;
@@ -655,7 +660,10 @@ void launch_gather_rows_of(const void *src, void *dst, const int32_t *cnt, const
 // 2 (tile extent) + R), in which case the full passes keep the slot streams.
 struct TileBuild {
     int64_t n, npad;
+    const int32_t *members;           // the interior list, or nullptr: every particle
+    int64_t nmem;
     int D, kmax;
+    const uint8_t *bnd;
     const int32_t *cnt, *nidx;
     const double *pos;                // SoA [d * npad + i]
     int periodic[3];
@@ -675,6 +683,7 @@ struct TileTables {
     float *coef = nullptr;
     int cw = 0, umax = 0;
     float wscale = 0.f;
+    int listed = 0;                   // tiles of the interior list
     int ok = 0;
     void release();
 };

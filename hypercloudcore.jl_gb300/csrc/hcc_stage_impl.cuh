@@ -514,6 +514,11 @@ __device__ __forceinline__ void limit_slopes(const StageArgs<T> &a, int64_t i, i
         }
 }
 
+// The particle of entry q of a full pass, or -1 past its end.
+template <typename T> __device__ __forceinline__ int64_t full_particle(const StageArgs<T> &a, int64_t q) {
+    return q >= a.nfull ? -1 : (a.ilist ? int64_t(a.ilist[q]) : q);
+}
+
 // ----------------------------------------------------------------------------------- gather pass
 // update_content! of MUSCL (MUSCL.jl:351-384) with NoLimiter: starved-order lowering, cached full-order fit
 // (apply_weights, Interpolators.jl:585-602), dynamic lower-degree fit, or zero (order 1).
@@ -546,44 +551,41 @@ __device__ __forceinline__ void gather_one(const StageArgs<T> &a, const int64_t 
     if constexpr (sizeof(T) == 4 && RDEG == 1) {
         // FP32, degree 1: the cached fit as one weight vector per slot (nidx + D floats per slot)
         if (p == a.sc.max_order && p > 1 && a.g.ok_r[i] && a.g.gw) {
-            // slots in groups of G: the group's indices, weights and neighbour states are all in flight together
+            // slots in groups of G: the states of a group, and the indices and weights of the next, are in flight
+            // while the group is summed (an index is what its state's load waits for)
             constexpr int G = 4;
-            int k = 0;
-            for (; k + G <= cnt; k += G) {
-                int32_t j[G];
-                T gk[G][D], df[G][M];
+            int32_t j[G];
+            T gk[G][D];
+            auto stream = [&](int k, int32_t *jk, T(*g)[D]) {
 #pragma unroll
                 for (int q = 0; q < G; ++q) {
-                    j[q] = a.g.nidx[int64_t(k + q) * np + i];
+                    const bool on = k + q < cnt;
+                    jk[q] = on ? a.g.nidx[int64_t(k + q) * np + i] : int32_t(i);
 #pragma unroll
-                    for (int d = 0; d < D; ++d) gk[q][d] = a.g.gw[(int64_t(k + q) * D + d) * np + i];
+                    for (int d = 0; d < D; ++d) g[q][d] = on ? a.g.gw[(int64_t(k + q) * D + d) * np + i] : T(0);
                 }
+            };
+            stream(0, j, gk);
+            for (int k = 0; k < cnt; k += G) {
+                T df[G][M], gn[G][D];
+                int32_t jn[G];
 #pragma unroll
                 for (int q = 0; q < G; ++q) load_vec<T, M>(a.U + int64_t(j[q]) * M, df[q]);
-                asm volatile("" ::: "memory");        // the compiler keeps the group's loads ahead of its sums
+                stream(k + G, jn, gn);
 #pragma unroll
                 for (int q = 0; q < G; ++q) {
-                    if (lim) extend_extrema<T, M>(df[q], umin, umax);
+                    if (k + q < cnt) {
+                        if (lim) extend_extrema<T, M>(df[q], umin, umax);
 #pragma unroll
-                    for (int m = 0; m < M; ++m) {
-                        const T dm = df[q][m] - fi[m];
+                        for (int m = 0; m < M; ++m) {
+                            const T dm = df[q][m] - fi[m];
 #pragma unroll
-                        for (int b = 0; b < BR; ++b) out[b][m] = out[b][m] + gk[q][b] * dm;
+                            for (int b = 0; b < BR; ++b) out[b][m] = out[b][m] + gk[q][b] * dm;
+                        }
                     }
-                }
-            }
-            for (; k < cnt; ++k) {
-                const int32_t j = a.g.nidx[int64_t(k) * np + i];
-                T gk[D], df[M];
+                    j[q] = jn[q];
 #pragma unroll
-                for (int d = 0; d < D; ++d) gk[d] = a.g.gw[(int64_t(k) * D + d) * np + i];
-                load_vec<T, M>(a.U + int64_t(j) * M, df);
-                if (lim) extend_extrema<T, M>(df, umin, umax);
-#pragma unroll
-                for (int m = 0; m < M; ++m) {
-                    const T dm = df[m] - fi[m];
-#pragma unroll
-                    for (int b = 0; b < BR; ++b) out[b][m] = out[b][m] + gk[b] * dm;
+                    for (int d = 0; d < D; ++d) gk[q][d] = gn[q][d];
                 }
             }
             done = true;
@@ -860,8 +862,8 @@ __global__ void __launch_bounds__(32 * split_warps<M>()) k_gather_tiles(const St
 template <typename T, int D, int M, int PDE, int RDEG, bool LIM>
 __global__ void __launch_bounds__(128) k_gather(const StageArgs<T> a) {
     if (a.full) {
-        const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-        if (i < a.g.n) gather_one<T, D, M, PDE, RDEG, LIM>(a, i);
+        const int64_t i = full_particle(a, int64_t(blockIdx.x) * blockDim.x + threadIdx.x);
+        if (i >= 0) gather_one<T, D, M, PDE, RDEG, LIM>(a, i);
         return;
     }
     const unsigned nt = *a.wcount;
@@ -1476,6 +1478,21 @@ template <typename T> __device__ __forceinline__ void list_failures(const StageA
     if (f && atomicOr(&a.tmask[i >> 5], 1u << (i & 31)) == 0u) list_append(a.ttiles, a.tcount, int32_t(i >> 5));
 }
 
+// ... of a warp of a full pass: its tile's, or each particle's own of an interior list.
+template <typename T> __device__ __forceinline__ void full_failures(const StageArgs<T> &a, int64_t i, bool f) {
+    if (a.ilist) list_failures(a, i, f);
+    else tile_failures(a, i >> 5, f);              // (lane 0's, the only one used: every lane of a tile is in its warp)
+}
+// The predictor's rough marks of a warp of a full pass (an interior list's words are cleared before the pass).
+template <typename T> __device__ __forceinline__ void full_rough(const StageArgs<T> &a, int64_t i, bool rough) {
+    if (a.ilist) {
+        if (rough) atomicOr(&a.rough_words[i >> 5], 1u << (i & 31));
+        return;
+    }
+    const unsigned b = __ballot_sync(0xffffffffu, rough);
+    if ((threadIdx.x & 31) == 0 && i >= 0) a.rough_words[i >> 5] = b;
+}
+
 // A full pass (one thread per particle; each warp reports the failed candidates of its tile) or an FP64 worklist pass over
 // the particles of the reach, 32 to a warp. The members of a listed tile are few of its 32 (7 to 9 around the extrema of
 // a smooth field, 22 around a front), and a warp instruction of the FP64 unit costs the same for any number of them. (The
@@ -1483,18 +1500,14 @@ template <typename T> __device__ __forceinline__ void list_failures(const StageA
 // loads.) The reach marks are cleared once read.
 template <typename T, int D, int M, int PDE, int RDEG, bool ALE, bool MOM = false>
 __global__ void __launch_bounds__(HCC_FLUX_BLOCK, flux_min_blocks<T, D, M>()) k_flux(const StageArgs<T> a) {
-    const int lane = int(threadIdx.x & 31);
     if (a.full) {
-        const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+        const int64_t i = full_particle(a, int64_t(blockIdx.x) * blockDim.x + threadIdx.x);
         bool rough = false;
-        const bool f = (i < a.g.n) ? flux_one<T, D, M, PDE, RDEG, ALE, false, MOM>(a, i, 0, 1, nullptr,
+        const bool f = (i >= 0) ? flux_one<T, D, M, PDE, RDEG, ALE, false, MOM>(a, i, 0, 1, nullptr,
                                                                                    a.rough_words ? &rough : nullptr)
                                    : false;
-        if (a.check) tile_failures(a, i >> 5, f);
-        if (a.rough_words) {
-            const unsigned b = __ballot_sync(0xffffffffu, rough);
-            if (lane == 0 && (i >> 5) * 32 < a.g.n) a.rough_words[i >> 5] = b;
-        }
+        if (a.check) full_failures(a, i, f);
+        if (a.rough_words) full_rough(a, i, rough);
         return;
     }
     const unsigned nm = *a.wcount;
@@ -1532,7 +1545,7 @@ __device__ __forceinline__ void ordered_round(const double *term, int lane, int 
 }
 // The particle of this lane's group in entry `g` of a full pass (every particle) or a worklist pass, or -1.
 template <typename T> __device__ __forceinline__ int64_t split_particle(const StageArgs<T> &a, unsigned g, unsigned count) {
-    return g < count ? (a.full ? int64_t(g) : int64_t(a.wlist[g])) : -1;
+    return a.full ? full_particle(a, int64_t(g)) : (g < count ? int64_t(a.wlist[g]) : -1);
 }
 
 // flux_one with the slots shared by eight lanes (no moment correction, no marks for the predictor).
@@ -1543,7 +1556,7 @@ __global__ void __launch_bounds__(128) k_flux_split(const StageArgs<double> a) {
     double *term = terms[threadIdx.x >> 5];
     const int lane = int(threadIdx.x & 31), h = lane % kSplit64;
     const int64_t np = a.g.npad;
-    const unsigned count = a.full ? unsigned(a.g.n) : *a.wcount;
+    const unsigned count = a.full ? unsigned(a.nfull) : *a.wcount;
     const unsigned step = gridDim.x * blockDim.x / kSplit64;
     const bool need_ext = a.check && (a.sc.criterion == HCC_MOOD_U1 || a.sc.criterion == HCC_MOOD_U2);
     for (unsigned g0 = (blockIdx.x * blockDim.x + threadIdx.x - lane) / kSplit64; g0 < count; g0 += step) {
@@ -1653,8 +1666,8 @@ __global__ void __launch_bounds__(128) k_gather_split(const StageArgs<double> a)
     double *term = terms[threadIdx.x >> 5];
     const int lane = int(threadIdx.x & 31), h = lane % kSplit64;
     const int64_t np = a.g.npad;
-    const int64_t i = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) / kSplit64;
-    const bool live = i < a.g.n && !a.g.bnd[i];
+    const int64_t i = full_particle(a, (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) / kSplit64);
+    const bool live = i >= 0 && !a.g.bnd[i];
     int cnt = 0;
     bool cached = false;
     double fi[M], sum[NE];
@@ -1869,10 +1882,10 @@ __global__ void __launch_bounds__(2 * HCC_TILE, tile_gather_min_blocks<D, M>()) 
     float *parts = sm + a.tv.umax * W;           // [HCC_TILE][D * M] partial gradients of the second threads
     __syncthreads();
     const int pl = int(threadIdx.x) % HCC_TILE, h = int(threadIdx.x) / HCC_TILE;
-    const int64_t i = t * HCC_TILE + pl;
+    const int64_t i = full_particle(a, t * HCC_TILE + pl);
     int mode = 0;                                 // 1: the cached fit here, 2: gather_one (first thread)
     int cnt = 0;
-    if (i < a.g.n && !a.g.bnd[i]) {
+    if (i >= 0 && !a.g.bnd[i]) {
         cnt = a.g.cnt[i];
         int q = a.orders[i];
         while (q > 1 && cnt < basis_count(D, q - 1)) --q;
@@ -1977,12 +1990,12 @@ __global__ void __launch_bounds__(HT * HCC_TILE, HT == 2 ? tile_flux_min_blocks<
     const int nu = int(a.tv.ustart[t + 1] - u0);
     int4 *spos = reinterpret_cast<int4 *>(sm);
     float *srow = sm + 4 * a.tv.umax;
-    FluxPart<float, M> *parts = reinterpret_cast<FluxPart<float, M> *>(srow + a.tv.umax * W);
+    FluxPart<float, M> *parts = reinterpret_cast<FluxPart<float, M> *>(sm);   // over the union, once it has been read
     // the particle's own global loads (count, union place, fit rows, the first union places of its slots) are issued
     // before the staging so that their latency overlaps it; none of them reads shared memory
     const int pl = int(threadIdx.x) % HCC_TILE, h = int(threadIdx.x) / HCC_TILE;
-    const int64_t i = t * HCC_TILE + pl;
-    const bool live = i < a.g.n && !a.g.bnd[i];
+    const int64_t i = full_particle(a, t * HCC_TILE + pl);
+    const bool live = i >= 0 && !a.g.bnd[i];
     const int64_t np = a.g.npad;
     // this thread's slots h, h + HT, ...: union places PF slots ahead (a rotating window), or in groups of PF with the
     // next group in flight (HCC_TILE_FLUX_GROUP > 0: the slot body unrolled over the group)
@@ -2131,21 +2144,22 @@ __global__ void __launch_bounds__(HT * HCC_TILE, HT == 2 ? tile_flux_min_blocks<
                 for (int m = 0; m < M; ++m) { mn[m] = vmin(mn[m], r[m]); mx[m] = vmax(mx[m], r[m]); }
             }
         }
-        if (h > 0) {
-            FluxPart<float, M> &part = parts[(h - 1) * HCC_TILE + pl];
+    }
+    __syncthreads();
+    if (h > 0 && live) {
+        FluxPart<float, M> &part = parts[(h - 1) * HCC_TILE + pl];
 #pragma unroll
-            for (int m = 0; m < M; ++m) {
-                part.s[m] = acc.s[m];
-                part.c[m] = acc.c[m];
-                part.mn[m] = mn[m];
-                part.mx[m] = mx[m];
-            }
+        for (int m = 0; m < M; ++m) {
+            part.s[m] = acc.s[m];
+            part.c[m] = acc.c[m];
+            part.mn[m] = mn[m];
+            part.mx[m] = mx[m];
         }
     }
     __syncthreads();
     if (h > 0) return;
     bool f = false, rough = false;
-    if (i < a.g.n) {
+    if (i >= 0) {
         if (a.g.bnd[i]) {
             float z[M];
 #pragma unroll
@@ -2178,11 +2192,8 @@ __global__ void __launch_bounds__(HT * HCC_TILE, HT == 2 ? tile_flux_min_blocks<
             f = stage_epilogue<float, D, M, PDE, 1>(a, i, fi, Kv, mn, mx);
         }
     }
-    if (a.check) tile_failures(a, i >> 5, f);
-    if (a.rough_words) {
-        const unsigned b = __ballot_sync(0xffffffffu, rough);
-        if ((threadIdx.x & 31) == 0 && (i >> 5) * 32 < a.g.n) a.rough_words[i >> 5] = b;
-    }
+    if (a.check) full_failures(a, i, f);
+    if (a.rough_words) full_rough(a, i, rough);
 }
 
 // ----------------------------------------------------------------------------------- wide linear systems (FP32)
@@ -2306,10 +2317,10 @@ __global__ void __launch_bounds__(kWideThreads, 3) k_flux_wide(const StageArgs<f
     constexpr int L = wide_lanes<M>(), W = wide_flux_row<D, M>(), RG = (D + 1) * L;   // 16-byte groups of a row
     constexpr int G = 4, P = kWideThreads / L;     // slots a group, particles at a time
     static_assert(L == 2 * D, "one of a slot's 2 D offsets and weights a lane");
-    __shared__ unsigned failed[HCC_TILE / 32], rough[HCC_TILE / 32];
+    __shared__ unsigned rough[HCC_TILE / 32];
     const int64_t t = blockIdx.x, u0 = a.tv.ustart[t], np = a.g.npad;
     const int nu = int(a.tv.ustart[t + 1] - u0);
-    if (threadIdx.x < HCC_TILE / 32) { failed[threadIdx.x] = 0u; rough[threadIdx.x] = 0u; }
+    if (threadIdx.x < HCC_TILE / 32) rough[threadIdx.x] = 0u;
     for (int e = threadIdx.x; e < nu * RG; e += kWideThreads) {
         const int64_t j = a.tv.uid[u0 + e / RG];
         const int g = e % RG;
@@ -2328,9 +2339,9 @@ __global__ void __launch_bounds__(kWideThreads, 3) k_flux_wide(const StageArgs<f
         for (int m = 0; m < 4; ++m) cm[d][m] = a.ph.c[d][off + m];
     __syncthreads();
     for (int pl = int(threadIdx.x) / L; pl < HCC_TILE; pl += P) {
-        const int64_t i = t * HCC_TILE + pl;
-        const bool bnd = i < a.g.n && a.g.bnd[i];
-        const bool live = i < a.g.n && !bnd;
+        const int64_t i = full_particle(a, t * HCC_TILE + pl);
+        const bool bnd = i >= 0 && a.g.bnd[i];
+        const bool live = i >= 0 && !bnd;
         float fi[4] = {0.0f, 0.0f, 0.0f, 0.0f}, mn[4], mx[4], Kv[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         if (bnd) store_vec<float, 4>(a.K + i * M + off, Kv);
         const int cnt = live ? a.g.cnt[i] : 0;
@@ -2424,18 +2435,12 @@ __global__ void __launch_bounds__(kWideThreads, 3) k_flux_wide(const StageArgs<f
             for (int m = 0; m < 4; ++m) r = r || (mx[m] - mn[m]) > 1e-6f * (fabsf(mx[m]) + fabsf(mn[m]));
             if (r) atomicOr(&rough[pl >> 5], 1u << (pl & 31));
         }
-        if (wide_epilogue<D, M, PDE>(a, i, off, live, fi, Kv, mn, mx) && c == 0)
-            atomicOr(&failed[pl >> 5], 1u << (pl & 31));
+        if (wide_epilogue<D, M, PDE>(a, i, off, live, fi, Kv, mn, mx) && c == 0) list_failures(a, i, true);
     }
-    if (!a.check && !a.rough_words) return;
+    if (!a.rough_words) return;
     __syncthreads();
-    const int64_t w32 = t * (HCC_TILE / 32) + threadIdx.x;
-    if (threadIdx.x >= HCC_TILE / 32 || w32 * 32 >= a.g.n) return;
-    if (a.check && failed[threadIdx.x]) {
-        a.tmask[w32] = failed[threadIdx.x];
-        a.ttiles[atomicAdd(a.tcount, 1u)] = int32_t(w32);
-    }
-    if (a.rough_words) a.rough_words[w32] = rough[threadIdx.x];
+    for (int pl = int(threadIdx.x); pl < HCC_TILE; pl += kWideThreads)      // (whole warps)
+        full_rough(a, full_particle(a, t * HCC_TILE + pl), (rough[pl >> 5] >> (pl & 31)) & 1u);
 }
 
 // The opt-in shared-memory limit of a block on the current device (the tile passes' dynamic allocation may go up
@@ -2451,8 +2456,8 @@ template <int D, int M> inline size_t tile_gather_smem(int umax) {
     return (size_t(umax) * tile_gather_row<D, M>() + size_t(HCC_TILE) * D * M) * sizeof(float);
 }
 template <int D, int M> inline size_t tile_flux_smem(int umax, int threads) {
-    return size_t(umax) * (4 + tile_flux_row<D, M>()) * sizeof(float) +
-           size_t(threads - 1) * HCC_TILE * sizeof(FluxPart<float, M>);
+    return std::max(size_t(umax) * (4 + tile_flux_row<D, M>()) * sizeof(float),
+                    size_t(threads - 1) * HCC_TILE * sizeof(FluxPart<float, M>));
 }
 // Whether a full flux pass of `ntiles` tiles takes four threads a particle: the waves of one block an SM, each half as
 // long, against those of two blocks an SM. Long passes keep two threads (their last wave is a small part).
@@ -2685,9 +2690,9 @@ template <typename T, int D>
 __global__ void __launch_bounds__(128) k_weno(const StageArgs<T> a) {
     const int lane = int(threadIdx.x & 31);
     if (a.full) {
-        const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-        const bool f = (i < a.g.n) ? weno_one<T, D>(a, i) : false;
-        if (a.check) tile_failures(a, i >> 5, f);
+        const int64_t i = full_particle(a, int64_t(blockIdx.x) * blockDim.x + threadIdx.x);
+        const bool f = (i >= 0) ? weno_one<T, D>(a, i) : false;
+        if (a.check) full_failures(a, i, f);
         return;
     }
     const unsigned nt = *a.wcount;
@@ -2908,9 +2913,9 @@ template <typename T, int D, int M, int PDE>
 __global__ void __launch_bounds__(128) k_weno_sys(const StageArgs<T> a) {
     const int lane = int(threadIdx.x & 31);
     if (a.full) {
-        const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-        const bool f = (i < a.g.n) ? weno_sys_one<T, D, M, PDE>(a, i) : false;
-        if (a.check) tile_failures(a, i >> 5, f);
+        const int64_t i = full_particle(a, int64_t(blockIdx.x) * blockDim.x + threadIdx.x);
+        const bool f = (i >= 0) ? weno_sys_one<T, D, M, PDE>(a, i) : false;
+        if (a.check) full_failures(a, i, f);
         return;
     }
     const unsigned nt = *a.wcount;
@@ -3012,9 +3017,9 @@ template <typename T, int D, int ALG>
 __global__ void __launch_bounds__(128) k_upwind(const StageArgs<T> a) {
     const int lane = int(threadIdx.x & 31);
     if (a.full) {
-        const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-        const bool f = (i < a.g.n) ? upwind_one<T, D, ALG>(a, i) : false;
-        if (a.check) tile_failures(a, i >> 5, f);
+        const int64_t i = full_particle(a, int64_t(blockIdx.x) * blockDim.x + threadIdx.x);
+        const bool f = (i >= 0) ? upwind_one<T, D, ALG>(a, i) : false;
+        if (a.check) full_failures(a, i, f);
         return;
     }
     const unsigned nt = *a.wcount;
@@ -3092,9 +3097,9 @@ template <typename T, int D, int M, int PDE>
 __global__ void __launch_bounds__(128) k_central(const StageArgs<T> a) {
     const int lane = int(threadIdx.x & 31);
     if (a.full) {
-        const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-        const bool f = (i < a.g.n) ? central_one<T, D, M, PDE>(a, i) : false;
-        if (a.check) tile_failures(a, i >> 5, f);
+        const int64_t i = full_particle(a, int64_t(blockIdx.x) * blockDim.x + threadIdx.x);
+        const bool f = (i >= 0) ? central_one<T, D, M, PDE>(a, i) : false;
+        if (a.check) full_failures(a, i, f);
         return;
     }
     const unsigned nt = *a.wcount;
@@ -3160,9 +3165,9 @@ __global__ void k_speeds(const StageArgs<T> a) {
 // the speeds recomputed in every slot); FP64 2-D, 68k, 31 us (122); FP32 2-D, 1.01M, 83 us (107).
 template <typename T, int D, int M, int PDE, int RDEG>
 __global__ void k_cfl(const StageArgs<T> a, unsigned long long *dt_bits) {
-    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    const int64_t i = full_particle(a, int64_t(blockIdx.x) * blockDim.x + threadIdx.x);
     double dti = INFINITY;
-    if (i < a.g.n && !a.g.bnd[i]) {
+    if (i >= 0 && !a.g.bnd[i]) {
         const int cnt = a.g.cnt[i];
         if (cnt > 0) {
             constexpr int LS = lam_stride<D>(), G = 4;
@@ -3203,7 +3208,7 @@ __global__ void k_cfl(const StageArgs<T> a, unsigned long long *dt_bits) {
     int cl = 0;
     bool whole_warp = true;
     if (a.cloud_id) {   // one minimum per cloud of a batch (a warp straddling two clouds: one atomic per lane)
-        cl = i < a.g.n ? a.cloud_id[i] : -1;
+        cl = i >= 0 ? a.cloud_id[i] : -1;
         whole_warp = __match_any_sync(0xffffffffu, cl) == 0xffffffffu;
         if (!whole_warp) {
             if (cl >= 0) atomicMin(dt_bits + cl, b);
@@ -3235,7 +3240,7 @@ __global__ void __launch_bounds__(2 * HCC_TILE) k_cfl_tile(const StageArgs<float
     const int64_t u0 = a.tv.ustart[t];
     const int nu = int(a.tv.ustart[t + 1] - u0);
     const int pl = int(threadIdx.x) % HCC_TILE, h = int(threadIdx.x) / HCC_TILE;
-    const int64_t i = t * HCC_TILE + pl;
+    const int64_t i = full_particle(a, t * HCC_TILE + pl);
     const int64_t np = a.g.npad;
     constexpr int PF = 4;
     const int64_t lstep = 2 * np;
@@ -3243,7 +3248,7 @@ __global__ void __launch_bounds__(2 * HCC_TILE) k_cfl_tile(const StageArgs<float
     int li = 0, mine = 0;
     int lb[PF];
     float A[D], B[D][D];
-    if (i < a.g.n && !a.g.bnd[i]) {
+    if (i >= 0 && !a.g.bnd[i]) {
         const int cnt = a.g.cnt[i];
         if (cnt > 0 && a.g.ok_d[i]) {
             li = int(a.tv.lself[i]);
@@ -3336,7 +3341,7 @@ __global__ void __launch_bounds__(2 * HCC_TILE) k_cfl_tile(const StageArgs<float
     __syncthreads();
     if (h == 1) return;
     double dti = INFINITY;
-    if (i < a.g.n && !a.g.bnd[i]) {
+    if (i >= 0 && !a.g.bnd[i]) {
         sum_c = sum_c + parts[pl];
         if (sum_c > floatmin_of<float>()) dti = double((1.0f / float(D)) / sum_c);
     }
@@ -3694,9 +3699,9 @@ __global__ void __launch_bounds__(128) k_weno_euler_f32(const StageArgs<float> a
     float *sop = wsm + int(threadIdx.x) * RS;
     const int lane = int(threadIdx.x & 31);
     if (a.full) {
-        const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-        const bool f = (i < a.g.n) ? weno_euler_f32_one<D>(a, i, sop) : false;
-        if (a.check) tile_failures(a, i >> 5, f);
+        const int64_t i = full_particle(a, int64_t(blockIdx.x) * blockDim.x + threadIdx.x);
+        const bool f = (i >= 0) ? weno_euler_f32_one<D>(a, i, sop) : false;
+        if (a.check) full_failures(a, i, f);
         return;
     }
     const unsigned nt = *a.wcount;
@@ -3718,8 +3723,8 @@ template <int D> inline size_t weno_euler_smem() {
 template <typename T, int D, int M, int PDE, int RDEG>
 struct StageInst {
     static unsigned grid(int64_t n, int bs) { return unsigned((n + bs - 1) / bs); }
-    static unsigned pass_grid(const StageArgs<T> &a, int64_t n, int bs) {
-        const unsigned g = grid(n, bs);
+    static unsigned pass_grid(const StageArgs<T> &a, int bs) {
+        const unsigned g = std::max(1u, grid(a.nfull, bs));
         return a.full ? g : std::max(1u, std::min(g, unsigned(a.list_blocks)));
     }
     // blocks of an FP32 split worklist pass (list_blocks counts blocks of four warps)
@@ -3758,16 +3763,16 @@ struct StageInst {
             }
         }
         if constexpr (sizeof(T) == 8 && M <= kSplit64) {
-            if (a.full && a.sc.limiter == HCC_LIMITER_NONE && n <= HCC_SPLIT64_GATHER) {
-                k_gather_split<D, M, PDE, RDEG><<<grid(n * kSplit64, 128), 128, 0, s>>>(a);
+            if (a.full && a.sc.limiter == HCC_LIMITER_NONE && a.nfull <= HCC_SPLIT64_GATHER) {
+                k_gather_split<D, M, PDE, RDEG><<<std::max(1u, grid(a.nfull * kSplit64, 128)), 128, 0, s>>>(a);
                 return;
             }
         }
         const int bs = a.full ? a.gather_block : 128;
         if (a.sc.limiter != HCC_LIMITER_NONE)
-            k_gather<T, D, M, PDE, RDEG, true><<<pass_grid(a, n, bs), bs, 0, s>>>(a);
+            k_gather<T, D, M, PDE, RDEG, true><<<pass_grid(a, bs), bs, 0, s>>>(a);
         else
-            k_gather<T, D, M, PDE, RDEG, false><<<pass_grid(a, n, bs), bs, 0, s>>>(a);
+            k_gather<T, D, M, PDE, RDEG, false><<<pass_grid(a, bs), bs, 0, s>>>(a);
     }
     template <bool MOM> static void flux_mom(const StageArgs<T> &a, int64_t n, cudaStream_t s) {
         if constexpr (sizeof(T) == 4) {
@@ -3780,9 +3785,9 @@ struct StageInst {
         }
         const int bs = a.full ? a.flux_block : HCC_FLUX_BLOCK;
         if (a.mover)
-            k_flux<T, D, M, PDE, RDEG, true, MOM><<<pass_grid(a, n, bs), bs, 0, s>>>(a);
+            k_flux<T, D, M, PDE, RDEG, true, MOM><<<pass_grid(a, bs), bs, 0, s>>>(a);
         else
-            k_flux<T, D, M, PDE, RDEG, false, MOM><<<pass_grid(a, n, bs), bs, 0, s>>>(a);
+            k_flux<T, D, M, PDE, RDEG, false, MOM><<<pass_grid(a, bs), bs, 0, s>>>(a);
     }
     static void flux(const void *args, int64_t n, cudaStream_t s) {
         const StageArgs<T> &a = *static_cast<const StageArgs<T> *>(args);
@@ -3826,8 +3831,8 @@ struct StageInst {
             }
         }
         if constexpr (sizeof(T) == 8 && M <= kSplit64) {
-            if (n <= (a.full ? HCC_SPLIT64_FLUX : HCC_SPLIT64_LIST) && !(a.full && a.rough_words)) {
-                const unsigned g = a.full ? grid(n * kSplit64, 128) : std::max(1u, unsigned(a.list_blocks));
+            if (a.nfull <= (a.full ? HCC_SPLIT64_FLUX : HCC_SPLIT64_LIST) && !(a.full && a.rough_words)) {
+                const unsigned g = a.full ? std::max(1u, grid(a.nfull * kSplit64, 128)) : std::max(1u, unsigned(a.list_blocks));
                 if (a.mover) k_flux_split<D, M, PDE, RDEG, true><<<g, 128, 0, s>>>(a);
                 else k_flux_split<D, M, PDE, RDEG, false><<<g, 128, 0, s>>>(a);
                 return;
@@ -3835,9 +3840,9 @@ struct StageInst {
         }
         const int bs = a.full ? a.flux_block : HCC_FLUX_BLOCK;
         if (a.mover)     // moving grid: the ALE-frame instantiation (grid velocities, shifted fluxes and speeds)
-            k_flux<T, D, M, PDE, RDEG, true><<<pass_grid(a, n, bs), bs, 0, s>>>(a);
+            k_flux<T, D, M, PDE, RDEG, true><<<pass_grid(a, bs), bs, 0, s>>>(a);
         else
-            k_flux<T, D, M, PDE, RDEG, false><<<pass_grid(a, n, bs), bs, 0, s>>>(a);
+            k_flux<T, D, M, PDE, RDEG, false><<<pass_grid(a, bs), bs, 0, s>>>(a);
     }
     static void stage1(const void *args, int64_t n, cudaStream_t s) {
         k_stage1<T, D, M, PDE, RDEG><<<grid(n, 256), 256, 0, s>>>(*static_cast<const StageArgs<T> *>(args));
@@ -3858,7 +3863,7 @@ struct StageInst {
             }
         }
         if constexpr (PDE == HCC_PDE_EULER) k_speeds<T, D, M, PDE><<<grid(n, 256), 256, 0, s>>>(a);
-        k_cfl<T, D, M, PDE, RDEG><<<grid(n, 256), 256, 0, s>>>(a, dt_bits);
+        k_cfl<T, D, M, PDE, RDEG><<<std::max(1u, grid(a.nfull, 256)), 256, 0, s>>>(a, dt_bits);
     }
     static void weno(const void *args, int64_t n, cudaStream_t s) {
         const StageArgs<T> &a = *static_cast<const StageArgs<T> *>(args);
@@ -3870,7 +3875,7 @@ struct StageInst {
                                          int(weno_euler_smem<D>()));
                     attr = true;
                 }
-                k_weno_euler_f32<D><<<pass_grid(a, n, 128), 128, weno_euler_smem<D>(), s>>>(a);
+                k_weno_euler_f32<D><<<pass_grid(a, 128), 128, weno_euler_smem<D>(), s>>>(a);
                 return;
             }
         }
@@ -3879,18 +3884,18 @@ struct StageInst {
             if (a.full && a.wflux64) k_weno_prep64<D><<<grid(n, 256), 256, 0, s>>>(a);
         }
         if constexpr (M == 1 && PDE == HCC_PDE_ADVECTION) {
-            k_weno<T, D><<<pass_grid(a, n, fbs(a)), fbs(a), 0, s>>>(a);
+            k_weno<T, D><<<pass_grid(a, fbs(a)), fbs(a), 0, s>>>(a);
         } else if constexpr (RDEG == 1) {       // systems (one instantiation: WENO has no reconstruction degree)
-            k_weno_sys<T, D, M, PDE><<<pass_grid(a, n, fbs(a)), fbs(a), 0, s>>>(a);
+            k_weno_sys<T, D, M, PDE><<<pass_grid(a, fbs(a)), fbs(a), 0, s>>>(a);
         }
     }
     static void upwind(const void *args, int64_t n, cudaStream_t s) {
         if constexpr (M == 1 && PDE == HCC_PDE_ADVECTION) {
             const StageArgs<T> &a = *static_cast<const StageArgs<T> *>(args);
             if (a.sc.upwind_alg == HCC_UPWIND_TIWARI)
-                k_upwind<T, D, HCC_UPWIND_TIWARI><<<pass_grid(a, n, fbs(a)), fbs(a), 0, s>>>(a);
+                k_upwind<T, D, HCC_UPWIND_TIWARI><<<pass_grid(a, fbs(a)), fbs(a), 0, s>>>(a);
             else if constexpr (D == 2)
-                k_upwind<T, D, HCC_UPWIND_PRAVEEN><<<pass_grid(a, n, fbs(a)), fbs(a), 0, s>>>(a);
+                k_upwind<T, D, HCC_UPWIND_PRAVEEN><<<pass_grid(a, fbs(a)), fbs(a), 0, s>>>(a);
         }
     }
     static void weno_geom(const WenoGeomArgs &g, cudaStream_t s) {
@@ -3902,7 +3907,7 @@ struct StageInst {
     }
     static void central(const void *args, int64_t n, cudaStream_t s) {
         const StageArgs<T> &a = *static_cast<const StageArgs<T> *>(args);
-        k_central<T, D, M, PDE><<<pass_grid(a, n, fbs(a)), fbs(a), 0, s>>>(a);
+        k_central<T, D, M, PDE><<<pass_grid(a, fbs(a)), fbs(a), 0, s>>>(a);
     }
     static const StageOps *ops() {
         static const StageOps o = {D, M, PDE, RDEG, RBasis<D, RDEG>::B, &gather, &flux, &stage1, &cfl,

@@ -30,9 +30,11 @@ template <typename P> void tfree(P *&p) {
 // are found with one read -- and only the distinct ones are sorted. Sorting all of them took 10.3 ms on 1.6M
 // particles with 66 neighbours, this takes 0.86 ms.
 // Shared memory: the set (hcap ints, a power of two >= 2 limit) and the list (lcap ints, a power of two >= limit).
-__global__ void __launch_bounds__(kUnionThreads) k_tile_union(int64_t n, int64_t npad, const int32_t *cnt,
-                                                              const int32_t *nidx, int limit, int hcap, int lcap,
-                                                              int32_t *tmp, int32_t *ucount) {
+// (Ghosts have no part in the passes: their neighbours do not join.)
+__global__ void __launch_bounds__(kUnionThreads) k_tile_union(int64_t nmem, const int32_t *members, int64_t npad,
+                                                              const uint8_t *bnd, const int32_t *cnt, const int32_t *nidx,
+                                                              int limit, int hcap, int lcap, int32_t *tmp,
+                                                              int32_t *ucount) {
     extern __shared__ int32_t sh[];
     int32_t *set = sh, *list = sh + hcap;
     __shared__ int count;
@@ -42,8 +44,9 @@ __global__ void __launch_bounds__(kUnionThreads) k_tile_union(int64_t n, int64_t
     __syncthreads();
     // a thread takes one particle's slots k0, k0 + step, ... (consecutive threads, consecutive particles)
     const int p = int(threadIdx.x) % HCC_TILE, k0 = int(threadIdx.x) / HCC_TILE, step = int(blockDim.x) / HCC_TILE;
-    const int64_t i = t * HCC_TILE + p;
-    const int slots = i < n ? cnt[i] + 1 : 0;      // slot 0: the particle itself
+    const int64_t q = t * HCC_TILE + p;
+    const int64_t i = q < nmem ? (members ? int64_t(members[q]) : q) : -1;
+    const int slots = i >= 0 && !bnd[i] ? cnt[i] + 1 : 0;      // slot 0: the particle itself
     const unsigned mask = unsigned(hcap - 1);
     for (int k = k0; k < slots; k += step) {
         const int32_t v = k == 0 ? int32_t(i) : nidx[int64_t(k - 1) * npad + i];
@@ -97,7 +100,8 @@ __device__ __forceinline__ double wrap_offset(double dx, int per, double L, doub
 }
 
 struct UnionArgs {
-    int64_t n, npad;
+    const int32_t *members;
+    int64_t npad;
     int D, cap;
     const int32_t *tmp;
     const int64_t *ustart;
@@ -117,7 +121,7 @@ __global__ void __launch_bounds__(256) k_tile_positions(const UnionArgs a) {
     const int64_t t = blockIdx.x;
     const int64_t u0 = a.ustart[t];
     const int nu = int(a.ustart[t + 1] - u0);
-    const int64_t iref = t * HCC_TILE;
+    const int64_t iref = a.members ? int64_t(a.members[t * HCC_TILE]) : t * HCC_TILE;
     double xr[3] = {0.0, 0.0, 0.0};
     for (int d = 0; d < a.D; ++d) xr[d] = a.pos[int64_t(d) * a.npad + iref];
     double ext[3] = {0.0, 0.0, 0.0};
@@ -174,11 +178,13 @@ __device__ __forceinline__ int find_in(const int32_t *u, int nu, int32_t v) {
 }
 
 // Step 4: the union place of every slot and of the particle itself.
-__global__ void k_tile_lidx(int64_t n, int64_t npad, const int32_t *cnt, const int32_t *nidx, const int64_t *ustart,
-                            const int32_t *uid, uint16_t *lidx, uint16_t *lself) {
-    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int64_t t = i / HCC_TILE;
+__global__ void k_tile_lidx(int64_t nmem, const int32_t *members, int64_t npad, const uint8_t *bnd, const int32_t *cnt,
+                            const int32_t *nidx, const int64_t *ustart, const int32_t *uid, uint16_t *lidx,
+                            uint16_t *lself) {
+    const int64_t q = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (q >= nmem) return;
+    const int64_t i = members ? int64_t(members[q]) : q, t = q / HCC_TILE;
+    if (bnd[i]) return;
     const int32_t *u = uid + ustart[t];
     const int nu = int(ustart[t + 1] - ustart[t]);
     lself[i] = uint16_t(find_in(u, nu, int32_t(i)));
@@ -214,19 +220,20 @@ __global__ void k_tile_coef(int64_t n, int D, const double *inv_r, const double 
 void TileTables::release() {
     tfree(ustart); tfree(uid); tfree(upos); tfree(quantum); tfree(lidx); tfree(lself); tfree(coef);
     ntiles = utotal = 0;
+    listed = 0;
     umax = 0;
     ok = 0;
 }
 
 hcc_status build_tile_tables(const TileBuild &b, TileTables &t, cudaStream_t s, std::string &err) {
     t.release();
-    if (b.n <= 0) return HCC_OK;
+    if (b.nmem <= 0) return HCC_OK;
     auto cu = [&](cudaError_t e, const char *what) -> hcc_status {
         if (e == cudaSuccess) return HCC_OK;
         err = std::string("tile tables: ") + what + ": " + cudaGetErrorString(e);
         return HCC_ERR_CUDA;
     };
-    const int64_t ntiles = (b.n + HCC_TILE - 1) / HCC_TILE;
+    const int64_t ntiles = (b.nmem + HCC_TILE - 1) / HCC_TILE;
     const int cap = int(std::min<int64_t>({int64_t(HCC_TILE) * (b.kmax + 1), int64_t(b.max_union), int64_t(65535)}));
     if (cap < 1 || b.kmax > 255) return HCC_OK;           // (stencils beyond 255 neighbours keep the slot streams)
     int hcap = 256, lcap = 128;
@@ -252,8 +259,8 @@ hcc_status build_tile_tables(const TileBuild &b, TileTables &t, cudaStream_t s, 
     if ((st = cu(cudaFuncSetAttribute(k_tile_union, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sort_smem)),
                  "sort shared memory")) != HCC_OK)
         return done(st);
-    k_tile_union<<<unsigned(ntiles), kUnionThreads, sort_smem, s>>>(b.n, b.npad, b.cnt, b.nidx, cap, hcap, lcap, tmp,
-                                                                    ucount);
+    k_tile_union<<<unsigned(ntiles), kUnionThreads, sort_smem, s>>>(b.nmem, b.members, b.npad, b.bnd, b.cnt, b.nidx, cap,
+                                                                    hcap, lcap, tmp, ucount);
     if ((st = cu(cudaGetLastError(), "union sort")) != HCC_OK) return done(st);
     std::vector<int32_t> h_count(ntiles);
     if ((st = cu(cudaMemcpyAsync(h_count.data(), ucount, size_t(ntiles) * sizeof(int32_t), cudaMemcpyDeviceToHost, s),
@@ -286,7 +293,7 @@ hcc_status build_tile_tables(const TileBuild &b, TileTables &t, cudaStream_t s, 
         (st = cu(cudaMemsetAsync(fail, 0, sizeof(int), s), "flag")) != HCC_OK)
         return done(st);
     UnionArgs ua{};
-    ua.n = b.n; ua.npad = b.npad; ua.D = b.D; ua.cap = cap; ua.tmp = tmp; ua.ustart = t.ustart; ua.pos = b.pos;
+    ua.members = b.members; ua.npad = b.npad; ua.D = b.D; ua.cap = cap; ua.tmp = tmp; ua.ustart = t.ustart; ua.pos = b.pos;
     for (int d = 0; d < 3; ++d) {
         ua.periodic[d] = b.periodic[d];
         ua.Lwrap[d] = b.Lwrap[d];
@@ -296,7 +303,8 @@ hcc_status build_tile_tables(const TileBuild &b, TileTables &t, cudaStream_t s, 
     ua.uid = t.uid; ua.upos = t.upos; ua.quantum = t.quantum; ua.fail = fail;
     k_tile_positions<<<unsigned(ntiles), 256, 0, s>>>(ua);
     const unsigned g = unsigned((b.n + 255) / 256);
-    k_tile_lidx<<<g, 256, 0, s>>>(b.n, b.npad, b.cnt, b.nidx, t.ustart, t.uid, t.lidx, t.lself);
+    k_tile_lidx<<<unsigned((b.nmem + 255) / 256), 256, 0, s>>>(b.nmem, b.members, b.npad, b.bnd, b.cnt,
+                                                                b.nidx, t.ustart, t.uid, t.lidx, t.lself);
     k_tile_coef<<<g, 256, 0, s>>>(b.n, b.D, b.inv_r, b.inv_d, b.ok_r, b.ok_d, b.invL, t.cw, t.coef);
     if ((st = cu(cudaGetLastError(), "tile tables")) != HCC_OK) return done(st);
     int h_fail = 0;

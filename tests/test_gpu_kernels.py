@@ -127,7 +127,8 @@ def test_worklists_short_and_long(hcc, oracle, cuda_lib, D, n):
 @pytest.mark.parametrize("n", [6, 11])
 def test_tile_unions(hcc, oracle, cuda_lib, n, shuffled):
     """Tile tables of a Morton-numbered cloud and of a randomly numbered one (unions of most of the cloud), partial last
-    tile: the union sizes, and the tile-staged right-hand side against the oracle's."""
+    tile: the union sizes (of the interior particles' tiles, unless these are too large for two blocks an SM), and the
+    tile-staged right-hand side against the oracle's."""
     h = 1.0 / n
     cloud = hcc.rectangular_cloud((0.0,) * 3, (1.0,) * 3, h, 2.5 * h, jitter=0.2 * h, seed=n)
     if shuffled:
@@ -138,12 +139,15 @@ def test_tile_unions(hcc, oracle, cuda_lib, n, shuffled):
     g, o = _pair(hcc, oracle, cfg, cloud, _euler(cloud).astype(np.float32).astype(np.float64))
     counts, idx, _, _ = o.neighbours()
     start = np.concatenate([[0], np.cumsum(counts)])
-    sizes = [len(np.union1d(np.arange(t, min(t + 128, cloud.n)), idx[start[t]:start[min(t + 128, cloud.n)]]))
-             for t in range(0, cloud.n, 128)]
+    inner, size = cloud.is_boundary == 0, []
+    for members in (np.flatnonzero(inner), np.arange(cloud.n)):
+        rows = [[idx[start[i]:start[i + 1]] for i in t if inner[i]] + [t[inner[t]]]
+                for t in np.split(members, range(128, len(members), 128))]
+        size.append([len(np.unique(np.concatenate(r))) for r in rows])
     got = g.tile_staging()
     if got["active"]:
-        assert got["union_entries"] == sum(sizes) and got["largest_union"] == max(sizes)
-    inner = cloud.is_boundary == 0
+        assert (got["union_entries"], got["largest_union"]) in [(sum(s), max(s)) for s in size]
+        assert got["union_entries"] == sum(size[0]) or max(size[0]) > 1100       # (two blocks an SM hold 1170 to 1205)
     assert _rel_l1(g.compute_rhs()[inner], o.compute_rhs()[inner]) < 1e-4
 
 
