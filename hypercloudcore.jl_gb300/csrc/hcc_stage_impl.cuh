@@ -1538,6 +1538,10 @@ __device__ __forceinline__ void ordered_round(const double *term, int lane, int 
         const int e = h + kSplit64 * j;
         if (e < E) {
 #pragma unroll
+// 2.7 k particles, 2-D, one variable: flux 54 -> 18 us, reconstruction 23 -> 11 us. With 66 slots a particle (3-D Euler)
+// the split also spreads the last wave, and no size is slower: a step of 22 k, 39 k, 64 k, 125 k, 216 k interior
+// particles took 6.08, 11.1, 14.5, 23.3, 37.0 ms with one thread in the full flux pass and 6.08, 9.55, 13.7, 23.1, 36.9
+// with eight lanes. With 20 slots the last round of eight is half empty, and large 2-D clouds keep one thread.
             for (int q = 0; q < kSplit64; ++q)
                 if (k0 + q < cnt) sum[j] = sum[j] + term[(g + q) * E + e];
         }
@@ -3855,7 +3859,7 @@ struct StageInst {
             }
         }
         if constexpr (sizeof(T) == 8 && M <= kSplit64) {
-            if (a.full && a.sc.limiter == HCC_LIMITER_NONE && a.nfull <= HCC_SPLIT64_GATHER) {
+            if (a.full && a.sc.limiter == HCC_LIMITER_NONE && (D == 3 || a.nfull <= HCC_SPLIT64_GATHER)) {
                 k_gather_split<D, M, PDE, RDEG><<<std::max(1u, grid(a.nfull * kSplit64, 128)), 128, 0, s>>>(a);
                 return;
             }
@@ -3923,7 +3927,7 @@ struct StageInst {
             }
         }
         if constexpr (sizeof(T) == 8 && M <= kSplit64) {
-            if (a.nfull <= (a.full ? HCC_SPLIT64_FLUX : HCC_SPLIT64_LIST) && !(a.full && a.rough_words)) {
+            if ((D == 3 || a.nfull <= (a.full ? HCC_SPLIT64_FLUX : HCC_SPLIT64_LIST)) && !(a.full && a.rough_words)) {
                 const unsigned g = a.full ? std::max(1u, grid(a.nfull * kSplit64, 128)) : std::max(1u, unsigned(a.list_blocks));
                 if (a.mover) k_flux_split<D, M, PDE, RDEG, true><<<g, 128, 0, s>>>(a);
                 else k_flux_split<D, M, PDE, RDEG, false><<<g, 128, 0, s>>>(a);
