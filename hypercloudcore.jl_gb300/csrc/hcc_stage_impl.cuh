@@ -1526,6 +1526,10 @@ __global__ void __launch_bounds__(HCC_FLUX_BLOCK, flux_min_blocks<T, D, M>()) k_
 // each, so every sum has the order of the one-thread pass and the result its bits. A warp instruction occupies the FP64
 // unit for 16 cycles and its result is some 40 cycles away, so the one-thread pass wants about four warps an SM
 // (20,000 particles on 152 SMs) before the unit is busy rather than the chain of one slot after another.
+// 2.7 k particles, 2-D, one variable: flux 54 -> 18 us, reconstruction 23 -> 11 us. With 66 slots a particle (3-D Euler)
+// the split also spreads the last wave, and no size is slower: a step of 22 k, 39 k, 64 k, 125 k, 216 k interior
+// particles took 6.08, 11.1, 14.5, 23.3, 37.0 ms with one thread in the full flux pass and 6.08, 9.55, 13.7, 23.1, 36.9
+// with eight lanes. With 20 slots the last round of eight is half empty, and large 2-D clouds keep one thread.
 constexpr int kSplit64 = 8;
 
 // Adds the round's terms (term[lane * E + e] of the slots k0 ... k0 + 7 of the warp's four particles) to this lane's
@@ -1538,10 +1542,6 @@ __device__ __forceinline__ void ordered_round(const double *term, int lane, int 
         const int e = h + kSplit64 * j;
         if (e < E) {
 #pragma unroll
-// 2.7 k particles, 2-D, one variable: flux 54 -> 18 us, reconstruction 23 -> 11 us. With 66 slots a particle (3-D Euler)
-// the split also spreads the last wave, and no size is slower: a step of 22 k, 39 k, 64 k, 125 k, 216 k interior
-// particles took 6.08, 11.1, 14.5, 23.3, 37.0 ms with one thread in the full flux pass and 6.08, 9.55, 13.7, 23.1, 36.9
-// with eight lanes. With 20 slots the last round of eight is half empty, and large 2-D clouds keep one thread.
             for (int q = 0; q < kSplit64; ++q)
                 if (k0 + q < cnt) sum[j] = sum[j] + term[(g + q) * E + e];
         }
