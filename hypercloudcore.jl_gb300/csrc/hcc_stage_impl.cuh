@@ -598,33 +598,45 @@ __device__ __forceinline__ void gather_one(const StageArgs<T> &a, const int64_t 
         for (int b = 0; b < BR; ++b)
 #pragma unroll
             for (int m = 0; m < M; ++m) bs[b][m] = T(0);
-        int32_t jn = cnt > 0 ? a.g.nidx[i] : 0;
-        T dn[D], wn = cnt > 0 ? a.g.wt[i] : T(0);
+        // slots in groups, as above: one at a time for several variables (registers)
+        constexpr int G = M == 1 ? 4 : 1;
+        int32_t j[G];
+        T dk[G][D], wk[G];
+        auto stream = [&](int k, int32_t *jk, T(*d)[D], T *w) {
 #pragma unroll
-        for (int d = 0; d < D; ++d) dn[d] = cnt > 0 ? a.g.dist[int64_t(d) * np + i] : T(0);
-        for (int k = 0; k < cnt; ++k) {
-            const int32_t j = jn;
-            T x[D], pb[BR];
+            for (int q = 0; q < G; ++q) {
+                const bool on = k + q < cnt;
+                const int64_t s1 = int64_t(k + q) * np + i;
+                jk[q] = on ? a.g.nidx[s1] : int32_t(i);
+                w[q] = on ? a.g.wt[s1] : T(0);
 #pragma unroll
-            for (int d = 0; d < D; ++d) x[d] = dn[d] * invL;
-            const T w = wn;
-            if (k + 1 < cnt) {
-                const int64_t s1 = int64_t(k + 1) * np + i;
-                jn = a.g.nidx[s1];
-                wn = a.g.wt[s1];
-#pragma unroll
-                for (int d = 0; d < D; ++d) dn[d] = a.g.dist[(int64_t(k + 1) * D + d) * np + i];
+                for (int e = 0; e < D; ++e) d[q][e] = on ? a.g.dist[(int64_t(k + q) * D + e) * np + i] : T(0);
             }
-            recon_basis<D, RDEG, T>(x, pb);
-            T df[M];
-            load_vec<T, M>(a.U + int64_t(j) * M, df);
-            if (lim) extend_extrema<T, M>(df, umin, umax);
+        };
+        stream(0, j, dk, wk);
+        for (int k = 0; k < cnt; k += G) {
+            T df[G][M], x[G][D], w[G];
 #pragma unroll
-            for (int m = 0; m < M; ++m) df[m] = df[m] - fi[m];
+            for (int q = 0; q < G; ++q) {
+                load_vec<T, M>(a.U + int64_t(j[q]) * M, df[q]);
+                w[q] = wk[q];
 #pragma unroll
-            for (int b = 0; b < BR; ++b)
+                for (int d = 0; d < D; ++d) x[q][d] = dk[q][d] * invL;
+            }
+            stream(k + G, j, dk, wk);
 #pragma unroll
-                for (int m = 0; m < M; ++m) bs[b][m] = bs[b][m] + w * (pb[b] * df[m]);
+            for (int q = 0; q < G; ++q) {
+                if (k + q >= cnt) break;
+                T pb[BR];
+                recon_basis<D, RDEG, T>(x[q], pb);
+                if (lim) extend_extrema<T, M>(df[q], umin, umax);
+#pragma unroll
+                for (int m = 0; m < M; ++m) df[q][m] = df[q][m] - fi[m];
+#pragma unroll
+                for (int b = 0; b < BR; ++b)
+#pragma unroll
+                    for (int m = 0; m < M; ++m) bs[b][m] = bs[b][m] + w[q] * (pb[b] * df[q][m]);
+            }
         }
         const T *inv = a.g.inv_r + i * (BR * BR);
         T invm[BR][BR];
