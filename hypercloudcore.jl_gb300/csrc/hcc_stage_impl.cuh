@@ -2221,8 +2221,6 @@ __global__ void __launch_bounds__(HT * HCC_TILE, HT == 2 ? tile_flux_min_blocks<
 // precede. Here a lane holds a quarter of that, the rows come from shared memory, and the slot streams (place in the
 // union, offsets, divergence weights: the FP32 streams of the stream-fed pass) do not depend on one another; the four
 // lanes load one of a slot's four stream words each and exchange them, four slots ahead of the sums.
-// (The reconstruction pass of these systems keeps k_gather: with a quarter of the arithmetic a slot, lanes sharing a
-// particle took 258 us against its 227.)
 template <int M> constexpr int wide_lanes() { return M / 4; }
 template <typename T, int M, int PDE> constexpr bool wide_system() {
     return sizeof(T) == 4 && PDE != HCC_PDE_EULER && M >= 8 && M % 4 == 0 && 32 % (M / 4) == 0;
@@ -2321,6 +2319,86 @@ __device__ __forceinline__ bool wide_epilogue(const StageArgs<float> &a, int64_t
     if (!live) return false;
     if (a.sc.criterion == HCC_MOOD_ONLY || !adm) return true;
     return (a.sc.criterion == HCC_MOOD_U1 || a.sc.criterion == HCC_MOOD_U2) && flag;
+}
+
+// Reconstruction of a wide linear system (no limiter): L lanes a particle, four components each, as in the flux pass. A
+// lane loads the index and weights of one of L slots and the lanes exchange them; the states of the next L slots (whole
+// rows: a thread a particle took a quarter of a sector from each of 32 lines a load) and the stream words of the ones
+// after are in flight while L slots are summed. 218 us against 241 on 1.0 M
+// particles of 16 components.
+template <int D, int M, int PDE> __device__ __noinline__ void gather_apart(const StageArgs<float> &a, int64_t i) {
+    gather_one<float, D, M, PDE, 1, false>(a, i);  // (its registers are not the loop's)
+}
+template <int D, int M, int PDE>
+__global__ void __launch_bounds__(kWideThreads, 4) k_gather_wide(const StageArgs<float> a) {
+    constexpr int L = wide_lanes<M>();
+    const int c = int(threadIdx.x) % L, off = 4 * c;
+    const int64_t i = full_particle(a, (int64_t(blockIdx.x) * kWideThreads + threadIdx.x) / L);
+    const bool live = i >= 0 && !a.g.bnd[i];
+    const int64_t np = a.g.npad;
+    bool cached = false;
+    int cnt = 0;
+    if (live) {
+        cnt = a.g.cnt[i];
+        int p = a.orders[i];
+        while (p > 1 && cnt < basis_count(D, p - 1)) --p;
+        cached = p == a.sc.max_order && p > 1 && a.g.ok_r[i];
+        if (!cached && c == 0) gather_apart<D, M, PDE>(a, i);
+    }
+    if (!cached) cnt = 0;
+    float fi[4] = {}, out[D][4] = {};
+    if (cached) load_vec<float, 4>(a.U + i * M + off, fi);
+    int32_t jn = 0;
+    float gn[D];
+    auto stream = [&](int k) {                     // slot k + c
+        const bool on = k + c < cnt;
+        jn = on ? a.g.nidx[int64_t(k + c) * np + i] : 0;
+#pragma unroll
+        for (int d = 0; d < D; ++d) gn[d] = on ? a.g.gw[(int64_t(k + c) * D + d) * np + i] : 0.0f;
+    };
+    float f[L][4], g[D];
+    auto rows = [&](int k) {                       // the states of slots k ... of the words loaded last
+#pragma unroll
+        for (int d = 0; d < D; ++d) g[d] = gn[d];
+#pragma unroll
+        for (int s = 0; s < L; ++s) {
+            const int32_t j = __shfl_sync(0xffffffffu, jn, s, L);
+            if (k + s < cnt) load_vec<float, 4>(a.U + int64_t(j) * M + off, f[s]);
+        }
+    };
+    const int kw = __reduce_max_sync(0xffffffffu, cnt);
+    stream(0);
+    rows(0);
+    stream(L);
+    for (int k = 0; k < kw; k += L) {
+        float df[L][4], w[D];
+#pragma unroll
+        for (int d = 0; d < D; ++d) w[d] = g[d];
+#pragma unroll
+        for (int s = 0; s < L; ++s)
+#pragma unroll
+            for (int m = 0; m < 4; ++m) df[s][m] = f[s][m];
+        rows(k + L);
+        stream(k + 2 * L);
+#pragma unroll
+        for (int s = 0; s < L; ++s) {
+            float ws[D];
+#pragma unroll
+            for (int d = 0; d < D; ++d) ws[d] = __shfl_sync(0xffffffffu, w[d], s, L);
+            if (k + s < cnt) {
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                    const float dm = df[s][m] - fi[m];
+#pragma unroll
+                    for (int d = 0; d < D; ++d) out[d][m] = out[d][m] + ws[d] * dm;
+                }
+            }
+        }
+    }
+    if (!cached) return;
+    float *row = a.grad + i * grad_row<float, D * M>() + off;
+#pragma unroll
+    for (int d = 0; d < D; ++d) store_vec<float, 4>(row + d * M, out[d]);
 }
 
 // flux_one for a linear system on a fixed grid, degree-1 reconstruction. With A = f_ij - f_i and B = f_ji - f_i the flux
@@ -3859,6 +3937,13 @@ struct StageInst {
                         k_gather_tile<D, M, PDE, true><<<unsigned(a.tv.ntiles), 2 * HCC_TILE, smem, s>>>(a);
                     else
                         k_gather_tile<D, M, PDE, false><<<unsigned(a.tv.ntiles), 2 * HCC_TILE, smem, s>>>(a);
+                    return;
+                }
+            }
+            if constexpr (wide_system<T, M, PDE>()) {
+                if (a.full && a.sc.limiter == HCC_LIMITER_NONE && a.g.gw) {
+                    k_gather_wide<D, M, PDE><<<std::max(1u, grid(a.nfull * wide_lanes<M>(), kWideThreads)), kWideThreads, 0,
+                                               s>>>(a);
                     return;
                 }
             }
