@@ -234,7 +234,16 @@ struct hcc_ctx {
     int half_sm = 0;                             // shared memory of a block that leaves room for a second one on its SM
     hcc_tuning tune{128, 128, 8, 2};             // launch shapes of the step (hcc_set_tuning / hcc_autotune)
     TileTables tiles;                            // tile staging of the FP32 full passes (hcc_tiles.cu)
-    int tile_enabled = 1;
+    int tile_enabled = 2;                        // 0 / 1: chosen by the caller; 2: where it measured faster
+    // 3-D stencils (K ~ 66): flux 7.05 against 10.4 ms at 8.0M points. Wide linear systems: flux 640 against 1007 us. 2-D
+    // stencils (K ~ 20), of which the flux pass and the CFL step alone are tile-staged: 893 against 970 us a step at 1.0M
+    // (Euler), 315 against 359 at 160k, 141 against 149 at 78k (advection), 303 against 342 at 360k but 620 against 611
+    // at 1.0M; below 32 tiles most of the chip has no tile, and the gain is within the launches' noise.
+    bool tiles_on() const {
+        if (!tiles.ok || moving() || tile_enabled == 0) return false;
+        if (tile_enabled == 1 || D == 3 || (cfg.pde != HCC_PDE_EULER && M >= 8)) return true;
+        return D == 2 && n_interior >= 32 * HCC_TILE && (cfg.pde == HCC_PDE_EULER || n_interior <= 500000);
+    }
     void apply_tuning() {
         list_blocks = std::max(1, sms) * tune.list_blocks_per_sm;
         drop_blocks = std::max(1, sms) * tune.drop_blocks_per_sm;
@@ -506,8 +515,7 @@ template <typename T> StageArgs<T> base_args(hcc_ctx *c) {
     a.tcount = &c->lcounts->t;
     a.inadm = c->inadm;
     a.list_blocks = c->list_blocks;
-    a.sms = c->sms;
-    const bool tiled = sizeof(T) == 4 && c->tiles.ok && c->tile_enabled && !c->moving();
+    const bool tiled = sizeof(T) == 4 && c->tiles_on();
     const bool listed = tiled ? c->tiles.listed : c->skip_ghosts();
     a.ilist = listed ? c->ilist : nullptr;
     a.nfull = listed ? c->n_interior : c->n;
@@ -1154,9 +1162,6 @@ hcc_status hcc_create(const hcc_config *cfg, int64_t capacity, hcc_ctx **out) {
     const hcc_config &f = c->cfg;
     if (f.abi_version != HCC_ABI_VERSION) return c->fail(HCC_ERR_INVALID, "abi_version mismatch");
     c->D = f.dim;
-    // tile staging by default where it measured faster: the 3-D stencils (K ~ 66; flux 7.05 vs 10.4 ms at 8.0M
-    // points); 2-D stencils (K ~ 19) ran faster stream-fed (flux 0.21 vs 0.30 ms at 1.0M)
-    c->tile_enabled = (f.dim == 3 || (f.pde != HCC_PDE_EULER && f.n_vars >= 8)) ? 1 : 0;
     c->M = f.n_vars;
     c->f32 = f.precision == HCC_FP32;
     c->capacity = capacity;
@@ -1696,7 +1701,7 @@ hcc_status hcc_set_tile_staging(hcc_ctx *c, int32_t enable) {
 
 hcc_status hcc_get_tile_staging(hcc_ctx *c, int32_t *active, int64_t *union_entries, int32_t *largest_union) {
     if (!c) return HCC_ERR_INVALID;
-    if (active) *active = (c->tiles.ok && c->tile_enabled && !c->moving()) ? 1 : 0;
+    if (active) *active = c->tiles_on() ? 1 : 0;
     if (union_entries) *union_entries = c->tiles.utotal;
     if (largest_union) *largest_union = c->tiles.umax;
     return HCC_OK;

@@ -348,7 +348,6 @@ template <typename T> struct StageArgs {
     unsigned *rlcount;
     const int32_t *wlist;             // FP64 flux worklist pass over the reach: its particles
     int list_blocks;                  // grid of a worklist pass (warp-stride over the tiles)
-    int sms;                          // SMs of the device
     int flux_block, gather_block;     // block sizes of the full flux / gather passes (multiples of 32, <= 128)
     // epilogue: next candidate (Y_{s+1} or the final state) and the MOOD check of checkpoint s+1
     int form_next;

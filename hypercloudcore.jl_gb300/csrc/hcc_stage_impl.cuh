@@ -1988,19 +1988,21 @@ __global__ void __launch_bounds__(2 * HCC_TILE, tile_gather_min_blocks<D, M>()) 
     }
 }
 
-// Flux pass, HT threads per particle of the tile (slots k = h, h + HT, ... for h < HT); the others write their
-// compensated partial sums and extrema to shared memory, the first combines them and runs the epilogue. Two threads and
-// two blocks an SM, or (few tiles) four threads and one block, which takes half as long over a tile: the better one is
-// the one whose last wave leaves less of the chip idle (flux_tile_wide).
-template <int D, int M> constexpr int tile_flux_min_blocks() { return M >= 8 ? 1 : 2; }
+// Flux pass, two threads per particle of the tile in 3-D (slots k = h, h + 2, ... for h = 0, 1); the second writes its
+// compensated partial sums and extrema to shared memory, the first combines them and runs the epilogue. (Four threads and
+// one block an SM where that saves a wave: never faster on 11 k to 290 k interior particles, at most 12 % slower.) In 2-D
+// one thread: with 20 slots the combination and the idle half of the epilogue cost more than the second thread gives
+// (970 us a step stream-fed, 893 with one thread, 1256 with two, 2-D Euler at 1.0M).
+template <int D> constexpr int tile_flux_threads() { return D == 3 ? 2 : 1; }
+template <int D> constexpr int tile_flux_min_blocks() { return D == 3 ? 2 : 5; }
 
 // PLAIN: EPD1 interface orders and the plain Rusanov flux (the usual configuration), known at compile time.
-template <int D, int M, int PDE, bool PLAIN, int HT>
-__global__ void __launch_bounds__(HT * HCC_TILE, HT == 2 ? tile_flux_min_blocks<D, M>() : 1) k_flux_tile(const StageArgs<float> a) {
+template <int D, int M, int PDE, bool PLAIN>
+__global__ void __launch_bounds__(tile_flux_threads<D>() * HCC_TILE, tile_flux_min_blocks<D>()) k_flux_tile(const StageArgs<float> a) {
     extern __shared__ __align__(16) float sm[];
     constexpr int W = tile_flux_row<D, M>();
     constexpr int RW = M + D * M;                 // used words of a row: the state, then the gradient
-    constexpr int GS = grad_row<float, D * M>();
+    constexpr int GS = grad_row<float, D * M>(), HT = tile_flux_threads<D>();
     const int64_t t = blockIdx.x;
     const int64_t u0 = a.tv.ustart[t];
     const int nu = int(a.tv.ustart[t + 1] - u0);
@@ -2015,8 +2017,7 @@ __global__ void __launch_bounds__(HT * HCC_TILE, HT == 2 ? tile_flux_min_blocks<
     const int64_t np = a.g.npad;
     // this thread's slots h, h + HT, ...: union places PF slots ahead (a rotating window), or in groups of PF with the
     // next group in flight (HCC_TILE_FLUX_GROUP > 0: the slot body unrolled over the group)
-    // (wide states, M >= 8, keep the window: the unrolled group spills their registers)
-    constexpr int GROUP = M >= 8 ? 0 : HCC_TILE_FLUX_GROUP;
+    constexpr int GROUP = HCC_TILE_FLUX_GROUP;
     constexpr int PF = GROUP > 0 ? GROUP : HCC_TILE_FLUX_PF;
     const int64_t lstep = HT * np;
     const uint16_t *lp = a.tv.lidx + int64_t(h) * np + i;
@@ -2161,19 +2162,20 @@ __global__ void __launch_bounds__(HT * HCC_TILE, HT == 2 ? tile_flux_min_blocks<
             }
         }
     }
-    __syncthreads();
-    if (h > 0 && live) {
-        FluxPart<float, M> &part = parts[(h - 1) * HCC_TILE + pl];
+    if constexpr (HT == 2) {
+        __syncthreads();
+        if (h == 1 && live) {
 #pragma unroll
-        for (int m = 0; m < M; ++m) {
-            part.s[m] = acc.s[m];
-            part.c[m] = acc.c[m];
-            part.mn[m] = mn[m];
-            part.mx[m] = mx[m];
+            for (int m = 0; m < M; ++m) {
+                parts[pl].s[m] = acc.s[m];
+                parts[pl].c[m] = acc.c[m];
+                parts[pl].mn[m] = mn[m];
+                parts[pl].mx[m] = mx[m];
+            }
         }
+        __syncthreads();
+        if (h == 1) return;
     }
-    __syncthreads();
-    if (h > 0) return;
     bool f = false, rough = false;
     if (i >= 0) {
         if (a.g.bnd[i]) {
@@ -2182,22 +2184,20 @@ __global__ void __launch_bounds__(HT * HCC_TILE, HT == 2 ? tile_flux_min_blocks<
             for (int m = 0; m < M; ++m) z[m] = 0.0f;
             store_vec<float, M>(a.K + i * M, z);
         } else {
-            // the compensated partials: their sum, minus their compensations and the rounding errors of that sum
+            // the two compensated partials: their sum, minus both compensations and the rounding error of that sum
             float Kv[M];
 #pragma unroll
             for (int m = 0; m < M; ++m) {
-                float sum = acc.s[m], comp = acc.c[m];
-#pragma unroll
-                for (int v = 0; v < HT - 1; ++v) {
-                    const FluxPart<float, M> &part = parts[v * HCC_TILE + pl];
-                    const float u = sum + part.s[m];
-                    const float cm = (u - sum) - part.s[m];
-                    comp = (comp + part.c[m]) + cm;
-                    sum = u;
-                    mn[m] = vmin(mn[m], part.mn[m]);
-                    mx[m] = vmax(mx[m], part.mx[m]);
+                if constexpr (HT == 1) {
+                    Kv[m] = -(acc.s[m] - acc.c[m]);
+                } else {
+                    const float s1 = parts[pl].s[m];
+                    const float u = acc.s[m] + s1;
+                    const float cm = (u - acc.s[m]) - s1;
+                    Kv[m] = -(u - ((acc.c[m] + parts[pl].c[m]) + cm));
+                    mn[m] = vmin(mn[m], parts[pl].mn[m]);
+                    mx[m] = vmax(mx[m], parts[pl].mx[m]);
                 }
-                Kv[m] = -(sum - comp);
             }
             if (a.rough_words) {
                 bool r = !need_ext;
@@ -2549,17 +2549,9 @@ inline int tile_smem_optin() {
 template <int D, int M> inline size_t tile_gather_smem(int umax) {
     return (size_t(umax) * tile_gather_row<D, M>() + size_t(HCC_TILE) * D * M) * sizeof(float);
 }
-template <int D, int M> inline size_t tile_flux_smem(int umax, int threads) {
+template <int D, int M> inline size_t tile_flux_smem(int umax) {
     return std::max(size_t(umax) * (4 + tile_flux_row<D, M>()) * sizeof(float),
-                    size_t(threads - 1) * HCC_TILE * sizeof(FluxPart<float, M>));
-}
-// Whether a full flux pass of `ntiles` tiles takes four threads a particle: the waves of one block an SM, each half as
-// long, against those of two blocks an SM. Long passes keep two threads (their last wave is a small part).
-template <int D, int M> inline bool flux_tile_wide(const StageArgs<float> &a) {
-    if (M >= 8 || D < 3 || a.tv.ntiles > int64_t(16) * a.sms) return false;
-    if (tile_flux_smem<D, M>(a.tv.umax, 4) > size_t(tile_smem_optin())) return false;
-    const int64_t w4 = (a.tv.ntiles + a.sms - 1) / a.sms, w2 = (a.tv.ntiles + 2 * a.sms - 1) / (2 * a.sms);
-    return w4 < 2 * w2;
+                    size_t(tile_flux_threads<D>() - 1) * HCC_TILE * sizeof(FluxPart<float, M>));
 }
 
 // ----------------------------------------------------------------------------------- WENO (scalar)
@@ -3922,8 +3914,10 @@ struct StageInst {
     static void gather(const void *args, int64_t n, cudaStream_t s) {
         const StageArgs<T> &a = *static_cast<const StageArgs<T> *>(args);
         if constexpr (sizeof(T) == 4 && RDEG == 1) {
-            if (a.full && a.tile) {   // FP32 full pass with tile tables: neighbours staged in shared memory (not wide systems)
-                if constexpr (!wide_system<T, M, PDE>()) {
+            if constexpr (D == 3 && !wide_system<T, M, PDE>()) {
+                // FP32 full pass with tile tables: neighbours staged in shared memory (in 2-D the slot streams are
+                // the faster form: 893 against 1027 us a step, 2-D Euler at 1.0M)
+                if (a.full && a.tile) {
                     static bool attr = false;
                     if (!attr) {
                         cudaFuncSetAttribute(k_gather_tile<D, M, PDE, true>,
@@ -3998,20 +3992,14 @@ struct StageInst {
                         const size_t smem = size_t(a.tv.umax) * wide_flux_row<D, M>() * sizeof(float);
                         k_flux_wide<D, M, PDE><<<unsigned(a.tv.ntiles), kWideThreads, smem, s>>>(a);
                     } else {
-                        auto go = [&](auto kernel, int threads) {
+                        auto go = [&](auto kernel) {
                             cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tile_smem_optin());
-                            kernel<<<unsigned(a.tv.ntiles), threads * HCC_TILE, tile_flux_smem<D, M>(a.tv.umax, threads),
+                            kernel<<<unsigned(a.tv.ntiles), tile_flux_threads<D>() * HCC_TILE, tile_flux_smem<D, M>(a.tv.umax),
                                      s>>>(a);
                         };
                         const bool plain = a.sc.strategy == HCC_EPD1 && !a.sc.aligned;
-                        if constexpr (D == 3 && M < 8) {
-                            if (plain && flux_tile_wide<D, M>(a)) {
-                                go(k_flux_tile<D, M, PDE, true, 4>, 4);
-                                return;
-                            }
-                        }
-                        if (plain) go(k_flux_tile<D, M, PDE, true, 2>, 2);
-                        else go(k_flux_tile<D, M, PDE, false, 2>, 2);
+                        if (plain) go(k_flux_tile<D, M, PDE, true>);
+                        else go(k_flux_tile<D, M, PDE, false>);
                     }
                     return;
                 }
@@ -4042,8 +4030,10 @@ struct StageInst {
     }
     static void cfl(const void *args, int64_t n, unsigned long long *dt_bits, cudaStream_t s) {
         const StageArgs<T> &a = *static_cast<const StageArgs<T> *>(args);
-        if constexpr (sizeof(T) == 4 && RDEG == 1) {
-            if (a.tile && !a.cloud_id) {   // FP32 with tile tables: the union's speeds staged in shared memory
+        if constexpr (sizeof(T) == 4 && RDEG == 1 && D == 3) {
+            // FP32 with tile tables: the union's speeds staged in shared memory (in 2-D the streams and the table of
+            // speeds are faster: 78 against 88 us at 1.0M)
+            if (a.tile && !a.cloud_id) {
                 const size_t smem = (size_t(a.tv.umax) * 8 + HCC_TILE) * sizeof(float);
                 static bool attr = false;
                 if (!attr) {
