@@ -236,13 +236,14 @@ struct hcc_ctx {
     TileTables tiles;                            // tile staging of the FP32 full passes (hcc_tiles.cu)
     int tile_enabled = 2;                        // 0 / 1: chosen by the caller; 2: where it measured faster
     // 3-D stencils (K ~ 66): flux 7.05 against 10.4 ms at 8.0M points. Wide linear systems: flux 640 against 1007 us. 2-D
-    // stencils (K ~ 20), of which the flux pass and the CFL step alone are tile-staged: 893 against 970 us a step at 1.0M
-    // (Euler), 315 against 359 at 160k, 141 against 149 at 78k (advection), 303 against 342 at 360k but 620 against 611
-    // at 1.0M; below 32 tiles most of the chip has no tile, and the gain is within the launches' noise.
+    // stencils of Euler (K ~ 20), of which the flux pass alone is tile-staged: 893 against 970 us a step at 1.0M, 315
+    // against 359 at 160k; below 32 tiles most of the chip has no tile, and the gain is within the launches' noise.
+    // (2-D advection: 156 against 179 us at 160k, 620 against 611 at 1.0M, with up to 10 % more rounding error from the
+    // recomputed weights, of which its right-hand side has little else: stream-fed.)
     bool tiles_on() const {
         if (!tiles.ok || moving() || tile_enabled == 0) return false;
         if (tile_enabled == 1 || D == 3 || (cfg.pde != HCC_PDE_EULER && M >= 8)) return true;
-        return D == 2 && n_interior >= 32 * HCC_TILE && (cfg.pde == HCC_PDE_EULER || n_interior <= 500000);
+        return D == 2 && cfg.pde == HCC_PDE_EULER && n_interior >= 32 * HCC_TILE;
     }
     void apply_tuning() {
         list_blocks = std::max(1, sms) * tune.list_blocks_per_sm;

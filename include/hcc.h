@@ -482,9 +482,8 @@ const char *hcc_build_info(void);
    and divergence / gradient weights from quantised positions and per-particle FP32 fit rows instead of reading the
    per-slot streams. Results agree with the stream-fed passes to FP32 rounding (both round the same FP64 geometry).
    Enabled by default where it measured faster than the stream-fed passes: 3-D contexts (about 66 neighbours a
-   particle), linear systems of eight variables and more, and 2-D contexts from 4,096 interior particles on (Euler;
-   scalar advection up to 500,000), of which the flux pass alone is tile-staged. Off by default in 1-D; enable = 1 / 0
-   chooses either way. */
+   particle), linear systems of eight variables and more, and 2-D Euler contexts from 4,096 interior particles on, of
+   which the flux pass alone is tile-staged. Off by default elsewhere; enable = 1 / 0 chooses either way. */
 hcc_status hcc_set_tile_staging(hcc_ctx *ctx, int32_t enable);
 /* Whether the full passes of the next step are tile-staged, the union entries over all tiles and the largest union
    (any output may be NULL). */
