@@ -211,6 +211,13 @@ template <> __device__ __forceinline__ bool positive<double>(double x) {
     return (unsigned long long)(__double_as_longlong(x) - 1) < 0x7ff0000000000000ull;
 }
 // x or -x by the sign bit
+// |a| >= |b| and neither a NaN; FP64 as integers (magnitudes order like their words, a NaN's above infinity's).
+template <typename T> __device__ __forceinline__ bool covers(T a, T b) { return fabs(a) >= fabs(b); }
+template <> __device__ __forceinline__ bool covers<double>(double a, double b) {
+    const unsigned long long m = 0x7fffffffffffffffull, inf = 0x7ff0000000000000ull;
+    const unsigned long long wa = __double_as_longlong(a) & m, wb = __double_as_longlong(b) & m;
+    return wa >= wb && wa <= inf;
+}
 __device__ __forceinline__ double negate_if(double x, bool neg) {
     return __longlong_as_double(__double_as_longlong(x) ^ (neg ? (long long)0x8000000000000000ull : 0ll));
 }
@@ -460,6 +467,40 @@ __device__ __forceinline__ T limiter_phi(int lim, T r) {
     return (rp * rp + T(2) * rp) / (rp * rp + rp + T(2));
 }
 
+// Positive numbers from 2^-900 (FP32: 2^-90) up, no NaN nor infinity; x < y of such (FP64 as integers).
+__device__ __forceinline__ bool in_range(double x) {
+    const unsigned hi = unsigned(__double2hiint(x));
+    return hi >= ((1023u - 900u) << 20) && hi < 0x7ff00000u;
+}
+__device__ __forceinline__ bool in_range(float x) { return x >= 8.0779357e-28f && x <= 3.0e38f; }
+__device__ __forceinline__ bool below(double x, double y) { return __double_as_longlong(x) < __double_as_longlong(y); }
+__device__ __forceinline__ bool below(float x, float y) { return x < y; }
+
+// Venkatakrishnan's coefficient over the slots: phi grows with r = room / recon up to r = 4.8, so the least r gives the
+// least phi, and the quotients are compared by their cross products (two multiplications where the quotient and phi take
+// three divisions, which a warp executes as soon as one of its lanes has such a slot). Ratios too close for the rounded
+// phi to follow their order (1e-13, FP32 1e-5; its rounding is some 1e-15 and its slope at least a quarter), and products
+// out of range, are evaluated one by one, so the minimum keeps its bits.
+template <typename T> struct LeastRatio {
+    T room, recon;                                // of the least ratio so far; recon 0: none
+    __device__ __forceinline__ LeastRatio() : room(T(0)), recon(T(0)) {}
+    __device__ __forceinline__ void add(int lim, T rm, T rc, T &phi) {       // magnitudes; rc > 0
+        constexpr T near = T(1) - (sizeof(T) == 8 ? T(1e-13) : T(1e-5));
+        if (rm == T(0)) { phi = T(0); return; }   // (phi(0) = 0, no other is less)
+        if (recon == T(0)) { room = rm; recon = rc; return; }
+        const T a = rm * recon, b = room * rc;
+        if (in_range(a) && in_range(b)) {
+            if (below(a, b * near)) { room = rm; recon = rc; return; }
+            if (below(b, a * near)) return;
+        }
+        if (rm == room && rc == recon) return;
+        phi = vmin(phi, limiter_phi<T>(lim, rm / rc));
+    }
+    __device__ __forceinline__ void finish(int lim, T &phi) const {
+        if (recon != T(0)) phi = vmin(phi, limiter_phi<T>(lim, room / recon));
+    }
+};
+
 template <typename T> __device__ __forceinline__ T eps16();
 template <> __device__ __forceinline__ double eps16<double>() { return 16.0 * 2.220446049250313e-16; }
 template <> __device__ __forceinline__ float eps16<float>() { return 16.0f * 1.1920929e-7f; }
@@ -487,24 +528,40 @@ __device__ __forceinline__ void limit_slopes(const StageArgs<T> &a, int64_t i, i
     const T tol16 = eps16<T>();
     const bool bj = a.sc.limiter == HCC_LIMITER_BJ_SOFT || a.sc.limiter == HCC_LIMITER_BJ_HARD;
     const T reach = bj ? T(1) : T(2.01);
+    // out.p(dk / 2) with the halves and quarters in the coefficients (powers of two: the same bits), the distances to the
+    // bounds formed once and the reach compared as integers: 17 -> 13 FP64 instructions a slot and variable
+    LeastRatio<T> least[M];
+    T half[BR][M], up[M], down[M];
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+        up[m] = umax[m] - fi[m];
+        down[m] = umin[m] - fi[m];
+#pragma unroll
+        for (int b = 0; b < BR; ++b) half[b][m] = out[b][m] * (b < D ? T(0.5) : T(0.25));
+    }
 #pragma unroll 2
     for (int k = 0; k < cnt; ++k) {
-        T hx[D], p[BR];
+        T x[D], p[BR];
 #pragma unroll
-        for (int d = 0; d < D; ++d) hx[d] = T(0.5) * a.g.dist[(int64_t(k) * D + d) * np + i];
-        recon_basis<D, RDEG, T>(hx, p);
+        for (int d = 0; d < D; ++d) x[d] = a.g.dist[(int64_t(k) * D + d) * np + i];
+        recon_basis<D, RDEG, T>(x, p);
 #pragma unroll
         for (int m = 0; m < M; ++m) {
-            T recon = out[0][m] * p[0];
+            T recon = half[0][m] * p[0];
 #pragma unroll
-            for (int b = 1; b < BR; ++b) recon = recon + out[b][m] * p[b];
-            const T bound = positive(recon) ? umax[m] : umin[m];
-            const T room = bound - fi[m];
-            if (fabs(room) >= fabs(reach * recon)) continue;      // (a NaN goes on)
+            for (int b = 1; b < BR; ++b) recon = recon + half[b][m] * p[b];
+            const bool pos = positive(recon);
+            const T room = pos ? up[m] : down[m], bound = pos ? umax[m] : umin[m];
+            if (covers(room, reach * recon)) continue;            // (a NaN goes on)
             const T tol = tol16 * vmax(fabs(fi[m]), fabs(bound));
-            if (fabs(recon) > tol) phi[m] = vmin(phi[m], limiter_phi<T>(a.sc.limiter, room / recon));
+            if (!(fabs(recon) > tol)) continue;
+            // (room and recon have the same sign: the ratio is that of their magnitudes)
+            if (bj) phi[m] = vmin(phi[m], limiter_phi<T>(a.sc.limiter, room / recon));
+            else least[m].add(a.sc.limiter, fabs(room), fabs(recon), phi[m]);
         }
     }
+#pragma unroll
+    for (int m = 0; m < M; ++m) least[m].finish(a.sc.limiter, phi[m]);
     const bool hard = a.sc.limiter == HCC_LIMITER_BJ_HARD || a.sc.limiter == HCC_LIMITER_VK_HARD;
 #pragma unroll
     for (int b = 0; b < BR; ++b)
