@@ -2324,9 +2324,14 @@ __device__ __forceinline__ bool wide_epilogue(const StageArgs<float> &a, int64_t
     if (a.implicit_mode) {
         float KIo[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         if constexpr (PDE == HCC_PDE_BGK) {
-            float u = (Y[0] + Y[1]) + (Y[2] + Y[3]);
+            // the sum over all components in their order, handed from lane to lane (as maxwellian adds them)
+            float u = ((Y[0] + Y[1]) + Y[2]) + Y[3];
 #pragma unroll
-            for (int o = 1; o < L; o <<= 1) u = u + __shfl_xor_sync(0xffffffffu, u, o);
+            for (int s = 1; s < L; ++s) {
+                const float before = __shfl_sync(0xffffffffu, u, s - 1, L);
+                if (4 * s == off) u = (((before + Y[0]) + Y[1]) + Y[2]) + Y[3];
+            }
+            u = __shfl_sync(0xffffffffu, u, L - 1, L);
             const float dto = cf->dt_ii * a.ph.inv_eps, denom = 1.0f / (1.0f + dto), inv_dt_ii = cf->inv_dt_ii;
 #pragma unroll
             for (int m = 0; m < 4; ++m) {
@@ -2464,10 +2469,10 @@ __global__ void __launch_bounds__(kWideThreads, 4) k_gather_wide(const StageArgs
     for (int d = 0; d < D; ++d) store_vec<float, 4>(row + d * M, out[d]);
 }
 
-// flux_one for a linear system on a fixed grid, degree-1 reconstruction. With A = f_ij - f_i and B = f_ji - f_i the flux
-// difference of a slot contracted with its divergence weights is
-//   cw (f_ij + f_ji - 2 f_i) - S (f_ji - f_ij) = (cw + S) A + (cw - S) B,   cw = sum_d w_d c_dm,
-// S = sum_d w_d s_d max lambda_d common to the components: formed from differences of the states, no flux cancels.
+// flux_one for a linear system on a fixed grid, degree-1 reconstruction. (The term of a slot from differences of the
+// states, (cw + S) (f_ij - f_i) + (cw - S) (f_ji - f_i) with cw = sum_d w_d c_dm and S = sum_d w_d s_d max lambda_d, takes
+// fewer instructions, 700 against 865 us, and rounds less; but MOOD then decides otherwise for a few candidates at a
+// bound, which moves a state more than the rounding does.)
 template <int D, int M, int PDE>
 __global__ void __launch_bounds__(kWideThreads, 3) k_flux_wide(const StageArgs<float> a) {
     extern __shared__ __align__(16) float sm[];
@@ -2529,7 +2534,7 @@ __global__ void __launch_bounds__(kWideThreads, 3) k_flux_wide(const StageArgs<f
         for (int k0 = 0; k0 < kw; k0 += G) {
             sp += int64_t(G) * (D * np);
             lp += int64_t(G) * np;
-            float vn[G], part[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            float vn[G];
             int ln[G];
 #pragma unroll
             for (int q = 0; q < G; ++q) {
@@ -2561,26 +2566,28 @@ __global__ void __launch_bounds__(kWideThreads, 3) k_flux_wide(const StageArgs<f
                 const int lo = oi_own < oj_own ? oi_own : oj_own;
                 const float si = (epd1 ? lo : oi_own) >= 2 ? 0.5f : 0.0f, sj = (epd1 ? lo : oj_own) >= 2 ? -0.5f : 0.0f;
                 const bool below = a.sc.aligned && (a.sc.max_order == 1 || lo < a.sc.max_order);
-                float S = 0.0f, pi[D], pj[D];
+                // the slot's term in flux_slot's form and order: the results keep the stream-fed pass's bits
+                float sw[D], pi[D], pj[D], t[4];
 #pragma unroll
                 for (int d = 0; d < D; ++d) {
-                    const float sw = (below ? wk[d] : dk[d]) > 0.0f ? a.ph.amax[d] : -a.ph.amax[d];
-                    S = (d == 0) ? wk[0] * sw : S + wk[d] * sw;
+                    sw[d] = (below ? wk[d] : dk[d]) > 0.0f ? a.ph.amax[d] : -a.ph.amax[d];
                     pi[d] = si * dk[d];
                     pj[d] = sj * dk[d];
                 }
 #pragma unroll
                 for (int m = 0; m < 4; ++m) {
-                    float A = gi[0][m] * pi[0], B = fj[m] - fi[m], cw = wk[0] * cm[0][m];
+                    float ri = gi[0][m] * pi[0], rj = gj[0][m] * pj[0];
 #pragma unroll
-                    for (int d = 0; d < D; ++d) {
-                        if (d > 0) { A = A + gi[d][m] * pi[d]; cw = cw + wk[d] * cm[d][m]; }
-                        B = B + gj[d][m] * pj[d];
-                    }
-                    part[m] = part[m] + ((cw + S) * A + (cw - S) * B);
+                    for (int d = 1; d < D; ++d) { ri = ri + gi[d][m] * pi[d]; rj = rj + gj[d][m] * pj[d]; }
+                    const float fij = fi[m] + ri, fji = fj[m] + rj;
+                    const float sum = (fij + fji) - 2.0f * fi[m], jump = fji - fij;
+                    float tm = wk[0] * (cm[0][m] * sum - sw[0] * jump);
+#pragma unroll
+                    for (int d = 1; d < D; ++d) tm = tm + wk[d] * (cm[d][m] * sum - sw[d] * jump);
+                    t[m] = tm;
                 }
+                acc.add(t);
             }
-            acc.add(part);
 #pragma unroll
             for (int q = 0; q < G; ++q) { v[q] = vn[q]; l[q] = ln[q]; }
         }
