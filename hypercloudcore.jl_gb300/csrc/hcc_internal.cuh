@@ -27,7 +27,8 @@
                                    // slower than scalar instructions in the tile-staged 3-D flux pass)
 #endif
 #ifndef HCC_SPLIT_WIDE_TILES
-#define HCC_SPLIT_WIDE_TILES 304   // FP32 worklist passes: lists of up to this many tiles take a whole block a tile
+#define HCC_SPLIT_WIDE_TILES 304   // FP32 worklist passes: lists of up to this many tiles take a whole block a tile (a
+                                   // 3-D step of 30 k to 1.0 M particles: as fast or up to 6 % slower with 1,216 or 4,864)
 #endif
 #ifndef HCC_SPLIT64_FLUX
 #define HCC_SPLIT64_FLUX 24000     // FP64 full flux passes of 1-D and 2-D clouds up to this size: eight lanes a particle

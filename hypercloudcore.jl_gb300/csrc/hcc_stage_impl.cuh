@@ -1921,12 +1921,10 @@ template <int RW> constexpr int tile_stage_unroll() {
     return RW <= 12 ? HCC_TILE_STAGE_UNROLL : (HCC_TILE_STAGE_UNROLL + 1) / 2;
 }
 
-template <int D, int M> constexpr int tile_gather_min_blocks() { return M >= 8 ? 1 : 3; }
-
 // LIM: slope limiters, which go through gather_one. Without one, a particle off the cached fit (an order below the full
 // one, a failed fit) has zero slopes, and the kernel does without gather_one's registers.
 template <int D, int M, int PDE, bool LIM>
-__global__ void __launch_bounds__(2 * HCC_TILE, tile_gather_min_blocks<D, M>()) k_gather_tile(const StageArgs<float> a) {
+__global__ void __launch_bounds__(2 * HCC_TILE, 3) k_gather_tile(const StageArgs<float> a) {
     extern __shared__ __align__(16) float sm[];
     constexpr int W = tile_gather_row<D, M>(), GS = grad_row<float, D * M>();
     const int64_t t = blockIdx.x;
