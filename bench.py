@@ -450,7 +450,7 @@ def roofline_of(workload, D, M, K, n_int, kt, peak, peak_kind, tiled=False):
     traffic = rec.get(f"flux_f32_{workload}_bytes_per_point_stage")
     g_traffic = rec.get(f"gather_f32_{workload}_bytes_per_point_stage")
     g_model = gather_b * n_int / (gather_ms / 1e3) / 1e9
-    gname = f"k_gather_tile<{D},{M},EULER>" if tiled else f"k_gather<float,{D},{M},EULER,1>"
+    gname = f"k_gather_tile<{D},{M},EULER>" if tiled and D == 3 else f"k_gather<float,{D},{M},EULER,1>"
     fname = f"k_flux_tile<{D},{M},EULER>" if tiled else f"k_flux<float,{D},{M},EULER,1>"
     gather_roof = {"kernel": gname, "bound": "hbm", "unit": "GB/s", "peak": peak,
                    "achieved": g_model, "frac": g_model / peak,
