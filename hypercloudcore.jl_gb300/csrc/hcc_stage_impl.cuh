@@ -932,7 +932,7 @@ __global__ void __launch_bounds__(32 * split_warps<M>()) k_gather_tiles(const St
 // share the slots, and a longer one a warp: all passes of an FP64 3-D step 707 -> 307 us (65.6 k interior particles, a
 // third of them listed), of a moving 2-D one 123 -> 46 us.
 template <typename T, int D, int M, int PDE, int RDEG, bool LIM>
-__global__ void __launch_bounds__(128) k_gather(const StageArgs<T> a) {
+__global__ void __launch_bounds__(128, sizeof(T) == 4 && M == 1 ? 9 : 1) k_gather(const StageArgs<T> a) {
     if (a.full) {
         const int64_t i = full_particle(a, int64_t(blockIdx.x) * blockDim.x + threadIdx.x);
         if (i >= 0) gather_one<T, D, M, PDE, RDEG, LIM>(a, i);
@@ -1144,7 +1144,10 @@ __device__ __forceinline__ int interface_terms(int o) {
 // (FP32 2-D scalar/Euler: 72 registers; wider states and FP64 need more).
 template <typename T, int D, int M> constexpr int flux_min_blocks() {
     if (sizeof(T) == 8) return M >= 8 ? 1 : (D * M >= 12 ? 2 : HCC_FLUX_MINB64);
-    return M >= 8 ? HCC_FLUX_MINB_MANY : (D * M >= 12 ? HCC_FLUX_MINB_WIDE : HCC_FLUX_MINB);
+    // one variable: a slot is few instructions and three dependent gathers, so the pass waits, and 36 warps an SM wait
+    // better than 28 (56 registers, some 50 bytes spilled; order 3 with limiter, 1.0 M: 3857 us for four steps with nine
+    // blocks an SM, 3926 with eight, 4222 with seven, 4441 with ten; the same for the reconstruction)
+    return M >= 8 ? HCC_FLUX_MINB_MANY : (D * M >= 12 ? HCC_FLUX_MINB_WIDE : M == 1 ? 9 : HCC_FLUX_MINB);
 }
 
 // The MUSCL functor (MUSCL.jl:390-508) in its streamed form: per slot, EPD interface reconstruction, physical
