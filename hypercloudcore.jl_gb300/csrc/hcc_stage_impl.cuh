@@ -2284,7 +2284,8 @@ __global__ void __launch_bounds__(tile_flux_threads<D>() * HCC_TILE, tile_flux_m
 // and extrema (219 registers, two blocks an SM) and waited for the twelve loads of a slot that its index load had to
 // precede. Here a lane holds a quarter of that, the rows come from shared memory, and the slot streams (place in the
 // union, offsets, divergence weights: the FP32 streams of the stream-fed pass) do not depend on one another; the four
-// lanes load one of a slot's four stream words each and exchange them, four slots ahead of the sums.
+// lanes load one of a slot's four stream words each and exchange them, two slots ahead of the sums (four: 72 bytes
+// spilled at three blocks an SM, 7883 us for two steps of 1.0 M particles against 6505; without spills at two: 6806).
 template <int M> constexpr int wide_lanes() { return M / 4; }
 template <typename T, int M, int PDE> constexpr bool wide_system() {
     return sizeof(T) == 4 && PDE != HCC_PDE_EULER && M >= 8 && M % 4 == 0 && 32 % (M / 4) == 0;
@@ -2472,13 +2473,13 @@ __global__ void __launch_bounds__(kWideThreads, 4) k_gather_wide(const StageArgs
 
 // flux_one for a linear system on a fixed grid, degree-1 reconstruction. (The term of a slot from differences of the
 // states, (cw + S) (f_ij - f_i) + (cw - S) (f_ji - f_i) with cw = sum_d w_d c_dm and S = sum_d w_d s_d max lambda_d, takes
-// fewer instructions, 700 against 865 us, and rounds less; but MOOD then decides otherwise for a few candidates at a
+// fewer instructions (700 against 865 us, both with four slots ahead) and rounds less; but MOOD then decides otherwise for a few candidates at a
 // bound, which moves a state more than the rounding does.)
 template <int D, int M, int PDE>
 __global__ void __launch_bounds__(kWideThreads, 3) k_flux_wide(const StageArgs<float> a) {
     extern __shared__ __align__(16) float sm[];
     constexpr int L = wide_lanes<M>(), W = wide_flux_row<D, M>(), RG = (D + 1) * L;   // 16-byte groups of a row
-    constexpr int G = 4, P = kWideThreads / L;     // slots a group, particles at a time
+    constexpr int G = 2, P = kWideThreads / L;     // slots a group, particles at a time
     static_assert(L == 2 * D, "one of a slot's 2 D offsets and weights a lane");
     __shared__ unsigned rough[HCC_TILE / 32];
     const int64_t t = blockIdx.x, u0 = a.tv.ustart[t], np = a.g.npad;
