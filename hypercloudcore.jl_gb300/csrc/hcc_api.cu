@@ -235,7 +235,7 @@ struct hcc_ctx {
     hcc_tuning tune{128, 128, 8, 2};             // launch shapes of the step (hcc_set_tuning / hcc_autotune)
     TileTables tiles;                            // tile staging of the FP32 full passes (hcc_tiles.cu)
     int tile_enabled = 2;                        // 0 / 1: chosen by the caller; 2: where it measured faster
-    // 3-D stencils (K ~ 66): flux 7.05 against 10.4 ms at 8.0M points. Wide linear systems: flux 865 against 1007 us. 2-D
+    // 3-D stencils (K ~ 66): flux 7.05 against 10.4 ms at 8.0M points. Wide linear systems: flux 650 against 1007 us. 2-D
     // stencils of Euler (K ~ 20), of which the flux pass alone is tile-staged: 893 against 970 us a step at 1.0M, 315
     // against 359 at 160k; below 32 tiles most of the chip has no tile, and the gain is within the launches' noise.
     // (2-D advection: 156 against 179 us at 160k, 620 against 611 at 1.0M, with up to 10 % more rounding error from the
