@@ -1090,8 +1090,7 @@ template <typename T> hcc_status run_cfl(hcc_ctx *c, double *dt_out) {
     hcc_status st = c->cuda(cudaMemcpyAsync(c->d_counters + 2, &inf_bits, sizeof(inf_bits), cudaMemcpyHostToDevice,
                                             c->stream), "dt init");
     if (st != HCC_OK) return st;
-    c->ops->cfl(&a, c->n, c->d_counters + 2, c->stream);
-    c->launches = (c->cfg.pde == HCC_PDE_EULER && !a.tile) ? 2 : 1;     // with the speed table
+    c->launches = c->ops->cfl(&a, c->n, c->d_counters + 2, c->stream);
     c->launches_total += c->launches;
     if ((st = launch_check(c, "cfl kernel")) != HCC_OK) return st;
     st = c->cuda(cudaMemcpyAsync(c->h_counters + 2, c->d_counters + 2, sizeof(unsigned long long),
@@ -1951,15 +1950,14 @@ hcc_status hcc_batch_time_steps(hcc_ctx *c, double *dt_out) {
         a.U = static_cast<const float *>(c->rhos);
         a.lam = static_cast<float *>(c->xfer);
         a.cloud_id = c->cloud_id;
-        c->ops->cfl(&a, c->n, c->cloud_dt, c->stream);
+        c->launches = c->ops->cfl(&a, c->n, c->cloud_dt, c->stream);
     } else {
         StageArgs<double> a = base_args<double>(c);
         a.U = static_cast<const double *>(c->rhos);
         a.lam = static_cast<double *>(c->xfer);
         a.cloud_id = c->cloud_id;
-        c->ops->cfl(&a, c->n, c->cloud_dt, c->stream);
+        c->launches = c->ops->cfl(&a, c->n, c->cloud_dt, c->stream);
     }
-    c->launches = c->cfg.pde == HCC_PDE_EULER ? 2 : 1;                  // with the speed table
     c->launches_total += c->launches;
     HCC_TRY(launch_check(c, "cfl kernel"));
     HCC_TRY(c->cuda(cudaMemcpyAsync(bits.data(), c->cloud_dt, size_t(nb) * sizeof(unsigned long long),

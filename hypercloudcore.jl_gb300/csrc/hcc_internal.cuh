@@ -484,7 +484,7 @@ struct StageOps {
     void (*gather)(const void *args, int64_t n, cudaStream_t s);
     void (*flux)(const void *args, int64_t n, cudaStream_t s);
     void (*stage1)(const void *args, int64_t n, cudaStream_t s);   // Y_1 (predictor + implicit part)
-    void (*cfl)(const void *args, int64_t n, unsigned long long *dt_bits, cudaStream_t s);
+    int (*cfl)(const void *args, int64_t n, unsigned long long *dt_bits, cudaStream_t s);   // returns the kernels launched
     void (*weno)(const void *args, int64_t n, cudaStream_t s);   // WENO flux pass (scalar advection only)
     void (*central)(const void *args, int64_t n, cudaStream_t s);   // CentralDivergence pass
     void (*upwind)(const void *args, int64_t n, cudaStream_t s);    // UpwindDivergence :Tiwari / :Praveen pass

@@ -4100,7 +4100,7 @@ struct StageInst {
     static void stage1(const void *args, int64_t n, cudaStream_t s) {
         k_stage1<T, D, M, PDE, RDEG><<<grid(n, 256), 256, 0, s>>>(*static_cast<const StageArgs<T> *>(args));
     }
-    static void cfl(const void *args, int64_t n, unsigned long long *dt_bits, cudaStream_t s) {
+    static int cfl(const void *args, int64_t n, unsigned long long *dt_bits, cudaStream_t s) {
         const StageArgs<T> &a = *static_cast<const StageArgs<T> *>(args);
         if constexpr (sizeof(T) == 4 && RDEG == 1 && D == 3) {
             // FP32 with tile tables: the union's speeds staged in shared memory (in 2-D the streams and the table of
@@ -4114,11 +4114,12 @@ struct StageInst {
                     attr = true;
                 }
                 k_cfl_tile<D, M, PDE><<<unsigned(a.tv.ntiles), 2 * HCC_TILE, smem, s>>>(a, dt_bits);
-                return;
+                return 1;
             }
         }
         if constexpr (PDE == HCC_PDE_EULER) k_speeds<T, D, M, PDE><<<grid(n, 256), 256, 0, s>>>(a);
         k_cfl<T, D, M, PDE, RDEG><<<std::max(1u, grid(a.nfull, 256)), 256, 0, s>>>(a, dt_bits);
+        return PDE == HCC_PDE_EULER ? 2 : 1;
     }
     static void weno(const void *args, int64_t n, cudaStream_t s) {
         const StageArgs<T> &a = *static_cast<const StageArgs<T> *>(args);
