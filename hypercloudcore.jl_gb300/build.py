@@ -60,7 +60,7 @@ def build(verbose: bool = False, jobs: int | None = None, extra_flags=None, lib_
     BUILD = Path(build_dir) if build_dir else PKG / "_build"
     LIB = Path(lib_path) if lib_path else PKG / "libhcc_gb300.so"
     BUILD.mkdir(parents=True, exist_ok=True)
-    headers = list(CSRC.glob("*.cuh")) + [PKG.parent / "include" / "hcc.h"]
+    headers = [*CSRC.glob("*.cuh"), *CSRC.glob("*.h"), PKG.parent / "include" / "hcc.h"]
     extra = list(extra_flags or [])
     cmds = []
     objs = []

@@ -1,12 +1,12 @@
 // hcc_api.cu — the C ABI (include/hcc.h): context lifecycle, device buffers and the host orchestration of one
 // time step (the GeneralRKTimeStepper functor, src/TimeStepping/TimeSteppers.jl:531-577) on one CUDA stream.
 #include "hcc_internal.cuh"
+#include "hcc_buffers.h"
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
 #include <limits>
 #include <new>
-#include <unordered_map>
 
 using namespace hcc;
 
@@ -361,35 +361,28 @@ struct hcc_ctx {
     }
     hcc_status sync(const char *what) { return cuda(cudaStreamSynchronize(stream), what); }
 
-    // The buffers of a cloud, its lists and its geometry are kept when the cloud, the lists or the geometry are replaced,
-    // and reused where they are large enough (and not more than four times too large): a moving grid rebuilds its
-    // geometry at every stage and its lists after every step, and a context may be given cloud after cloud. Allocating
-    // and releasing them each time took 2.2 of the 8.8 ms of three moving 2-D FP64 steps on 15k particles.
-    // `spare` elements are added when memory has to be allocated. Only the context's own members are kept this way;
-    // they are freed with the context.
-    std::unordered_map<const void *, size_t> kept;
-    template <typename P> hcc_status reserve(P *&p, size_t count, const char *what, size_t spare = 0) {
-        void *v = p;
-        const hcc_status st = reserve_bytes(v, std::max<size_t>(count, 1) * sizeof(P), what, spare * sizeof(P));
-        p = static_cast<P *>(v);
-        return st;
+    // The buffers of a cloud (0), its lists (1) and its geometry (2) are kept when these are replaced (hcc_buffers.h);
+    // they are freed with the context. rebuild(group) precedes the reservations of a group. `spare`: elements added when
+    // memory has to be allocated.
+    struct DeviceMemory {
+        int allocate(void **p, size_t bytes) {
+            const cudaError_t e = cudaMalloc(p, bytes);
+            if (e != cudaSuccess) cudaGetLastError();      // reported by reserve; not left for the next launch check
+            return int(e);
+        }
+        void release(void *p) { cudaFree(p); }
+    };
+    KeptBuffers<DeviceMemory> kept;
+    int kept_group = 0;
+    void rebuild(int group) {
+        kept_group = group;
+        kept.begin(group);
     }
-    hcc_status reserve_bytes(void *&p, size_t bytes, const char *what, size_t spare = 0) {
-        if (p) {
-            const auto it = kept.find(p);
-            if (it != kept.end() && it->second >= bytes && it->second / 4 <= bytes) return HCC_OK;
-            if (it != kept.end()) kept.erase(it);
-            cudaFree(p);
-            p = nullptr;
-        }
-        const hcc_status st = cuda(cudaMalloc(&p, std::max<size_t>(bytes + spare, 1)), what);
-        if (st == HCC_OK) {
-            kept[p] = std::max<size_t>(bytes + spare, 1);
-        } else {
-            p = nullptr;
-            cudaGetLastError();      // reported here; not left for the next launch check
-        }
-        return st;
+    template <typename P> hcc_status reserve(P *&p, size_t count, const char *what, size_t spare = 0) {
+        return cuda(cudaError_t(kept.reserve(&p, count * sizeof(P), spare * sizeof(P), kept_group)), what);
+    }
+    hcc_status reserve_bytes(void *&p, size_t bytes, const char *what) {
+        return cuda(cudaError_t(kept.reserve(&p, bytes, 0, kept_group)), what);
     }
 
     // A new cloud: what describes the old one is dropped (the buffers of upload_cloud are kept).
@@ -1300,6 +1293,8 @@ hcc_status hcc_upload_cloud(hcc_ctx *c, int64_t n, const double *pos, const uint
     c->reset_slots();
     c->have_cloud = c->have_nb = c->have_geom = c->have_state = false;
     c->batch_offsets.clear();
+    c->rebuild(0);
+    if (c->n != n) c->kept.release_stale();       // a cloud of another size: nothing of the old one stays allocated
     c->n = n;
     c->npad = ((n + 31) / 32) * 32;
     const int D = c->D, M = c->M;
@@ -1392,6 +1387,7 @@ static hcc_status enqueue_neighbours(hcc_ctx *c) {
     if (!c) return HCC_ERR_INVALID;
     if (!c->have_cloud) return c->fail(HCC_ERR_STATE, "no cloud uploaded");
     c->have_nb = c->have_geom = false;       // until every buffer below is there and filled
+    c->rebuild(1);
     const hcc_config &f = c->cfg;
     const int D = c->D;
     hcc_status st;
@@ -1706,6 +1702,7 @@ static hcc_status enqueue_geometry(hcc_ctx *c) {
     if (!c) return HCC_ERR_INVALID;
     if (!c->have_nb) return c->fail(HCC_ERR_STATE, "neighbour lists missing");
     c->have_geom = false;
+    c->rebuild(2);
     hcc_status st;
     const int D = c->D;
     const size_t slots = size_t(std::max(c->kmax, 1)) * c->npad, spare = c->spare_slots();

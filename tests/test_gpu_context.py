@@ -42,3 +42,69 @@ def test_launches_of_a_cfl_step(hcc, cuda_lib, kind, D, tiles, launches):
     ctx.time_step()
     after = ctx.counters()
     assert after["kernel_launches"] == launches and after["kernel_launches_total"] - before == launches
+
+
+def _used():
+    import torch
+    torch.cuda.synchronize()
+    free, total = torch.cuda.mem_get_info()
+    return total - free
+
+
+def _boxes(hcc, D, sizes, seed=0):
+    """Boxes of different numbers of cells a side, one spacing (so one configuration serves all, the largest one's)."""
+    h = 1.0 / max(sizes)
+    return [hcc.rectangular_cloud((0.0,) * D, (n * h,) * (D - 1) + (n * h + h,), h, 2.5 * h, jitter=0.2 * h, seed=seed + k)
+            for k, n in enumerate(sizes)]
+
+
+def test_a_smaller_cloud_gives_memory_back(hcc, cuda_lib):
+    """A context that held a cloud three times as large holds what a new context takes for the second one (to a quarter,
+    and to the 2 MB that the driver rounds each of some 60 buffers to)."""
+    small, big = _boxes(hcc, 3, (44, 66))
+    cfg = hcc.make_config(hcc.Euler(3), big, scheme=hcc.MUSCL(2, 2), bc_map=OUTFLOW)
+    one = hcc.Context(cfg)
+    start = _used()
+    _prepare(one, small)
+    need = _used() - start
+    ctx = hcc.Context(cfg)
+    start = _used()
+    _prepare(ctx, big)
+    held = _used() - start
+    _prepare(ctx, small)
+    assert held > 2.5 * need and _used() - start < 1.25 * need + (128 << 20)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("kind,D,sizes", [("euler", 3, (11, 7, 13, 13)), ("euler", 2, (70, 20, 75, 75)), ("weno", 3, (9, 7, 10, 10)),
+                                          ("order3", 2, (24, 13, 40, 40)), ("moving", 2, (24, 13, 40, 40))])
+def test_clouds_one_after_another(hcc, cuda_lib, kind, D, sizes, precision):
+    """Clouds given to one context, a smaller one, a larger one and another of the same size: steps, orders and flags are
+    those of a new context, bit for bit."""
+    clouds = _boxes(hcc, D, sizes)
+    pde = hcc.LinearAdvection(((1.0,), (0.5,))) if kind == "order3" else hcc.Euler(D)
+    scheme = hcc.WENO(2) if kind == "weno" else hcc.MUSCL(3, 0, "vk_hard") if kind == "order3" else hcc.MUSCL(2, 2)
+    cfg = hcc.make_config(pde, clouds[2], scheme=scheme, mood=hcc.MOOD(hcc.EPD1, hcc.MOODu1(1e-8)), bc_map=OUTFLOW,
+                          precision=precision)
+
+    def results(ctx, cloud):
+        U = (np.cos(3 * cloud.pos).sum(axis=1) + 3.0)[:, None] if kind == "order3" else _euler(cloud)
+        if kind != "moving":
+            U = U * np.where(cloud.pos[:, :1] > 0.4, 1.0, 0.4)           # a jump: worklists
+        _prepare(ctx, cloud)
+        ctx.upload_state(U)
+        dt = 0.1 * ctx.time_step()
+        for _ in range(2):
+            ctx.step(0.0, dt)
+        return [np.float64(dt), ctx.download_state(), ctx.orders(), ctx.mood_flags(), ctx.positions()]
+
+    def context():
+        ctx = hcc.Context(cfg)
+        if kind == "moving":
+            ctx.set_mover(hcc.mover("lagrangian"))
+        return ctx
+
+    kept = context()
+    for cloud in clouds:
+        for a, b in zip(results(kept, cloud), results(context(), cloud)):
+            assert np.ascontiguousarray(a).tobytes() == np.ascontiguousarray(b).tobytes()
