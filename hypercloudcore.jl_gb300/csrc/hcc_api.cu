@@ -1637,7 +1637,7 @@ hcc_status hcc_download_neighbours_of(hcc_ctx *c, int64_t n_sel, const int64_t *
 // fit, no moment correction, EPD0/EPD1/StrictEPD0 interface orders): every full gather and flux pass then reads
 // its neighbours from shared memory and recomputes the slot offsets and weights. Contexts or clouds that do not
 // qualify keep the stream-fed passes (tiles.ok = 0).
-hcc_status build_tiles(hcc_ctx *c) {
+static hcc_status build_unions(hcc_ctx *c) {
     c->tiles.release();
     const int pde = c->cfg.pde;
     const bool eligible = c->f32 && c->rdeg == 1 && c->max_order <= 2 && c->ddeg == 1 && !c->no_recon() &&
@@ -1679,6 +1679,12 @@ hcc_status build_tiles(hcc_ctx *c) {
     b.nmem = c->n;
     b.max_union = most;
     return build_tile_tables(b, c->tiles, c->stream, c->err);
+}
+
+hcc_status build_tiles(hcc_ctx *c) {
+    hcc_status st = build_unions(c);
+    if (st == HCC_OK && c->tiles.ok) st = c->cuda(c->ops->tile_setup(), "shared memory of the tile passes");
+    return st;
 }
 
 hcc_status hcc_set_tile_staging(hcc_ctx *c, int32_t enable) {

@@ -489,6 +489,7 @@ struct StageOps {
     void (*central)(const void *args, int64_t n, cudaStream_t s);   // CentralDivergence pass
     void (*upwind)(const void *args, int64_t n, cudaStream_t s);    // UpwindDivergence :Tiwari / :Praveen pass
     void (*weno_geom)(const WenoGeomArgs &g, cudaStream_t s);      // FP32 Euler WENO operators (or nullptr)
+    cudaError_t (*tile_setup)();      // the tile passes' shared memory, on the current device (once per set of tables)
 };
 
 const StageOps *stage_ops_f64_r1(int D, int M, int pde);

@@ -3990,14 +3990,6 @@ struct StageInst {
                 // FP32 full pass with tile tables: neighbours staged in shared memory (in 2-D the slot streams are
                 // the faster form: 893 against 1027 us a step, 2-D Euler at 1.0M)
                 if (a.full && a.tile) {
-                    static bool attr = false;
-                    if (!attr) {
-                        cudaFuncSetAttribute(k_gather_tile<D, M, PDE, true>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, tile_smem_optin());
-                        cudaFuncSetAttribute(k_gather_tile<D, M, PDE, false>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, tile_smem_optin());
-                        attr = true;
-                    }
                     const size_t smem = tile_gather_smem<D, M>(a.tv.umax);
                     if (a.sc.limiter != HCC_LIMITER_NONE)
                         k_gather_tile<D, M, PDE, true><<<unsigned(a.tv.ntiles), 2 * HCC_TILE, smem, s>>>(a);
@@ -4059,13 +4051,10 @@ struct StageInst {
             if constexpr (RDEG == 1) {
                 if (a.full && a.tile) {   // full pass with tile tables: neighbours staged in shared memory
                     if constexpr (wide_system<T, M, PDE>()) {
-                        cudaFuncSetAttribute(k_flux_wide<D, M, PDE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             tile_smem_optin() - 1024);
                         const size_t smem = size_t(a.tv.umax) * wide_flux_row<D, M>() * sizeof(float);
                         k_flux_wide<D, M, PDE><<<unsigned(a.tv.ntiles), kWideThreads, smem, s>>>(a);
                     } else {
                         auto go = [&](auto kernel) {
-                            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tile_smem_optin());
                             kernel<<<unsigned(a.tv.ntiles), tile_flux_threads<D>() * HCC_TILE, tile_flux_smem<D, M>(a.tv.umax),
                                      s>>>(a);
                         };
@@ -4107,12 +4096,6 @@ struct StageInst {
             // speeds are faster: 78 against 88 us at 1.0M)
             if (a.tile && !a.cloud_id) {
                 const size_t smem = (size_t(a.tv.umax) * 8 + HCC_TILE) * sizeof(float);
-                static bool attr = false;
-                if (!attr) {
-                    cudaFuncSetAttribute(k_cfl_tile<D, M, PDE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         tile_smem_optin());
-                    attr = true;
-                }
                 k_cfl_tile<D, M, PDE><<<unsigned(a.tv.ntiles), 2 * HCC_TILE, smem, s>>>(a, dt_bits);
                 return 1;
             }
@@ -4161,12 +4144,35 @@ struct StageInst {
         const StageArgs<T> &a = *static_cast<const StageArgs<T> *>(args);
         k_central<T, D, M, PDE><<<pass_grid(a, fbs(a)), fbs(a), 0, s>>>(a);
     }
+    // The opt-in shared memory of the tile passes. The attribute belongs to a kernel on a device: it is set when the tables
+    // of a context are built, on the device that will run them.
+    static cudaError_t tile_setup() {
+        cudaError_t err = cudaSuccess;
+        if constexpr (sizeof(T) == 4 && RDEG == 1) {
+            const int most = tile_smem_optin();
+            auto allow = [&](auto kernel, int bytes) {
+                if (err == cudaSuccess) err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+            };
+            if constexpr (wide_system<T, M, PDE>()) {
+                allow(k_flux_wide<D, M, PDE>, most - 1024);        // (it has a static part)
+            } else {
+                allow(k_flux_tile<D, M, PDE, true>, most);
+                allow(k_flux_tile<D, M, PDE, false>, most);
+            }
+            if constexpr (D == 3 && !wide_system<T, M, PDE>()) {
+                allow(k_gather_tile<D, M, PDE, true>, most);
+                allow(k_gather_tile<D, M, PDE, false>, most);
+            }
+            if constexpr (D == 3) allow(k_cfl_tile<D, M, PDE>, most);
+        }
+        return err;
+    }
     static const StageOps *ops() {
         static const StageOps o = {D, M, PDE, RDEG, RBasis<D, RDEG>::B, &gather, &flux, &stage1, &cfl,
                                    ((M == 1 && PDE == HCC_PDE_ADVECTION) || RDEG == 1) ? &weno : nullptr,
                                    RDEG == 1 ? &central : nullptr,
                                    (RDEG == 1 && M == 1 && PDE == HCC_PDE_ADVECTION) ? &upwind : nullptr,
-                                   (PDE == HCC_PDE_EULER && RDEG == 1) ? &weno_geom : nullptr};
+                                   (PDE == HCC_PDE_EULER && RDEG == 1) ? &weno_geom : nullptr, &tile_setup};
         return &o;
     }
 };
