@@ -115,3 +115,12 @@ def test_reconstruction_of_a_squeezed_cloud(hcc, cuda_lib):
     """Tile-staged reconstruction where the fits are ill-conditioned: 1.061 times the stream-fed passes' error with the
     gradient weights formed per slot, bounded by 1.064 (the inputs are fixed)."""
     assert _tiled_over_streamed(hcc, _squeezed(hcc), range(6)) < 1.064
+
+
+def test_offsets_of_interior_tiles(hcc, cuda_lib):
+    """Tiles of the interior list reach farther than tiles of consecutive particles, so their offsets need the finer
+    quantum: 1.014 times the stream-fed passes' error with tiles of all particles, bounded by that for these too (the inputs
+    are fixed)."""
+    h = 1.0 / 31
+    cloud = hcc.rectangular_cloud((0.0,) * 3, (1.0,) * 3, h, 2.5 * h, jitter=0.25 * h, seed=31)
+    assert _tiled_over_streamed(hcc, cloud, range(8)) < 1.0145
