@@ -236,10 +236,10 @@ struct hcc_ctx {
     TileTables tiles;                            // tile staging of the FP32 full passes (hcc_tiles.cu)
     int tile_enabled = 2;                        // 0 / 1: chosen by the caller; 2: where it measured faster
     // 3-D stencils (K ~ 66): flux 7.05 against 10.4 ms at 8.0M points. Wide linear systems: flux 650 against 1007 us. 2-D
-    // stencils of Euler (K ~ 20), of which the flux pass alone is tile-staged: 893 against 970 us a step at 1.0M, 315
-    // against 359 at 160k; below 32 tiles most of the chip has no tile, and the gain is within the launches' noise.
-    // (2-D advection: 156 against 179 us at 160k, 620 against 611 at 1.0M, with up to 10 % more rounding error from the
-    // recomputed weights, of which its right-hand side has little else: stream-fed.)
+    // stencils of Euler (K ~ 20), of which the flux pass alone is tile-staged (the slot streams stay, and the bits with
+    // them): 1045 against 1120 us a step at 1.0M, 362 against 393 at 160k, 263 against 262 at 90k, 167 against 178 at
+    // 4.4k; below 32 tiles most of the chip has no tile, and the gain is within the launches' noise.
+    // (2-D advection: 234 against 208 us at 160k, 128 against 133 at 10k: stream-fed.)
     bool tiles_on() const {
         if (!tiles.ok || moving() || tile_enabled == 0) return false;
         if (tile_enabled == 1 || D == 3 || (cfg.pde != HCC_PDE_EULER && M >= 8)) return true;

@@ -47,6 +47,10 @@
 #define HCC_TILE_FLUX_GROUP 2      // tile-staged flux pass: union places in groups of this size, the slot body unrolled
                                    // over a group (0: a rotating window of HCC_TILE_FLUX_PF places)
 #endif
+#ifndef HCC_TILE_STREAM_GROUP
+#define HCC_TILE_STREAM_GROUP 2    // tile-staged flux pass of 1-D and 2-D clouds: slots of the streams in groups of this size,
+                                   // the next group in flight (2-D Euler at 1.0 M: 1045 us a step, 1182 with one)
+#endif
 #ifndef HCC_FLUX_STREAM_GROUP
 #define HCC_FLUX_STREAM_GROUP 1    // stream-fed FP32 full flux pass: slots in groups of this size, the body unrolled
 #endif
@@ -286,8 +290,9 @@ template <typename T> struct Geometry {
 // multiples of the tile's power-of-two quantum (so x_j - x_i is an exact integer difference, rounded once when
 // converted to FP32); per particle the FP32 rows of its cached fits: A_d and B_de of the divergence weights
 // dw_k[d] = w_k (A_d + sum_e B_de x_e) and G_bc of the gradient weights gw_k[b] = w_k sum_c G_bc x_c, with
-// w_k = w(|x_k|^2) the weight function. The slot streams of distances, weights and divergence weights are then
-// never read by the full passes: they recompute them from positions that come from shared memory.
+// w_k = w(|x_k|^2) the weight function. The 3-D full passes then never read the slot streams of distances, weights and
+// divergence weights: they recompute them from positions that come from shared memory. (The 1-D, 2-D and wide linear
+// passes read the streams and take only the neighbours' rows from shared memory.)
 #ifndef HCC_TILE
 #define HCC_TILE 128
 #endif

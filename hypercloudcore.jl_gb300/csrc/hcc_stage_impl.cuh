@@ -1864,13 +1864,14 @@ __global__ void __launch_bounds__(32 * flux_split_warps<D, M>()) k_flux_tiles(co
 // consecutive particles first copies the tile's neighbour union into shared memory -- positions (and orders), states,
 // and for the flux pass the gradients; a thread copies whole entries, and the ascending union ids make a warp's loads
 // cover contiguous runs -- then every slot reads its neighbour from shared memory with 16-byte loads. Offsets
-// x_j - x_i are exact differences of the quantised union positions, rounded once to FP32; the weight w(|x|^2) and the
-// slot's gradient and divergence weights follow from the particle's FP32 fit rows. The arithmetic after that is
+// x_j - x_i are (in 3-D) exact differences of the quantised union positions, rounded once to FP32; the weight w(|x|^2) and
+// the slot's gradient and divergence weights follow from the particle's FP32 fit rows. The arithmetic after that is
 // flux_slot / the cached gather of the stream-fed passes. Each thread loads the union place of its next slot while
 // it computes the current one.
 
 // Shared-memory layout. Gather pass: one row per union entry, the position (D ints) then the state. Flux pass: an
-// int4 array of positions (the order in .w), then one row per entry of the state and the gradient. Rows are whole
+// int4 array of positions (the order in .w), then one row per entry of the state and the gradient; without positions
+// (1-D, 2-D) the rows, then the orders. Rows are whole
 // 16-byte groups, an odd number of them, so the rows that the lanes of a warp read spread over the banks.
 constexpr int tile_odd_groups(int words) {
     const int g = (words + 3) / 4;
@@ -2064,11 +2065,17 @@ __global__ void __launch_bounds__(2 * HCC_TILE, 3) k_gather_tile(const StageArgs
 
 // Flux pass, two threads per particle of the tile in 3-D (slots k = h, h + 2, ... for h = 0, 1); the second writes its
 // compensated partial sums and extrema to shared memory, the first combines them and runs the epilogue. (Four threads and
-// one block an SM where that saves a wave: never faster on 11 k to 290 k interior particles, at most 12 % slower.) In 2-D
-// one thread: with 20 slots the combination and the idle half of the epilogue cost more than the second thread gives
-// (970 us a step stream-fed, 893 with one thread, 1256 with two, 2-D Euler at 1.0M).
+// one block an SM where that saves a wave: never faster on 11 k to 290 k interior particles, at most 12 % slower.)
+// In 2-D and 1-D one thread: with 20 slots the combination and the idle half of the epilogue cost more than the second
+// thread gives. There the offsets and divergence weights come from the FP32 slot streams, and every slot is compensated on
+// its own, so the results have the bits of the stream-fed pass (in 2-D): only the neighbours' rows come from shared
+// memory. 2-D Euler, us a step with tiles / stream-fed: 167 / 178 at 4.4 k interior particles, 189 / 199 at 10 k,
+// 228 / 234 at 53 k, 263 / 262 at 90 k, 362 / 393 at 160 k, 679 / 711 at 518 k, 1045 / 1120 at 1.0 M. (Offsets and weights
+// recomputed from the quantised positions, sums compensated in blocks of four: no faster, and up to 0.5 % more error of the
+// right-hand side. Four blocks an SM 1144, six 1117 at 1.0 M.)
 template <int D> constexpr int tile_flux_threads() { return D == 3 ? 2 : 1; }
 template <int D> constexpr int tile_flux_min_blocks() { return D == 3 ? 2 : 5; }
+template <int D> constexpr bool tile_flux_streams() { return D < 3; }
 
 // PLAIN: EPD1 interface orders and the plain Rusanov flux (the usual configuration), known at compile time.
 template <int D, int M, int PDE, bool PLAIN>
@@ -2077,11 +2084,13 @@ __global__ void __launch_bounds__(tile_flux_threads<D>() * HCC_TILE, tile_flux_m
     constexpr int W = tile_flux_row<D, M>();
     constexpr int RW = M + D * M;                 // used words of a row: the state, then the gradient
     constexpr int GS = grad_row<float, D * M>(), HT = tile_flux_threads<D>();
+    constexpr bool STREAMS = tile_flux_streams<D>();
     const int64_t t = blockIdx.x;
     const int64_t u0 = a.tv.ustart[t];
     const int nu = int(a.tv.ustart[t + 1] - u0);
-    int4 *spos = reinterpret_cast<int4 *>(sm);
-    float *srow = sm + 4 * a.tv.umax;
+    int4 *spos = reinterpret_cast<int4 *>(sm);    // positions and orders, then the rows; without positions the rows,
+    float *srow = sm + (STREAMS ? 0 : 4 * a.tv.umax);                                      // then the orders
+    int *sord = reinterpret_cast<int *>(srow + a.tv.umax * W);
     FluxPart<float, M> *parts = reinterpret_cast<FluxPart<float, M> *>(sm);   // over the union, once it has been read
     // the particle's own global loads (count, union place, fit rows, the first union places of its slots) are issued
     // before the staging so that their latency overlaps it; none of them reads shared memory
@@ -2091,7 +2100,7 @@ __global__ void __launch_bounds__(tile_flux_threads<D>() * HCC_TILE, tile_flux_m
     const int64_t np = a.g.npad;
     // this thread's slots h, h + HT, ...: union places PF slots ahead (a rotating window), or in groups of PF with the
     // next group in flight (HCC_TILE_FLUX_GROUP > 0: the slot body unrolled over the group)
-    constexpr int GROUP = HCC_TILE_FLUX_GROUP;
+    constexpr int GROUP = STREAMS ? HCC_TILE_STREAM_GROUP : HCC_TILE_FLUX_GROUP;
     constexpr int PF = GROUP > 0 ? GROUP : HCC_TILE_FLUX_PF;
     const int64_t lstep = HT * np;
     const uint16_t *lp = a.tv.lidx + int64_t(h) * np + i;
@@ -2099,20 +2108,33 @@ __global__ void __launch_bounds__(tile_flux_threads<D>() * HCC_TILE, tile_flux_m
     bool wok = false;
     int lb[PF];
     float A[D], B[D][D];
+    float xb[PF][D], wb[PF][D];                   // the offsets and divergence weights of a group's slots (STREAMS)
+    auto stream = [&](int s, float *x, float *w) {
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+            x[d] = s < mine ? a.g.dist[(int64_t(s) * D + d) * np + i] : 0.0f;
+            w[d] = s < mine ? a.g.dw[(int64_t(s) * D + d) * np + i] : 0.0f;
+        }
+    };
     if (live) {
         cnt = a.g.cnt[i];
         li = int(a.tv.lself[i]);
         wok = cnt > 0 && a.g.ok_d[i];
-        const float *cf = a.tv.coef + i * a.tv.cw;
+        if constexpr (!STREAMS) {
+            const float *cf = a.tv.coef + i * a.tv.cw;
 #pragma unroll
-        for (int d = 0; d < D; ++d) {
-            A[d] = cf[d];
+            for (int d = 0; d < D; ++d) {
+                A[d] = cf[d];
 #pragma unroll
-            for (int e = 0; e < D; ++e) B[d][e] = cf[D + d * D + e];
+                for (int e = 0; e < D; ++e) B[d][e] = cf[D + d * D + e];
+            }
         }
         mine = cnt > h ? (cnt - h + HT - 1) / HT : 0;
 #pragma unroll
-        for (int q = 0; q < PF; ++q) lb[q] = q < mine ? int(lp[int64_t(q) * lstep]) : 0;
+        for (int q = 0; q < PF; ++q) {
+            lb[q] = q < mine ? int(lp[int64_t(q) * lstep]) : 0;
+            if constexpr (STREAMS) stream(q, xb[q], wb[q]);
+        }
         lp += int64_t(PF) * lstep;
     }
     {
@@ -2129,7 +2151,7 @@ __global__ void __launch_bounds__(tile_flux_threads<D>() * HCC_TILE, tile_flux_m
             for (int u = 0; u < SU; ++u) {
                 if (e0 + u * nt >= nu) break;
                 const int64_t j = jj[u];
-                qq[u] = a.tv.upos[u0 + e0 + u * nt];
+                if constexpr (!STREAMS) qq[u] = a.tv.upos[u0 + e0 + u * nt];
                 qq[u].w = a.orders[j];
 #pragma unroll
                 for (int m = 0; m < M; ++m) v[u][m] = a.U[j * M + m];
@@ -2138,21 +2160,28 @@ __global__ void __launch_bounds__(tile_flux_threads<D>() * HCC_TILE, tile_flux_m
 #pragma unroll
             for (int u = 0; u < SU; ++u) {
                 if (e0 + u * nt >= nu) break;
-                spos[e0 + u * nt] = qq[u];
+                if constexpr (STREAMS) sord[e0 + u * nt] = qq[u].w;
+                else spos[e0 + u * nt] = qq[u];
                 sts_words<RW>(srow + (e0 + u * nt) * W, v[u]);
             }
         }
     }
     __syncthreads();
     const bool need_ext = a.check && (a.sc.criterion == HCC_MOOD_U1 || a.sc.criterion == HCC_MOOD_U2);
-    BlockAccum<M, HCC_FLUX_KAHAN_BLOCK> blk;
+    // (with the streams each slot is compensated on its own, as in the stream-fed pass)
+    BlockAccum<M, STREAMS ? 1 : HCC_FLUX_KAHAN_BLOCK> blk;
     AccumV<float, M> &acc = blk.sum;
     float mn[M], mx[M], fi[M];
     float gi[D][M], Fi[D][M];
     if (live) {
-        const int4 q4 = spos[li];
-        const int qi[3] = {q4.x, q4.y, q4.z};
-        const int oi_own = q4.w;
+        int qi[3] = {0, 0, 0}, oi_own;
+        if constexpr (STREAMS) {
+            oi_own = sord[li];
+        } else {
+            const int4 q4 = spos[li];
+            qi[0] = q4.x; qi[1] = q4.y; qi[2] = q4.z;
+            oi_own = q4.w;
+        }
         {
             float own[RW];
             lds_words<RW>(srow + li * W, own);
@@ -2165,22 +2194,30 @@ __global__ void __launch_bounds__(tile_flux_threads<D>() * HCC_TILE, tile_flux_m
         }
         own_flux<float, D, M, PDE, false, false>(a.ph, fi, Fi, nullptr);
         if (wok) {
-            const float qt = a.tv.quantum[t], ws = a.tv.wscale;
-            auto slot = [&](const int l, const int k) {
-                const int4 qj4 = spos[l];
-                const int qj[3] = {qj4.x, qj4.y, qj4.z};
+            const float qt = STREAMS ? 0.0f : a.tv.quantum[t], ws = a.tv.wscale;
+            auto slot = [&](const int l, const float *xs, const float *wsl, const int k) {
                 float dk[D], wk[D];
-                tile_offset<D>(qj, qi, qt, dk);
-                float r2 = dk[0] * dk[0];
+                int oj_own;
+                if constexpr (STREAMS) {
+                    oj_own = sord[l];
 #pragma unroll
-                for (int d = 1; d < D; ++d) r2 = r2 + dk[d] * dk[d];
-                const float w = tile_weight(r2, ws);
+                    for (int d = 0; d < D; ++d) { dk[d] = xs[d]; wk[d] = wsl[d]; }
+                } else {
+                    const int4 qj4 = spos[l];
+                    const int qj[3] = {qj4.x, qj4.y, qj4.z};
+                    oj_own = qj4.w;
+                    tile_offset<D>(qj, qi, qt, dk);
+                    float r2 = dk[0] * dk[0];
 #pragma unroll
-                for (int d = 0; d < D; ++d) {
-                    float v = A[d];
+                    for (int d = 1; d < D; ++d) r2 = r2 + dk[d] * dk[d];
+                    const float w = tile_weight(r2, ws);
 #pragma unroll
-                    for (int e = 0; e < D; ++e) v = v + B[d][e] * dk[e];
-                    wk[d] = w * v;
+                    for (int d = 0; d < D; ++d) {
+                        float v = A[d];
+#pragma unroll
+                        for (int e = 0; e < D; ++e) v = v + B[d][e] * dk[e];
+                        wk[d] = w * v;
+                    }
                 }
                 float r[RW];
                 lds_words<RW>(srow + l * W, r);
@@ -2188,7 +2225,6 @@ __global__ void __launch_bounds__(tile_flux_threads<D>() * HCC_TILE, tile_flux_m
 #pragma unroll
                     for (int m = 0; m < M; ++m) { mn[m] = vmin(mn[m], r[m]); mx[m] = vmax(mx[m], r[m]); }
                 }
-                const int oj_own = qj4.w;
                 int oi, oj;
                 if (PLAIN || a.sc.strategy == HCC_EPD1) { oi = oj = (oi_own < oj_own ? oi_own : oj_own); }
                 else { oi = oi_own; oj = oj_own; }
@@ -2200,25 +2236,35 @@ __global__ void __launch_bounds__(tile_flux_threads<D>() * HCC_TILE, tile_flux_m
             if constexpr (GROUP > 0) {
                 for (int s0 = 0; s0 < mine; s0 += PF) {
                     int ln[PF];
+                    float xn[PF][D], wn[PF][D];
 #pragma unroll
-                    for (int q = 0; q < PF; ++q) ln[q] = s0 + PF + q < mine ? int(lp[int64_t(q) * lstep]) : 0;
+                    for (int q = 0; q < PF; ++q) {
+                        ln[q] = s0 + PF + q < mine ? int(lp[int64_t(q) * lstep]) : 0;
+                        if constexpr (STREAMS) stream(s0 + PF + q, xn[q], wn[q]);
+                    }
                     lp += int64_t(PF) * lstep;
 #pragma unroll
                     for (int q = 0; q < PF; ++q) {
                         if (s0 + q >= mine) break;
-                        slot(lb[q], h + HT * (s0 + q));
+                        slot(lb[q], xb[q], wb[q], h + HT * (s0 + q));
                     }
 #pragma unroll
-                    for (int q = 0; q < PF; ++q) lb[q] = ln[q];
+                    for (int q = 0; q < PF; ++q) {
+                        lb[q] = ln[q];
+                        if constexpr (STREAMS)
+#pragma unroll
+                            for (int d = 0; d < D; ++d) { xb[q][d] = xn[q][d]; wb[q][d] = wn[q][d]; }
+                    }
                 }
             } else {
+                static_assert(!STREAMS || GROUP > 0, "the streams come in groups");
                 for (int s = 0; s < mine; ++s) {
                     const int l = lb[0];
 #pragma unroll
                     for (int q = 0; q + 1 < PF; ++q) lb[q] = lb[q + 1];
                     lb[PF - 1] = s + PF < mine ? int(*lp) : 0;
                     lp += lstep;
-                    slot(l, h + HT * s);
+                    slot(l, nullptr, nullptr, h + HT * s);
                 }
             }
             blk.flush();
@@ -2263,7 +2309,7 @@ __global__ void __launch_bounds__(tile_flux_threads<D>() * HCC_TILE, tile_flux_m
 #pragma unroll
             for (int m = 0; m < M; ++m) {
                 if constexpr (HT == 1) {
-                    Kv[m] = -(acc.s[m] - acc.c[m]);
+                    Kv[m] = -acc.s[m];
                 } else {
                     const float s1 = parts[pl].s[m];
                     const float u = acc.s[m] + s1;
@@ -2632,7 +2678,7 @@ template <int D, int M> inline size_t tile_gather_smem(int umax) {
     return (size_t(umax) * tile_gather_row<D, M>() + size_t(HCC_TILE) * D * M) * sizeof(float);
 }
 template <int D, int M> inline size_t tile_flux_smem(int umax) {
-    return std::max(size_t(umax) * (4 + tile_flux_row<D, M>()) * sizeof(float),
+    return std::max(size_t(umax) * ((tile_flux_streams<D>() ? 1 : 4) + tile_flux_row<D, M>()) * sizeof(float),
                     size_t(tile_flux_threads<D>() - 1) * HCC_TILE * sizeof(FluxPart<float, M>));
 }
 

@@ -478,12 +478,17 @@ const char *hcc_build_info(void);
    neighbours through the slot views, NeighbourViews.jl:11-43). For an FP32 context with MUSCL of order <= 2, the
    degree-1 divergence fit, EPD0/EPD1/StrictEPD0 interface orders and a fixed grid, hcc_prepare_geometry also builds
    tile tables: per tile of 128 consecutive particles the union of their neighbours, which one thread block stages in
-   shared memory, and per slot the neighbour's place in it; the full passes then recompute the slot offsets, weights
-   and divergence / gradient weights from quantised positions and per-particle FP32 fit rows instead of reading the
-   per-slot streams. Results agree with the stream-fed passes to FP32 rounding (both round the same FP64 geometry).
+   shared memory, and per slot the neighbour's place in it. What reads them:
+   - 3-D, up to five variables: reconstruction, flux and CFL pass, which recompute the slot offsets, weights and divergence /
+     gradient weights from quantised positions and per-particle FP32 fit rows instead of reading the slot streams. Results
+     agree with the stream-fed passes to FP32 rounding (both round the same FP64 geometry).
+   - 1-D and 2-D, up to four variables: the flux pass, which keeps the slot streams and takes the neighbours' rows from
+     shared memory; in 2-D the results have the bits of the stream-fed passes.
+   - linear systems of eight variables and more: the flux pass likewise. (Their reconstruction has lanes that share a
+     particle, staged or not.)
    Enabled by default where it measured faster than the stream-fed passes: 3-D contexts (about 66 neighbours a
-   particle), linear systems of eight variables and more, and 2-D Euler contexts from 4,096 interior particles on, of
-   which the flux pass alone is tile-staged. Off by default elsewhere; enable = 1 / 0 chooses either way. */
+   particle), linear systems of eight variables and more, and 2-D Euler contexts from 4,096 interior particles on.
+   Off by default elsewhere; enable = 1 / 0 chooses either way. */
 hcc_status hcc_set_tile_staging(hcc_ctx *ctx, int32_t enable);
 /* Whether the full passes of the next step are tile-staged, the union entries over all tiles and the largest union
    (any output may be NULL). */
