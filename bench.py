@@ -442,12 +442,14 @@ def per_launch(kt, name):
 def roofline_of(workload, D, M, K, n_int, kt, peak, peak_kind, tiled=False):
     """The flux pass (dominant kernel) and the reconstruction pre-pass against the HBM copy peak: algorithmic bytes
     per point-stage x interior points / CUDA-event launch time; `traffic` = the ncu DRAM bytes per point-stage of
-    profiles/traffic.txt for this workload, scaled to the launch. `tiled`: the tile-staged passes ran."""
+    profiles/traffic.txt for this workload and the pass that ran, scaled to the launch. `tiled`: the tile-staged passes
+    ran (the flux pass alone in 2-D)."""
     flux_b, gather_b = algorithmic_bytes(K, D, M, D, D + 1, 4)
     rec = recorded_traffic()
     flux_ms, gather_ms = per_launch(kt, "flux"), per_launch(kt, "gather")
     achieved = flux_b * n_int / (flux_ms / 1e3) / 1e9
-    traffic = rec.get(f"flux_f32_{workload}_bytes_per_point_stage")
+    form = "flux_tile" if tiled and D < 3 else "flux"
+    traffic = rec.get(f"{form}_f32_{workload}_bytes_per_point_stage")
     g_traffic = rec.get(f"gather_f32_{workload}_bytes_per_point_stage")
     g_model = gather_b * n_int / (gather_ms / 1e3) / 1e9
     gname = f"k_gather_tile<{D},{M},EULER>" if tiled and D == 3 else f"k_gather<float,{D},{M},EULER,1>"
@@ -465,15 +467,28 @@ def roofline_of(workload, D, M, K, n_int, kt, peak, peak_kind, tiled=False):
             "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum per point-stage (profiles/traffic.txt)"
                               " x interior points",
             "algorithmic_bytes_per_point_stage": {"flux": flux_b, "gather": gather_b},
-            "limiter": ("FP32 instruction issue, not HBM: 68 % issue-active, FMA pipe 47 %, DRAM traffic 1.1x the model "
-                        "bytes (ncu, profiles/stage_f32_euler3d_blast_262k_tile.md)") if tiled else
-                       ("issue / latency (ncu, profiles/stage_f32_euler2d_quadrant_1M.md)"),
+            "limiter": flux_limiter(D, tiled),
             "flux_ms_per_launch": flux_ms, "gather_ms_per_launch": gather_ms,
             "recompute_ms_total": kt["recompute_ms"], "recompute_launches": kt["recompute_launches"],
             "predict_ms_per_step": kt["predict_ms"] / max(kt["steps"], 1),
             "kernel_times": "CUDA events on the context's stream around each launch of a separate host-driven run "
                             "of the same steps",
             "gather": gather_roof}
+
+
+def flux_limiter(D, tiled):
+    """What bounds the FP32 flux pass that ran, from its own capture."""
+    if tiled and D == 3:
+        return ("FP32 instruction issue, not HBM: 68 % issue-active, FMA pipe 47 %, DRAM traffic 1.1x the model "
+                "bytes (ncu, profiles/stage_f32_euler3d_blast_262k_tile.md)")
+    if tiled:
+        return "issue / latency of the slot streams"
+    return "issue / latency (ncu, profiles/stage_f32_euler2d_quadrant_1M.md)"
+
+
+def fp64_flux_kernel(D, M, n_int):
+    """The kernel of a full FP64 flux pass of Euler: eight lanes a particle in 3-D and on small clouds."""
+    return f"k_flux_split<{D},{M},EULER,1>" if D == 3 or n_int <= 24000 else f"k_flux<double,{D},{M},EULER,1>"
 
 
 def fp64_roofline(D, M, K, n_int, kt, fp64_peak):
@@ -484,7 +499,7 @@ def fp64_roofline(D, M, K, n_int, kt, fp64_peak):
     flops = fp64_flops_per_slot(D, M)
     ms = per_launch(kt, "flux")
     achieved = flops * K * n_int / (ms / 1e3) / 1e12
-    return {"bound": "fp64", "kernel": f"k_flux<double,{D},{M},EULER,1>", "flops_per_slot": flops,
+    return {"bound": "fp64", "kernel": fp64_flux_kernel(D, M, n_int), "flops_per_slot": flops,
             "achieved": achieved, "unit": "TFLOP/s", "peak": fp64_peak.get("tflops") if fp64_peak else None,
             "frac": (achieved / fp64_peak["tflops"]) if fp64_peak and fp64_peak.get("tflops") else None,
             "peak_source": fp64_peak.get("source") if fp64_peak else None, "flux_ms_per_launch": ms,
