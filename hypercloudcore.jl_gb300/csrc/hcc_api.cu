@@ -199,7 +199,6 @@ struct hcc_ctx {
     float *wops = nullptr; int32_t *wcnt = nullptr;             // FP32 Euler WENO operators, stencil sizes
     double *wchol = nullptr; uint8_t *wok = nullptr;             // FP64 Euler WENO: packed factors and flags
     double *wflux64 = nullptr;                                    // FP64 Euler WENO: the stage's flux table
-    std::vector<uint8_t> h_bnd; std::vector<int32_t> h_tags;
     // cell list
     int dims[3] = {1, 1, 1}; double csize[3] = {1, 1, 1};
     int64_t nbins = 0; int noff = 1;
@@ -1302,8 +1301,6 @@ hcc_status hcc_upload_cloud(hcc_ctx *c, int64_t n, const double *pos, const uint
     std::vector<double> soa(size_t(D) * np, 0.0);
     for (int64_t i = 0; i < n; ++i)
         for (int d = 0; d < D; ++d) soa[d * np + i] = pos[i * D + d];
-    c->h_bnd.assign(is_boundary, is_boundary + n);
-    c->h_tags.assign(tags, tags + n);
     c->n_interior = 0;
     for (int64_t i = 0; i < n; ++i) c->n_interior += is_boundary[i] ? 0 : 1;
     std::vector<double> v(size_t(std::max<int64_t>(n, 1)), 1.0);

@@ -210,7 +210,6 @@ template <typename T> __device__ __forceinline__ bool positive(T x) { return x >
 template <> __device__ __forceinline__ bool positive<double>(double x) {
     return (unsigned long long)(__double_as_longlong(x) - 1) < 0x7ff0000000000000ull;
 }
-// x or -x by the sign bit
 // |a| >= |b| and neither a NaN; FP64 as integers (magnitudes order like their words, a NaN's above infinity's).
 template <typename T> __device__ __forceinline__ bool covers(T a, T b) { return fabs(a) >= fabs(b); }
 template <> __device__ __forceinline__ bool covers<double>(double a, double b) {
@@ -218,6 +217,7 @@ template <> __device__ __forceinline__ bool covers<double>(double a, double b) {
     const unsigned long long wa = __double_as_longlong(a) & m, wb = __double_as_longlong(b) & m;
     return wa >= wb && wa <= inf;
 }
+// x or -x by the sign bit
 __device__ __forceinline__ double negate_if(double x, bool neg) {
     return __longlong_as_double(__double_as_longlong(x) ^ (neg ? (long long)0x8000000000000000ull : 0ll));
 }
