@@ -659,8 +659,9 @@ __device__ __forceinline__ void gather_one(const StageArgs<T> &a, const int64_t 
         for (int b = 0; b < BR; ++b)
 #pragma unroll
             for (int m = 0; m < M; ++m) bs[b][m] = T(0);
-        // slots in groups, as above: one at a time for several variables (registers)
-        constexpr int G = M == 1 ? 4 : 1;
+        // slots in groups, as above: one at a time for several variables, two for a 3-D scalar (registers; four of them in
+        // 3-D: 1979 us a step with limiter, two 1762)
+        constexpr int G = M == 1 ? (D == 3 ? 2 : 4) : 1;
         int32_t j[G];
         T dk[G][D], wk[G];
         auto stream = [&](int k, int32_t *jk, T(*d)[D], T *w) {
@@ -930,13 +931,22 @@ __global__ void __launch_bounds__(32 * split_warps<M>()) k_gather_tiles(const St
     }
 }
 
+// Blocks an SM of the stream-fed reconstruction pass in FP32. One variable: nine in 1-D and 2-D (flux_min_blocks), eight in
+// 3-D, where a slot's basis is longer and nine spilled up to 540 bytes a thread. 3-D, 343k interior particles, order 3, us
+// a step: 1938 (limiter 1711) with eight here and seven in the flux pass, 2754 (2257) with nine in both, 2483 (2213)
+// when one slot was in flight.
+template <typename T, int D, int M> constexpr int gather_min_blocks() {
+    if (sizeof(T) == 8) return 1;
+    return M == 1 ? (D == 3 ? 8 : 9) : 1;
+}
+
 // A full pass (one thread per particle) or a worklist pass over tiles (the members of a word) that also marks the one-hop
 // reach of each member in rmask / rtiles. Most listed members have dropped to order 1 and have nothing to fit: the pass
 // is bound by the marks, slot after slot, so a list of no more tiles than warps gives each tile a block, whose warps
 // share the slots, and a longer one a warp: all passes of an FP64 3-D step 707 -> 307 us (65.6 k interior particles, a
 // third of them listed), of a moving 2-D one 123 -> 46 us.
 template <typename T, int D, int M, int PDE, int RDEG, bool LIM>
-__global__ void __launch_bounds__(128, sizeof(T) == 4 && M == 1 ? 9 : 1) k_gather(const StageArgs<T> a) {
+__global__ void __launch_bounds__(128, gather_min_blocks<T, D, M>()) k_gather(const StageArgs<T> a) {
     if (a.full) {
         const int64_t i = full_particle(a, int64_t(blockIdx.x) * blockDim.x + threadIdx.x);
         if (i >= 0) gather_one<T, D, M, PDE, RDEG, LIM>(a, i);
@@ -1145,13 +1155,14 @@ __device__ __forceinline__ int interface_terms(int o) {
 }
 
 // Resident blocks per SM the flux kernel is compiled for: as many as its registers allow without spilling
-// (FP32 2-D scalar/Euler: 72 registers; wider states and FP64 need more).
+// (FP32 2-D Euler and 3-D scalars: 72 registers; wider states and FP64 need more), but for 1-D and 2-D scalars.
 template <typename T, int D, int M> constexpr int flux_min_blocks() {
     if (sizeof(T) == 8) return M >= 8 ? 1 : (D * M >= 12 ? 2 : HCC_FLUX_MINB64);
-    // one variable: a slot is few instructions and three dependent gathers, so the pass waits, and 36 warps an SM wait
-    // better than 28 (56 registers, some 50 bytes spilled; order 3 with limiter, 1.0 M: 3857 us for four steps with nine
-    // blocks an SM, 3926 with eight, 4222 with seven, 4441 with ten; the same for the reconstruction)
-    return M >= 8 ? HCC_FLUX_MINB_MANY : (D * M >= 12 ? HCC_FLUX_MINB_WIDE : M == 1 ? 9 : HCC_FLUX_MINB);
+    // one variable in 1-D and 2-D: a slot is few instructions and three dependent gathers, so the pass waits, and 36 warps an
+    // SM wait better than 28 (56 registers, 46 to 68 bytes spilled in 2-D at order 3; with limiter, 1.0 M: 3857 us for four
+    // steps with nine blocks an SM in this pass and the reconstruction, 3926 with eight, 4222 with seven, 4441 with ten). In
+    // 3-D the spills cost more than the warps give: see gather_min_blocks.
+    return M >= 8 ? HCC_FLUX_MINB_MANY : (D * M >= 12 ? HCC_FLUX_MINB_WIDE : M == 1 && D < 3 ? 9 : HCC_FLUX_MINB);
 }
 
 // The MUSCL functor (MUSCL.jl:390-508) in its streamed form: per slot, EPD interface reconstruction, physical
