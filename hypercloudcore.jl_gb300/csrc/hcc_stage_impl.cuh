@@ -613,8 +613,9 @@ __device__ __forceinline__ void gather_one(const StageArgs<T> &a, const int64_t 
         // FP32, degree 1: the cached fit as one weight vector per slot (nidx + D floats per slot)
         if (p == a.sc.max_order && p > 1 && a.g.ok_r[i] && a.g.gw) {
             // slots in groups of G: the states of a group, and the indices and weights of the next, are in flight
-            // while the group is summed (an index is what its state's load waits for)
-            constexpr int G = 4;
+            // while the group is summed (an index is what its state's load waits for). Two with the extrema of a limited
+            // pair of variables: four of them spill within the bound of gather_min_blocks (449 us a step, 428 with two).
+            constexpr int G = LIM && M == 2 ? 2 : 4;
             int32_t j[G];
             T gk[G][D];
             auto stream = [&](int k, int32_t *jk, T(*g)[D]) {
@@ -934,10 +935,12 @@ __global__ void __launch_bounds__(32 * split_warps<M>()) k_gather_tiles(const St
 // Blocks an SM of the stream-fed reconstruction pass in FP32. One variable: nine in 1-D and 2-D (flux_min_blocks), eight in
 // 3-D, where a slot's basis is longer and nine spilled up to 540 bytes a thread. 3-D, 343k interior particles, order 3, us
 // a step: 1938 (limiter 1711) with eight here and seven in the flux pass, 2754 (2257) with nine in both, 2483 (2213)
-// when one slot was in flight.
+// when one slot was in flight. Two variables in 2-D: ten (48 registers; a warp waits for its gathers); 360k particles, us a
+// step with Barth-Jespersen limiter / without: 423 / 414 with ten, 461 / 415 with eight, 501 / 425 unbounded (80 and 76
+// registers), 442 / 433 with one thread's slots in three sweeps.
 template <typename T, int D, int M> constexpr int gather_min_blocks() {
     if (sizeof(T) == 8) return 1;
-    return M == 1 ? (D == 3 ? 8 : 9) : 1;
+    return M == 1 ? (D == 3 ? 8 : 9) : M == 2 && D == 2 ? 10 : 1;
 }
 
 // A full pass (one thread per particle) or a worklist pass over tiles (the members of a word) that also marks the one-hop

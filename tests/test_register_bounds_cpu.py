@@ -39,3 +39,11 @@ def test_3d_scalar_passes_do_not_spill(tmp_path):
     assert len(got) == 6
     for name, (registers, spilled) in got.items():
         assert spilled == 0 and registers <= (64 if "gather" in name else 72), (name, registers, spilled)
+
+
+def test_2d_two_variable_reconstruction_keeps_its_warps(tmp_path):
+    """Ten blocks of four warps an SM: 48 registers."""
+    got = _compile(tmp_path, _instances("k_gather", "2, 2, HCC_PDE_ADVECTION, 1, false", "2, 2, HCC_PDE_ADVECTION, 1, true"))
+    assert len(got) == 2
+    for name, (registers, spilled) in got.items():
+        assert registers <= 51 and spilled <= 80, (name, registers, spilled)
