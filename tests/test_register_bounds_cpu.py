@@ -47,3 +47,8 @@ def test_2d_two_variable_reconstruction_keeps_its_warps(tmp_path):
     assert len(got) == 2
     for name, (registers, spilled) in got.items():
         assert registers <= 51 and spilled <= 80, (name, registers, spilled)
+
+
+def test_central_passes_take_the_list_in_fp64_only(tmp_path):
+    """The FP32 pass reads its slot streams in step with the warps."""
+    _compile(tmp_path, "static_assert(central_lists<double>() && !central_lists<float>(), \"lists of the central pass\");\n")
