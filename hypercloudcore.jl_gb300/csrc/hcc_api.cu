@@ -241,8 +241,21 @@ struct hcc_ctx {
     // (2-D advection: 234 against 208 us at 160k, 128 against 133 at 10k: stream-fed.)
     bool tiles_on() const {
         if (!tiles.ok || moving() || tile_enabled == 0) return false;
-        if (tile_enabled == 1 || D == 3 || (cfg.pde != HCC_PDE_EULER && M >= 8)) return true;
+        if (tile_enabled == 1 || D == 3) return true;
+        if (tiles.umax > default_union()) return false;
+        if (cfg.pde != HCC_PDE_EULER && M >= 8) return true;
         return D == 2 && cfg.pde == HCC_PDE_EULER && n_interior >= 32 * HCC_TILE;
+    }
+    // The largest union up to which tile staging is a default outside 3-D. Clouds numbered along a space-filling curve have
+    // unions of about 300 entries; long thin ones, and clouds numbered otherwise, larger ones, which cost staging and
+    // blocks an SM. 2-D Euler, stream-fed time over tile-staged: 1.02 to 1.09 up to 761 entries, 0.92 at 817, 1.01 at 864,
+    // 0.93 at 1034, 0.84 to 0.90 at 1300 to 1700, 0.64 at 2027 and 0.43 at 2481 (650k particles in random order: 2526
+    // against 1082 us a step). Wide linear systems need two blocks an SM (556 entries for 16 velocities): 1.3 up to 340,
+    // 1.10 to 1.15 at 400 to 533, 0.72 to 0.93 at 594 to 761.
+    int default_union() const {
+        if (M < 8) return 6 * HCC_TILE;
+        const int groups = (M + D * M + 1 + 3) / 4;          // the row of k_flux_wide, an odd number of 16-byte groups
+        return half_sm / (16 * (groups % 2 == 1 ? groups : groups + 1));
     }
     void apply_tuning() {
         list_blocks = std::max(1, sms) * tune.list_blocks_per_sm;
@@ -1662,12 +1675,12 @@ static hcc_status build_unions(hcc_ctx *c) {
     b.invL = c->invL;
     b.wscale = c->cfg.weight_alpha / (c->cfg.radius * c->cfg.radius);
     const int most = int(std::max(0L, budget / (4L * W)));
-    // Tiles of the interior list, where there is one, unless their unions cost the flux pass its second block on an SM:
-    // 128 interior particles spread wider than 128 consecutive ones (in 3-D at most 1162 against 963 entries on 64^3).
+    // Tiles of the interior list, where there is one, unless their unions cost the flux pass its second block on an SM (or,
+    // outside 3-D, the default): 128 interior particles spread wider than 128 consecutive ones (in 3-D at most 1162 against 963 entries on 64^3).
     if (c->skip_ghosts()) {
         b.members = c->ilist;
         b.nmem = c->n_interior;
-        b.max_union = M >= 8 ? most : std::min(most, c->half_sm / (4 * W));
+        b.max_union = std::min(most, D == 3 ? c->half_sm / (4 * W) : c->default_union());
         const hcc_status st = build_tile_tables(b, c->tiles, c->stream, c->err);
         c->tiles.listed = c->tiles.ok;
         if (st != HCC_OK || c->tiles.ok) return st;

@@ -108,3 +108,41 @@ def test_clouds_one_after_another(hcc, cuda_lib, kind, D, sizes, precision):
     for cloud in clouds:
         for a, b in zip(results(kept, cloud), results(context(), cloud)):
             assert np.ascontiguousarray(a).tobytes() == np.ascontiguousarray(b).tobytes()
+
+
+@pytest.mark.parametrize("kind", ["euler", "kinetic"])
+def test_default_form_follows_the_numbering(hcc, cuda_lib, kind):
+    """Tile staging by default for a cloud numbered along a curve; not for the same cloud in random order or in rows of a
+    long box, whose unions are too large (more than 768 entries; more than two blocks an SM hold for 16 velocities), though a
+    caller can still choose it; the steps of both forms agree bit for bit."""
+    h = 1.0 / 70
+    curve = hcc.rectangular_cloud((0.0, 0.0), (1.0, 1.0), h, 2.5 * h, jitter=0.2 * h, seed=1)
+    ring = tuple((float(np.cos(2 * np.pi * q / 16)), float(np.sin(2 * np.pi * q / 16))) for q in range(16))
+    pde = hcc.Euler(2) if kind == "euler" else hcc.KineticRelaxation(ring, epsilon=1e-3, macro_velocity=(1.0, 0.5))
+    q = np.random.default_rng(1).permutation(curve.n) if kind == "euler" else \
+        np.argsort(np.arange(curve.n) + np.random.default_rng(1).uniform(0, 480, curve.n))
+
+    def numbered(q):
+        return hcc.Cloud(curve.pos[q], curve.is_boundary[q], curve.tags[q], curve.volumes[q], curve.dx, curve.radius,
+                         curve.domain_min, curve.domain_max, curve.canvas_min, curve.canvas_max, curve.periodic)
+
+    for cloud, default in ((numbered(np.arange(curve.n)), True), (numbered(q), False)):
+        cfg = hcc.make_config(pde, cloud, scheme=hcc.MUSCL(2, 2), bc_map=OUTFLOW, precision="fp32",
+                              tableau="RK3_SSP" if kind == "euler" else "IMEX_ARS222",
+                              mood=hcc.MOOD(hcc.EPD1, hcc.MOODu1(1e-8)))
+        ctx = hcc.Context(cfg)
+        _prepare(ctx, cloud)
+        got = ctx.tile_staging()
+        assert bool(got["active"]) == default
+        assert (got["largest_union"] <= (768 if kind == "euler" else 556)) == default
+        U = _euler(cloud) if kind == "euler" else pde.maxwellian(1.0 + 0.2 * np.sin(2 * np.pi * cloud.pos[:, 0]))
+        out = []
+        for tiles in (False, True):
+            ctx.set_tile_staging(tiles)
+            assert bool(ctx.tile_staging()["active"]) == tiles
+            ctx.upload_state(U)
+            dt = 0.3 * ctx.time_step()
+            for _ in range(2):
+                ctx.step(0.0, dt)
+            out.append((ctx.download_state(), ctx.orders()))
+        assert out[0][0].tobytes() == out[1][0].tobytes() and np.array_equal(out[0][1], out[1][1])
