@@ -213,8 +213,12 @@ struct hcc_ctx {
     int32_t *status = nullptr, *root = nullptr;
     int32_t *blist = nullptr, *bsrc = nullptr; int64_t nbnd = 0;
     int32_t *ilist = nullptr;                    // the interior particles
-    // whether full passes run over the interior list: from one ghost in ten on. (A list costs the slot streams their
-    // alignment to the warps; without ghosts worth skipping it only loses.)
+    // Whether full passes run over the interior list: from one ghost in ten on. A list saves the ghosts' share of the lanes
+    // and costs the slot streams their alignment to the warps. Time without the list over time with it, FP64 3-D Euler:
+    // 1.04 from 5 to 22 % ghosts, 1.09 at 30 %; 2-D order 3: 1.00 to 1.15; FP32 3-D scalars of order 3: 1.00 at 5 %, 1.03
+    // at 10 %, 1.04 at 15 %, 1.12 at 22 %; FP32 3-D Euler (tiles; the number of tile waves counts for more): 1.02 at 5 %,
+    // 0.99 at 8 %, 1.10 at 10 %, 0.98 to 1.02 from 15 to 30 %, 1.08 and more at 24 to 40 % of 452k and 57k particles;
+    // FP32 2-D: 0.98 to 1.04 at any share. Below one in ten FP32 gains nothing that can be told from the waves.
     bool skip_ghosts() const { return nbnd * 10 >= n; }
     // state (element type double or float)
     void *rhos = nullptr, *cand = nullptr, *grad = nullptr;
@@ -244,7 +248,11 @@ struct hcc_ctx {
         if (tile_enabled == 1 || D == 3) return true;
         if (tiles.umax > default_union()) return false;
         if (cfg.pde != HCC_PDE_EULER && M >= 8) return true;
-        return D == 2 && cfg.pde == HCC_PDE_EULER && n_interior >= 32 * HCC_TILE;
+        // (five tiles are resident on an SM: a second wave that is less than half full costs more than the rows in shared
+        // memory give, 0.95 to 1.00 times the stream-fed speed from 103k to 134k particles; 1.03 at 97k, 1.07 at 150k, 1.02
+        // and more at the later waves)
+        const bool short_wave = tiles.ntiles > 5 * int64_t(sms) && tiles.ntiles < 7 * int64_t(sms);
+        return D == 2 && cfg.pde == HCC_PDE_EULER && n_interior >= 32 * HCC_TILE && !short_wave;
     }
     // The largest union up to which tile staging is a default outside 3-D. Clouds numbered along a space-filling curve have
     // unions of about 300 entries; long thin ones, and clouds numbered otherwise, larger ones, which cost staging and

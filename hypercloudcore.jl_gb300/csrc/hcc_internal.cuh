@@ -27,18 +27,26 @@
                                    // slower than scalar instructions in the tile-staged 3-D flux pass)
 #endif
 #ifndef HCC_SPLIT_WIDE_TILES
-#define HCC_SPLIT_WIDE_TILES 304   // FP32 worklist passes: lists of up to this many tiles take a whole block a tile (a
-                                   // 3-D step of 30 k to 1.0 M particles: as fast or up to 6 % slower with 1,216 or 4,864)
+#define HCC_SPLIT_WIDE_TILES 304   // FP32 worklist passes: lists of up to this many tiles take a whole block a tile, two
+                                   // blocks an SM. A step with 304 against none: 3 % (490 k particles) to 16 % (8 k)
+                                   // faster in 3-D, 2 to 4 % in 2-D; 76 and 152 lie between; 1,216 and 4,864: as fast
+                                   // or up to 6 % slower from 30 k to 1.0 M
 #endif
 #ifndef HCC_SPLIT64_FLUX
-#define HCC_SPLIT64_FLUX 24000     // FP64 full flux passes of 1-D and 2-D clouds up to this size: eight lanes a particle
-                                   // (2-D Euler at 66 k: 5709 us for two steps with them, 5183 without)
+// FP64 full flux passes of 1-D and 2-D clouds up to this size: eight lanes a particle. The one-thread pass steps up with
+// every 128 threads an SM (19.5 k particles), the split grows evenly. Time of a step with one thread over that with eight
+// lanes, in the flux and the reconstruction: 2-D advection 1.36 at 4 k, 1.16 at 9 k, 0.84 at 16 k, 0.92 at 22 k, 0.76 at
+// 32 k; order 3 1.38, 1.19, 0.93, 1.07, 0.90; Euler 1.80, 1.32, 0.89, 1.11, 0.85 (and 0.85 at 65 k); 1-D Euler 0.98 at 6 k,
+// 0.87 at 16 k. So it pays up to some 12 k particles and, but for advection, again where the second step begins.
+#define HCC_SPLIT64_FLUX 24000
 #endif
 #ifndef HCC_SPLIT64_GATHER
 #define HCC_SPLIT64_GATHER 24000   // FP64 full reconstruction passes likewise (3-D ones of both kinds: at any size)
 #endif
 #ifndef HCC_SPLIT64_LIST
-#define HCC_SPLIT64_LIST 400000    // FP64 worklist flux passes of clouds up to this size (their reach is a fraction of it)
+#define HCC_SPLIT64_LIST 400000    // FP64 worklist flux passes of clouds up to this size (their reach is a fraction of it): a
+                                   // step with jumps 1.49 times as fast with eight lanes at 16 k, 1.25 at 65 k, 1.10 at
+                                   // 160 k, 1.06 at 360 k, and 1.04 at 518 k, which the line leaves out
 #endif
 #ifndef HCC_TILE_FLUX_PF
 #define HCC_TILE_FLUX_PF 8         // tile-staged flux pass: union places of a thread's slots fetched this many slots ahead

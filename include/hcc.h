@@ -489,7 +489,8 @@ const char *hcc_build_info(void);
    Enabled by default where it measured faster than the stream-fed passes: 3-D contexts (about 66 neighbours a
    particle), linear systems of eight variables and more, and 2-D Euler contexts from 4,096 interior particles on; the last
    two where the largest union is small enough (a cloud numbered along a space-filling curve; a random numbering or a very
-   long box is not). Off by default elsewhere; enable = 1 / 0 chooses either way. */
+   long box is not), and in 2-D not where the tiles' second wave over the GPU would be less than half full (about 100k to
+   135k particles). Off by default elsewhere; enable = 1 / 0 chooses either way. */
 hcc_status hcc_set_tile_staging(hcc_ctx *ctx, int32_t enable);
 /* Whether the full passes of the next step are tile-staged, the union entries over all tiles and the largest union
    (any output may be NULL). */

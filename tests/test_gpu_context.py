@@ -146,3 +146,14 @@ def test_default_form_follows_the_numbering(hcc, cuda_lib, kind):
                 ctx.step(0.0, dt)
             out.append((ctx.download_state(), ctx.orders()))
         assert out[0][0].tobytes() == out[1][0].tobytes() and np.array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("waves,default", [(0.9, True), (1.15, False), (1.5, True)])
+def test_default_form_in_2d_follows_the_waves(hcc, cuda_lib, waves, default):
+    """2-D Euler, five tiles of 128 particles on an SM: the stream-fed pass where a second wave of tiles is nearly empty."""
+    import torch
+    n = round((waves * 5 * 128 * torch.cuda.get_device_properties(0).multi_processor_count) ** 0.5)
+    cloud = _box(hcc, 2, n)
+    ctx = hcc.Context(hcc.make_config(hcc.Euler(2), cloud, scheme=hcc.MUSCL(2, 2), bc_map=OUTFLOW, precision="fp32"))
+    _prepare(ctx, cloud)
+    assert bool(ctx.tile_staging()["active"]) == default
