@@ -393,7 +393,7 @@ __device__ __forceinline__ void speeds(const PhysParams<T> &ph, const T *U, T *l
             T q2 = T(0);
 #pragma unroll
             for (int d = 0; d < D; ++d) {
-                u[d] = __fdiv_rn(U[1 + d], U[0]);
+                u[d] = U[1 + d] * inv_rho;
                 q2 = q2 + U[1 + d] * u[d];
             }
             c = __fsqrt_rn(ph.gamma * ph.gm1 * (U[D + 1] - T(0.5) * q2) * inv_rho);
@@ -3424,9 +3424,10 @@ __global__ void k_speeds(const StageArgs<T> a) {
 // in flight at once. The sum runs over the slots in order; in FP32 a group at a time, compensated (the step's error against
 // 64 bits 4.1e-8 rms instead of 8.0e-8 on 70^2 points, 5.8e-8 instead of 1.27e-7 on 31^3, at the same time). With the
 // table: FP64 3-D, 103k particles, 117 us (723 with the speeds recomputed in every slot); FP64 2-D, 68k, 31 us (122);
-// FP32 2-D, 1.01M, 83 us (107).
+// FP32 2-D, 1.01M, 83 us (107). FP32: five blocks an SM leave a group's loads their registers (3-D stream-fed, the call on
+// 33k / 373k interior particles: 30 / 114 us, 51 / 163 with the 32 registers of the unbounded kernel).
 template <typename T, int D, int M, int PDE, int RDEG>
-__global__ void k_cfl(const StageArgs<T> a, unsigned long long *dt_bits) {
+__global__ void __launch_bounds__(sizeof(T) == 4 ? 256 : 1024, sizeof(T) == 4 ? 5 : 1) k_cfl(const StageArgs<T> a, unsigned long long *dt_bits) {
     const int64_t i = full_particle(a, int64_t(blockIdx.x) * blockDim.x + threadIdx.x);
     double dti = INFINITY;
     if (i >= 0 && !a.g.bnd[i]) {
