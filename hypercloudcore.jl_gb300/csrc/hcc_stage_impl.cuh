@@ -3397,10 +3397,11 @@ __global__ void k_stage1(const StageArgs<T> a) {
 // Spacing of the speed table's rows: whole vectors.
 template <int D> constexpr int lam_stride() { return D == 3 ? 4 : D; }
 
-// s + x with the rounding error of the sum kept in c (FP32 CFL sums: a group of slots at a time).
+// s + x with the rounding error of the sum kept in c (FP32 CFL sums: a group of slots at a time). A sum that overflows stays
+// infinite (there is no error to keep): its step is zero, not unbounded.
 template <typename T> __device__ __forceinline__ void compensated(T &s, T &c, T x) {
-    const T y = x - c, u = s + y;
-    c = (u - s) - y;
+    const T y = x - c, u = s + y, e = (u - s) - y;
+    c = isfinite(e) ? e : T(0);
     s = u;
 }
 

@@ -193,3 +193,24 @@ def test_cfl_step(hcc, cuda_lib, D, n, tiles, bound):
         want = ctx["fp64"].time_step()
         error.append((ctx["fp32"].time_step() - want) / want)
     assert np.sqrt(np.mean(np.square(error))) < bound
+
+
+@pytest.mark.parametrize("D,tiles", [(2, False), (3, False), (3, True)])
+@pytest.mark.parametrize("system", ["advection", "euler"])
+def test_cfl_step_of_a_sum_that_overflows(hcc, cuda_lib, system, D, tiles):
+    """Speeds whose sum over the slots passes the largest float: the step is zero, as one over infinity."""
+    h = 1.0 / 12
+    cloud = hcc.rectangular_cloud((0.0,) * D, (1.0,) * D, h, 2.5 * h, jitter=0.25 * h, seed=D)
+    N = len(cloud.pos)
+    if system == "advection":
+        pde, U = hcc.LinearAdvection(((3e38,),) * D), np.ones((N, 1), np.float32)
+    else:
+        pde, U = hcc.Euler(D), np.zeros((N, D + 2), np.float32)
+        U[:, 0], U[:, D + 1] = 1e-4, 1e38
+    c = hcc.Context(hcc.make_config(pde, cloud, scheme=hcc.MUSCL(2, 2), bc_map=OUTFLOW, precision="fp32"))
+    c.upload_cloud(cloud)
+    c.build_neighbours()
+    c.prepare_geometry()
+    c.set_tile_staging(tiles)
+    c.upload_state(U)
+    assert c.time_step() == 0.0
