@@ -832,9 +832,12 @@ __device__ __forceinline__ void gather_one(const StageArgs<T> &a, const int64_t 
 // tile; longer ones keep four warps a tile, whose partial sums cost less to combine. The line depends on the list
 // alone, so results do not depend on the launch shape. States of 8 and more components keep blocks of four warps
 // (shared memory of their partial sums), and so does the flux pass in 1-D and 2-D: about 20 slots are few for 16 warps
-// (15.7 us a pass with 16 warps, 12.9 with four; the reconstruction pass 8.8 against 12.5).
+// (15.7 us a pass with 16 warps, 12.9 with four; the reconstruction pass 8.8 against 12.5). Third-order systems in 3-D have
+// eight in the flux pass: a slot takes up to 192 registers, and 16 warps leave 128 (188 bytes spilled). 3-D Euler, us a
+// step with 16 / eight: blast at 64k interior particles 3902 / 3793, 343k 9923 / 9825 (limiter 4707 / 4582, 12960 / 12870);
+// smooth, where lists are short, 2525 / 2483 and 6715 / 6816.
 template <int M> constexpr int split_warps() { return M >= 8 ? 4 : 16; }
-template <int D, int M> constexpr int flux_split_warps() { return M >= 8 || D < 3 ? 4 : 16; }
+template <int D, int M, int RDEG> constexpr int flux_split_warps() { return M >= 8 || D < 3 ? 4 : RDEG >= 2 && M > 2 ? 8 : 16; }
 template <int NW> __device__ __forceinline__ int split_share(unsigned nt) {
     return NW > 4 && nt <= HCC_SPLIT_WIDE_TILES ? NW : 4;
 }
@@ -1841,8 +1844,8 @@ __global__ void __launch_bounds__(128) k_gather_split(const StageArgs<double> a)
 // first warp combines the compensated partial sums (Kahan over the partials, minus their compensations) and the
 // extrema, and runs the epilogue. Block-stride over the list.
 template <typename T, int D, int M, int PDE, int RDEG, bool ALE, bool MOM = false>
-__global__ void __launch_bounds__(32 * flux_split_warps<D, M>()) k_flux_tiles(const StageArgs<T> a) {
-    constexpr int NW = flux_split_warps<D, M>();
+__global__ void __launch_bounds__(32 * flux_split_warps<D, M, RDEG>()) k_flux_tiles(const StageArgs<T> a) {
+    constexpr int NW = flux_split_warps<D, M, RDEG>();
     __shared__ FluxPart<T, M> parts[NW][32];
     const int lane = int(threadIdx.x & 31), wb = int(threadIdx.x >> 5);
     const unsigned nt = *a.wcount;
@@ -4144,7 +4147,7 @@ struct StageInst {
     template <bool MOM> static void flux_mom(const StageArgs<T> &a, int64_t n, cudaStream_t s) {
         if constexpr (sizeof(T) == 4) {
             if (!a.full) {
-                const unsigned g = split_grid(a, flux_split_warps<D, M>()), nth = 32 * flux_split_warps<D, M>();
+                const unsigned g = split_grid(a, flux_split_warps<D, M, RDEG>()), nth = 32 * flux_split_warps<D, M, RDEG>();
                 if (a.mover) k_flux_tiles<T, D, M, PDE, RDEG, true, MOM><<<g, nth, 0, s>>>(a);
                 else k_flux_tiles<T, D, M, PDE, RDEG, false, MOM><<<g, nth, 0, s>>>(a);
                 return;
@@ -4182,7 +4185,7 @@ struct StageInst {
                 }
             }
             if (!a.full) {   // FP32 worklist pass: split tiles
-                const unsigned g = split_grid(a, flux_split_warps<D, M>()), nth = 32 * flux_split_warps<D, M>();
+                const unsigned g = split_grid(a, flux_split_warps<D, M, RDEG>()), nth = 32 * flux_split_warps<D, M, RDEG>();
                 if (a.mover) k_flux_tiles<T, D, M, PDE, RDEG, true><<<g, nth, 0, s>>>(a);
                 else k_flux_tiles<T, D, M, PDE, RDEG, false><<<g, nth, 0, s>>>(a);
                 return;

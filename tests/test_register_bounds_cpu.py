@@ -52,3 +52,10 @@ def test_2d_two_variable_reconstruction_keeps_its_warps(tmp_path):
 def test_central_passes_take_the_list_in_fp64_only(tmp_path):
     """The FP32 pass reads its slot streams in step with the warps."""
     _compile(tmp_path, "static_assert(central_lists<double>() && !central_lists<float>(), \"lists of the central pass\");\n")
+
+
+def test_third_order_worklists_of_3d_systems_do_not_spill(tmp_path):
+    got = _compile(tmp_path, _instances("k_flux_tiles", "3, 5, HCC_PDE_EULER, 2, false, false", "3, 5, HCC_PDE_EULER, 2, true, false"))
+    assert len(got) == 2
+    for name, (registers, spilled) in got.items():
+        assert spilled == 0, (name, registers, spilled)
