@@ -1964,8 +1964,11 @@ template <int RW> constexpr int tile_stage_unroll() {
 
 // LIM: slope limiters, which go through gather_one. Without one, a particle off the cached fit (an order below the full
 // one, a failed fit) has zero slopes, and the kernel does without gather_one's registers.
+// Two blocks an SM with a limiter (three spilled 104 bytes): 3-D Euler, us a step with three / two, Barth-Jespersen at 64k
+// interior particles 1360 / 1149 (blast 1325 / 1165), at 343k 3872 / 3787 (3938 / 3913); Venkatakrishnan 1426 / 1240
+// (1300 / 1152), 4154 / 4176 (3933 / 3906).
 template <int D, int M, int PDE, bool LIM>
-__global__ void __launch_bounds__(2 * HCC_TILE, 3) k_gather_tile(const StageArgs<float> a) {
+__global__ void __launch_bounds__(2 * HCC_TILE, LIM ? 2 : 3) k_gather_tile(const StageArgs<float> a) {
     extern __shared__ __align__(16) float sm[];
     constexpr int W = tile_gather_row<D, M>(), GS = grad_row<float, D * M>();
     const int64_t t = blockIdx.x;

@@ -59,3 +59,10 @@ def test_third_order_worklists_of_3d_systems_do_not_spill(tmp_path):
     assert len(got) == 2
     for name, (registers, spilled) in got.items():
         assert spilled == 0, (name, registers, spilled)
+
+
+def test_limited_reconstruction_of_3d_tiles_does_not_spill(tmp_path):
+    got = _compile(tmp_path, "template __global__ void k_gather_tile<3, 5, HCC_PDE_EULER, true>(const StageArgs<float>);\n")
+    assert len(got) == 1
+    for name, (registers, spilled) in got.items():
+        assert spilled == 0, (name, registers, spilled)
